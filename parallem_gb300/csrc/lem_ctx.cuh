@@ -120,9 +120,9 @@ struct DevState {
     // the basin graph with basins numbered 0..n_basins-1 per step
     int32_t* bid;               // per label: its basin number
     int32_t* blab;              // per basin: its label
-    int32_t* boff;              // per basin: the spill round that last lowered it
-    unsigned long long* bdist;  // per basin: minimax distance to basin 0 (ordered key)
-    int32_t* adj_v;             // per edge: its two basin numbers
+    int32_t* boff;              // per basin: the basin whose component absorbed it in the spill
+    unsigned long long* bdist;  // per basin: the boundary height it was absorbed over (ordered key)
+    int32_t* adj_v;             // per edge: the components of its two basins
     DevScalars* sc;
     DemCtx dems;                // the DEMs of the grid
     int32_t* chunk_start;       // streaming passes: first chunk of each DEM (n + 1 entries)

@@ -40,36 +40,6 @@ __device__ __forceinline__ unsigned long long warp_min_u64(unsigned long long v)
     return v;
 }
 
-// Exclusive prefix sum over a block of 256 threads; s_scan holds 9 ints;
-// *total receives the block's sum.  Every thread of the block calls it.
-__device__ __forceinline__ int block_exclusive_scan(int v, int* s_scan, int* total) {
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-    }
-    if (lane == 31) s_scan[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-        const int x = lane < 8 ? s_scan[lane] : 0;
-        int ix = x;
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, ix, o);
-            if (lane >= o) ix += t;
-        }
-        if (lane < 8) s_scan[lane] = ix - x;
-        if (lane == 7) s_scan[8] = ix;
-    }
-    __syncthreads();
-    const int ex = s_scan[wid] + incl - v;
-    *total = s_scan[8];
-    __syncthreads();  // s_scan is free for the next call
-    return ex;
-}
-
 // Warp-aggregated append of `pred` lanes to list[*count].
 __device__ __forceinline__ void warp_append(bool pred, int32_t value, int32_t* list, int32_t* count, int cap,
                                             uint32_t* err) {
@@ -1195,185 +1165,179 @@ __global__ void k_flood_compact(const unsigned long long* __restrict__ ekey, con
 // Spill heights.  The Kruskal pass of routeflow.cu:520-572 gives every basin
 // that can drain to basin 0 the smallest height h at which it connects to
 // basin 0 through boundaries no higher than h: its minimax distance to basin 0
-// over the basin-pair edges.  It is computed here as the fixpoint raise(a) =
-// min over edges (a, b, w) of max(w, raise(b)), basin 0 at 0, with basins
-// numbered compactly.  The kernel first groups the edges by basin (the edges
-// of basin 0 left out: nothing lowers it), then relaxes in rounds: the first
-// sweeps the edge list for the edges of basin 0; every later round only the
-// edges of the basins lowered since the round before.
-__global__ void k_flood_spill(const int32_t* __restrict__ ea, const int32_t* __restrict__ eb,
-                              const unsigned long long* __restrict__ ew, unsigned long long* raise, int32_t* comp,
-                              unsigned long long* cdist, unsigned long long* cmaxw, const int32_t* __restrict__ bid,
-                              const int32_t* __restrict__ blab, int32_t* stamp, unsigned long long* bdist,
-                              int32_t* euv, int32_t* adj_e, int32_t* adj_v, int32_t* cursor, int list_cap,
-                              DevScalars* sc) {
+// over the basin-pair edges.  It is computed by Boruvka rounds.  In a round
+// every component but basin 0's takes its lowest outgoing edge (ties by list
+// position) and merges along it.  Following these choices from component to
+// component the edge heights never rise, so they end at basin 0's component or
+// at a pair that chose the same edge, whose smaller index stands for the merged
+// component.  A component is raised at least to its lowest edge and, having
+// merged along it, to whatever the component it joined is raised to; the
+// heights one representative takes in successive rounds never fall.  So the
+// minimax distance of a basin is the largest height on its chain of
+// absorptions: up[c] (the representative that absorbed c) and wup[c] (the edge
+// taken then), walked once at the end.
+//
+// Bound by the grid-wide rounds, then by atomics: relaxing the distances
+// hop by hop took as many rounds as the longest minimax path has basins (154
+// at 4096 x 4096 cells, 1.52 ms), while components shrink threefold per round.
+// Three barriers a round: pick the edge at the lowest height, absorb, relabel
+// the edges (dropping those inside a component) and take the new components'
+// lowest heights.  Once at most kSpillSolo edges are left block 0 runs the
+// remaining rounds alone with block barriers.
+constexpr int kSpillSolo = 2048;  // a block barrier and 8 edges per thread cost less than a grid barrier
+
+__device__ __forceinline__ void lower_u64(unsigned long long* p, unsigned long long v) {
+    if (v < __ldcg(p)) atomicMin(p, v);
+}
+
+__global__ void __launch_bounds__(256)
+    k_flood_spill(const int32_t* __restrict__ ea, const int32_t* __restrict__ eb,
+                  const unsigned long long* __restrict__ ew, unsigned long long* raise, int32_t* comp,
+                  unsigned long long* cdist, unsigned long long* cmaxw, int32_t* bid,
+                  const int32_t* __restrict__ blab, int32_t* up, unsigned long long* wup, int2* uv0, int2* uv1,
+                  int32_t* id0, int32_t* id1, int32_t* pick, int32_t* reps, int list_cap, DevScalars* sc) {
     if (sc->sinkcount_pass1 == 0) return;
     const int n = sc->n_edges;
     const int nb = sc->n_basins;
-    if (nb > list_cap) {  // `cursor` holds list_cap entries
+    if (nb > list_cap) {  // `pick` and `reps` hold list_cap entries
         if (blockIdx.x == 0 && threadIdx.x == 0) raise_error(&sc->err, ErrFlags::kCapacity);
         return;
     }
     cg::grid_group grid = cg::this_grid();
-    __shared__ int s_scan[9];
-    const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t gstride = (size_t)gridDim.x * blockDim.x;
-    const int lane = threadIdx.x & 31;
+    __shared__ int s_cnt[9];
+    size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    size_t gstride = (size_t)gridDim.x * blockDim.x;
     const int32_t z = nb > 0 ? bid[0] : -1;  // basin 0 is on an edge whenever it borders a basin
-    // The edges grouped by basin: offsets in comp (nb + 1 entries), chunk sums
-    // of their prefix sum in cmaxw; both are idle until the walled-in pass.
-    int32_t* const off = comp;
-    int32_t* const csum = reinterpret_cast<int32_t*>(cmaxw);
+    constexpr int32_t kNone = 0x7fffffff;
+    // per component, by round parity: lowest outgoing height and the position
+    // of the edge taken (comp, cdist and cmaxw are idle until the walled-in
+    // pass); per round % 3: edges and representatives left
+    auto low = [&](int parity) { return parity ? cmaxw : cdist; };
+    auto best = [&](int parity) { return parity ? comp : pick; };
+    int32_t* const nlive = sc->counters;
+    int32_t* const nreps = sc->counters + 3;
     for (size_t i = gtid; i < (size_t)nb; i += gstride) {
-        bdist[i] = (int32_t)i == z ? 0ull : ~0ull;
-        stamp[i] = -1;
-        cursor[i] = 0;
+        up[i] = (int32_t)i;
+        low(1)[i] = ~0ull;
+        best(1)[i] = kNone;
     }
-    if (gtid == 0) sc->flag[0] = sc->flag[1] = sc->flag[2] = 0;
-    grid.sync();
-    for (size_t i = gtid; i < (size_t)n; i += gstride) {  // degrees
-        const int32_t a = bid[ea[i]], b = bid[eb[i]];
-        euv[2 * i] = a;
-        euv[2 * i + 1] = b;
-        if (a != z && b != z) {
-            atomicAdd(cursor + a, 1);
-            atomicAdd(cursor + b, 1);
-        }
-    }
-    grid.sync();
-    // exclusive prefix sum of the degrees: per chunk of at least 256 basins,
-    // then over the chunk sums (block 0), then within the chunks again
-    const int chunk = max(256, (nb + (int)gridDim.x - 1) / (int)gridDim.x);
-    const int nchunks = (nb + chunk - 1) / chunk;
-    const int c0 = min(nb, (int)blockIdx.x * chunk), c1 = min(nb, c0 + chunk);
-    if ((int)blockIdx.x < nchunks) {
-        int part = 0;
-        for (int i = c0 + (int)threadIdx.x; i < c1; i += blockDim.x) part += cursor[i];
-        int total = 0;
-        block_exclusive_scan(part, s_scan, &total);
-        if (threadIdx.x == 0) csum[blockIdx.x] = total;
-    }
-    grid.sync();
-    if (blockIdx.x == 0) {
-        int carry = 0;
-        for (int b0 = 0; b0 < nchunks; b0 += blockDim.x) {
-            const int b = b0 + (int)threadIdx.x;
-            const int v = b < nchunks ? csum[b] : 0;
-            int total = 0;
-            const int ex = block_exclusive_scan(v, s_scan, &total);
-            if (b < nchunks) csum[b] = carry + ex;
-            carry += total;
-        }
-        if (threadIdx.x == 0) off[nb] = carry;
-    }
-    grid.sync();
-    if ((int)blockIdx.x < nchunks) {
-        int carry = csum[blockIdx.x];
-        for (int i0 = c0; i0 < c1; i0 += blockDim.x) {
-            const int i = i0 + (int)threadIdx.x;
-            const int v = i < c1 ? cursor[i] : 0;
-            int total = 0;
-            const int ex = block_exclusive_scan(v, s_scan, &total);
-            if (i < c1) {
-                off[i] = carry + ex;
-                cursor[i] = carry + ex;  // where the basin's next edge goes
-            }
-            carry += total;
-        }
-    }
+    if (gtid < 6) sc->counters[gtid] = 0;
     grid.sync();
     for (size_t i = gtid; i < (size_t)n; i += gstride) {
-        const int32_t a = euv[2 * i], b = euv[2 * i + 1];
-        if (a == z || b == z) continue;
-        const int pa = atomicAdd(cursor + a, 1), pb = atomicAdd(cursor + b, 1);
-        adj_e[pa] = (int32_t)i;
-        adj_v[pa] = b;
-        adj_e[pb] = (int32_t)i;
-        adj_v[pb] = a;
+        const int32_t a = bid[ea[i]], b = bid[eb[i]];
+        const unsigned long long w = ew[i];
+        uv0[i] = make_int2(a, b);
+        id0[i] = (int32_t)i;
+        if (a != z) lower_u64(low(1) + a, w);
+        if (b != z) lower_u64(low(1) + b, w);
     }
     grid.sync();
-    // Round r relaxes the edges of every basin lowered in round r - 1 or
-    // earlier in round r (its stamp: the last round that lowered it), from
-    // the distance the basin has when its warp reaches it; a round that
-    // lowers nothing ends the loop.
-    const size_t warp = gtid >> 5, nwarps = gstride >> 5;
-    int round = 1;
-    for (;; ++round) {
-        if (gtid == 0) sc->flag[(round + 1) % 3] = 0;
-        bool lowered = false;
-        if (round == 1) {
-            for (size_t i = gtid; i < (size_t)n; i += gstride) {
-                const int2 uv = *reinterpret_cast<const int2*>(euv + 2 * i);
-                if (uv.x != z && uv.y != z) continue;
-                const int32_t v = uv.x == z ? uv.y : uv.x;
-                const unsigned long long cv = ew[i];
-                if (cv < __ldcg(bdist + v) && atomicMin(bdist + v, cv) > cv) {
-                    stamp[v] = round;
-                    lowered = true;
-                }
-            }
-        } else {
-            // the edge lists of a warp's 32 basins that are active,
-            // concatenated and relaxed 32 edges at a time; a lane finds the
-            // basin of its edge by a search over the lanes' prefix sums
-            for (size_t u0 = warp * 32; u0 < (size_t)nb; u0 += nwarps * 32) {
-                const size_t mine = u0 + lane;
-                const bool act = mine < (size_t)nb && __ldcg(stamp + mine) >= round - 1;
-                int j0 = 0, deg = 0;
-                unsigned long long du = 0;
-                if (act) {
-                    j0 = off[mine];
-                    deg = off[mine + 1] - j0;
-                    du = __ldcg(bdist + mine);
-                }
-                int incl = deg;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += t;
-                }
-                const int total = __shfl_sync(0xffffffffu, incl, 31);
-                for (int t0 = 0; t0 < total; t0 += 32) {
-                    const int t = t0 + lane;
-                    int k = 0;  // the first lane whose inclusive sum exceeds t
-#pragma unroll
-                    for (int step = 16; step > 0; step >>= 1) {
-                        const int pk = __shfl_sync(0xffffffffu, incl, k + step - 1);
-                        if (pk <= t) k += step;
-                    }
-                    const int kin = __shfl_sync(0xffffffffu, incl, k);
-                    const int kdeg = __shfl_sync(0xffffffffu, deg, k);
-                    const int kj0 = __shfl_sync(0xffffffffu, j0, k);
-                    const unsigned long long kdu = __shfl_sync(0xffffffffu, du, k);
-                    if (t < total) {
-                        const int j = kj0 + t - (kin - kdeg);
-                        const int32_t v = adj_v[j];
-                        const unsigned long long w = ew[adj_e[j]];
-                        const unsigned long long cv = w > kdu ? w : kdu;
-                        if (cv < __ldcg(bdist + v) && atomicMin(bdist + v, cv) > cv) {
-                            stamp[v] = round;
-                            lowered = true;
-                        }
-                    }
-                }
-            }
-        }
-        if (__any_sync(0xffffffffu, lowered) && lane == 0 && __ldcg(&sc->flag[round % 3]) == 0)
-            sc->flag[round % 3] = 1;
-        grid.sync();
-        if (*((volatile int32_t*)&sc->flag[round % 3]) == 0) break;
+    bool solo = false;
+    int round = 1, live = n, nrep = nb;
+    for (; live > 0; ++round) {
         if (round >= round_cap_of(sc)) {
             if (gtid == 0) raise_error(&sc->err, ErrFlags::kNoConverge);
             break;
         }
+        if (!solo && live <= kSpillSolo) {  // the same decision in every block
+            if (blockIdx.x != 0) break;
+            solo = true;
+            gstride = blockDim.x;
+        }
+        auto barrier = [&] {
+            if (solo)
+                __syncthreads();
+            else
+                grid.sync();
+        };
+        const int cur = round & 1, nxt = cur ^ 1;
+        const int2* const uv = cur ? uv0 : uv1;
+        const int32_t* const id = cur ? id0 : id1;
+        // of a component's lowest edges the first of the list
+        for (size_t i = gtid; i < (size_t)live; i += gstride) {
+            const int2 e = __ldcg(uv + i);
+            const unsigned long long w = ew[__ldcg(id + i)];
+            if (e.x != z && __ldcg(low(cur) + e.x) == w) atomicMin(best(cur) + e.x, (int32_t)i);
+            if (e.y != z && __ldcg(low(cur) + e.y) == w) atomicMin(best(cur) + e.y, (int32_t)i);
+        }
+        if (gtid == 0) nlive[(round + 1) % 3] = nreps[(round + 1) % 3] = 0;
+        barrier();
+        // representatives: round 1 takes every basin, later rounds the list of
+        // the round before (at most half of its predecessor: bid is spent)
+        const int32_t* const from = cur ? bid : reps;
+        int32_t* const to = cur ? reps : bid;
+        for (size_t base = gtid - threadIdx.x; base < (size_t)nrep; base += gstride) {
+            const size_t i = base + threadIdx.x;
+            int32_t c = -1;
+            if (i < (size_t)nrep) c = round == 1 ? (int32_t)i : __ldcg(from + i);
+            int32_t root = -1, p = c >= 0 && c != z ? __ldcg(best(cur) + c) : kNone;
+            if (p != kNone) {  // (a component without an edge keeps up[c] == c and leaves the list)
+                for (int32_t x = c, hop = 0; root < 0 && hop < nb; ++hop) {
+                    const int2 e = __ldcg(uv + p);
+                    const int32_t o = e.x == x ? e.y : e.x;
+                    const int32_t po = o == z ? kNone : __ldcg(best(cur) + o);
+                    if (o == z)
+                        root = z;
+                    else if (po == p)
+                        root = min(x, o);
+                    x = o;
+                    p = po;
+                }
+                if (root == c) {
+                    low(nxt)[c] = ~0ull;
+                    best(nxt)[c] = kNone;
+                } else {
+                    up[c] = root;
+                    wup[c] = __ldcg(low(cur) + c);
+                }
+            }
+            const int at = block_reserve(root >= 0 && root == c, nreps + round % 3, s_cnt);
+            if (at >= 0) to[at] = c;
+        }
+        barrier();
+        int2* const uvn = cur ? uv1 : uv0;
+        int32_t* const idn = cur ? id1 : id0;
+        for (size_t base = gtid - threadIdx.x; base < (size_t)live; base += gstride) {
+            const size_t i = base + threadIdx.x;
+            int2 e = make_int2(0, 0);
+            int32_t k = 0;
+            if (i < (size_t)live) {
+                e = __ldcg(uv + i);
+                k = __ldcg(id + i);
+                e = make_int2(__ldcg(up + e.x), __ldcg(up + e.y));
+            }
+            const int at = block_reserve(e.x != e.y, nlive + round % 3, s_cnt);
+            if (at >= 0) {
+                const unsigned long long w = ew[k];
+                uvn[at] = e;
+                idn[at] = k;
+                if (e.x != z) lower_u64(low(nxt) + e.x, w);
+                if (e.y != z) lower_u64(low(nxt) + e.y, w);
+            }
+        }
+        barrier();
+        live = *((volatile int32_t*)&nlive[round % 3]);
+        nrep = *((volatile int32_t*)&nreps[round % 3]);
     }
+    gstride = (size_t)gridDim.x * blockDim.x;
+    grid.sync();
     for (size_t i = gtid; i < (size_t)nb; i += gstride) {
         const int32_t L = blab[i];
-        if (L != 0) raise[L] = __ldcg(bdist + i);
+        if (L == 0) continue;
+        int32_t c = (int32_t)i;
+        unsigned long long h = 0ull;
+        while (c != z) {
+            const int32_t u = __ldcg(up + c);
+            if (u == c) break;  // a component that never reaches basin 0
+            const unsigned long long w = __ldcg(wup + c);
+            h = w > h ? w : h;
+            c = u;
+        }
+        raise[L] = c == z ? h : ~0ull;
     }
     if (gtid == 0) raise[0] = 0ull;
     if (gtid == 0) {
-        sc->spill_rounds = round + 1;
+        sc->spill_rounds = round;
         sc->flag[3] = 0;
     }
     grid.sync();
@@ -1672,21 +1636,23 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
         int32_t* comp = s.comp;
         unsigned long long* cdist = s.cdist;
         unsigned long long* cmaxw = s.cmaxw;
-        const int32_t* bidp = s.bid;
+        int32_t* bidp = s.bid;
         const int32_t* blab = s.blab;
-        int32_t* stamp = s.boff;
-        unsigned long long* bdist = s.bdist;
-        int32_t* euv = s.adj_v;
-        // the basin-pair table is idle after compaction: 2 * ecap int32 each
-        int32_t* adj_e = reinterpret_cast<int32_t*>(s.ekey);
-        int32_t* adj_v = reinterpret_cast<int32_t*>(s.ewt);
-        int32_t* cursor = s.pending;  // an int32 grid unused from the label jumping to the second direction pass
-        int list_cap = (int)std::min<size_t>((size_t)k.W * k.H, (size_t)INT32_MAX);  // entries of `pending`
+        int32_t* up = s.boff;
+        unsigned long long* wup = s.bdist;
+        // edge lists of the rounds; the basin-pair table is idle after compaction
+        int2* uv0 = reinterpret_cast<int2*>(s.adj_v);
+        int2* uv1 = reinterpret_cast<int2*>(s.ewt);
+        int32_t* id0 = reinterpret_cast<int32_t*>(s.ekey);
+        int32_t* id1 = id0 + s.ecap;
+        int32_t* pick = s.pending;  // int32 grids unused from the label jumping to the second direction pass
+        int32_t* reps = s.list_a;
+        int list_cap = (int)std::min<size_t>((size_t)k.W * k.H, (size_t)INT32_MAX);  // entries of `pick` and `reps`
         DevScalars* sc = s.sc;
-        void* args[] = {(void*)&ea,    (void*)&eb,    (void*)&ew,     (void*)&raise, (void*)&comp,
-                        (void*)&cdist, (void*)&cmaxw, (void*)&bidp,   (void*)&blab,  (void*)&stamp,
-                        (void*)&bdist, (void*)&euv,   (void*)&adj_e,  (void*)&adj_v, (void*)&cursor,
-                        (void*)&list_cap, (void*)&sc};
+        void* args[] = {(void*)&ea,   (void*)&eb,   (void*)&ew,   (void*)&raise, (void*)&comp, (void*)&cdist,
+                        (void*)&cmaxw, (void*)&bidp, (void*)&blab, (void*)&up,    (void*)&wup,  (void*)&uv0,
+                        (void*)&uv1,  (void*)&id0,  (void*)&id1,  (void*)&pick,  (void*)&reps, (void*)&list_cap,
+                        (void*)&sc};
         if ((r = coop("k_flood_spill", (const void*)k_flood_spill, s.coop_blocks[kCkSpill], args, L)) != LEM_OK) return r;
     }
     LEM_LAUNCH(L, k_flood_raise, flat_blocks(span, T, big), T, s.z, s.mask, s.ws, s.raise, s.zf, k, s.sc, s.dems,
