@@ -656,8 +656,8 @@ lem_status create_common(const lem_grid_desc* grid, const lem_params* params, in
     ALLOC(s.contrib, N);
     ALLOC(s.t_dst, N);
     ALLOC(s.t_pend, N);
-    ALLOC(s.t_orng, N);
-    ALLOC(s.t_la, N);
+    ALLOC(s.t_rec, N);
+    ALLOC(s.t_nxt, N);
     {
         const size_t tiles = (size_t)((grid->width + kTile - 1) / kTile) * ((grid->height + kTile - 1) / kTile);
         ALLOC(s.t_ent, tiles * kTileEnt);

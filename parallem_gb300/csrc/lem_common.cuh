@@ -99,7 +99,7 @@ struct DevScalars {
     int32_t flag[4];                 // convergence flags of the cooperative loops
     int32_t counters[8];
     int32_t tiled_ok;                // 1: this step's accumulation may take the tiled path
-    int32_t tile_src;                // tile outlets with no pending inflow (coarse sources)
+    int32_t tile_src;                // tile outlets listed for the coarse wave
     int32_t sed_tiled_ok;            // 1: this step's sediment routing may take the tiled path
     int32_t epoch;                   // flow-direction stages run so far (first-seen marks of basin labels)
     int32_t round_cap;               // rounds of every device loop before it gives up (0: kDefaultRoundCap)

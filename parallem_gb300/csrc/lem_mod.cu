@@ -324,7 +324,6 @@ struct SedCell {
     __device__ __forceinline__ int receivers(int32_t cur, int x, int y, int32_t* r) const {
         return code_receivers(fd, mask, cur, x, y, W, H, r);
     }
-    __device__ __forceinline__ void prefetch(int32_t) const {}
 };
 
 // The sediment wave: every source starts it; cells follow as their last donor
@@ -357,7 +356,6 @@ __global__ void k_sed_walk(const uint8_t* __restrict__ mask, const uint8_t* __re
 // Cell classes follow MFDsedbud: in-catchment cells off row 0 and column 0 are
 // computed; every other in-grid donor blocks its receiver.
 
-constexpr int kProgLocal = 256;  // program nodes the coarse evaluator keeps in local memory
 constexpr int kFinNz = 1;      // final-pass slot: the cell's sediment column is not empty
 constexpr int kFinOutlet = 2;  // final-pass slot: an outlet (the coarse wave stored it; counted only)
 constexpr int kPool = kTilePool;
@@ -493,10 +491,10 @@ __global__ void __launch_bounds__(256, 5)
     k_sedt_local(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd, const float* __restrict__ ero,
                  const float* __restrict__ inci, const float* __restrict__ geli, float* depo, float* stone,
                  float* fines, float* soilT, int32_t* __restrict__ t_dst, int32_t* __restrict__ t_pend,
-                 int32_t* __restrict__ t_orng, float2* __restrict__ t_out, float4* __restrict__ p_abc,
-                 int32_t* __restrict__ p_ref, float4* __restrict__ p_map, uint8_t* __restrict__ t_stat,
-                 int4* __restrict__ f_idx, float4* __restrict__ f_map, float2* __restrict__ f_ds,
-                 int32_t* __restrict__ t_fcnt, int32_t* srcs, ModelConsts k, DevScalars* sc, DemCtx dc, TileSet ts) {
+                 int4* __restrict__ t_rec, float4* __restrict__ p_abc, int32_t* __restrict__ p_ref,
+                 float4* __restrict__ p_map, uint8_t* __restrict__ t_stat, int4* __restrict__ f_idx,
+                 float4* __restrict__ f_map, float2* __restrict__ f_ds, int32_t* __restrict__ t_fcnt, int32_t* outs,
+                 ModelConsts k, DevScalars* sc, DemCtx dc, TileSet ts) {
     if (!sc->sed_tiled_ok) return;
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
@@ -522,13 +520,15 @@ __global__ void __launch_bounds__(256, 5)
     __shared__ uint8_t s_nz[kTile * kTile];
     __shared__ int16_t s_olist[kTileEnt];
     __shared__ int32_t s_ocnt[kTileEnt];
+    // per outlet, its program's nodes in the low half and their inputs in the
+    // high half: the counts, and where each starts
     __shared__ int32_t s_pcnt[kTileEnt];
-    __shared__ int16_t s_pstart[kTileEnt];
+    __shared__ int32_t s_pstart[kTileEnt];
     __shared__ int16_t s_pfill[kTileEnt];
     __shared__ int16_t s_q[kTile * kTile];
     __shared__ int16_t s_rnd[kTile * kTile];
-    __shared__ int s_no, s_nt, s_done, s_pool, s_dem, s_qn, s_qend, s_fn;
-    __shared__ int s_wcnt[9];  // per-warp counts of the outlet list and the source append
+    __shared__ int s_no, s_nt, s_done, s_dem, s_qn, s_qend, s_fn;
+    __shared__ int s_wcnt[9];  // per-warp counts of the outlet list and its append
     const int W = k.W, H = k.H, TW = (W + kTile - 1) / kTile;
     const int t = ts.tile(blockIdx.x);
     const int tx0 = (t % TW) * kTile, ty0 = (t / TW) * kTile;
@@ -716,11 +716,11 @@ __global__ void __launch_bounds__(256, 5)
     // from another tile, join two waiting branches, or are the outlet.  The
     // waiting cells between nodes pass one value on; they become the maps of
     // the nodes' inputs.
-    int32_t* s_node = s_pend;  // the in-degrees are spent
+    int32_t* s_node = s_pend;  // a node's number of inputs, 0 elsewhere (the in-degrees are spent)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        bool node = false;
+        int node = 0;
         if (s_flag[l] == (kFDone | kFTaint) && s_kind[s_ptr[l]] == kKindOutlet) {
             int ntd = 0;
 #pragma unroll
@@ -731,7 +731,8 @@ __global__ void __launch_bounds__(256, 5)
                     (s_flag[nly * kTile + nlx] & kFTaint))
                     ++ntd;
             }
-            node = s_ext[l] != 0 || ntd >= 2 || s_kind[l] == kKindOutlet;
+            // every input of a node is waiting or comes from another tile
+            if (s_ext[l] != 0 || ntd >= 2 || s_kind[l] == kKindOutlet) node = s_ext[l] + ntd;
         }
         s_node[l] = node;
     }
@@ -739,7 +740,7 @@ __global__ void __launch_bounds__(256, 5)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int l = (ly0 + 8 * q) * kTile + lx;
-        if (s_node[l]) atomicAdd(&s_pcnt[s_oslot[s_ptr[l]]], 1);
+        if (s_node[l]) atomicAdd(&s_pcnt[s_oslot[s_ptr[l]]], 1 | (s_node[l] << 16));
     }
     // Every waiting cell between nodes: its map v -> stone from its one waiting
     // in-tile donor (in place of its own coefficients, which only nodes need
@@ -798,14 +799,14 @@ __global__ void __launch_bounds__(256, 5)
     }
     __syncthreads();
     const int no = s_no, nt = s_nt;
-    if (threadIdx.x == 0) {
-        int a = 0;
-        for (int i = 0; i < no; ++i) {
-            s_pstart[i] = (int16_t)a;
-            s_pfill[i] = (int16_t)a;
-            a += s_pcnt[i];
-        }
-        s_pool = 0;
+    if (threadIdx.x < 32) outlet_starts(s_pcnt, s_pstart, no);
+    __syncthreads();
+    const int j = threadIdx.x;
+    const int pcnt = j < no ? s_pcnt[j] : 0, pstart = j < no ? s_pstart[j] : 0;
+    int32_t* const s_ifill = s_pcnt;  // where the program's next node's inputs go (the counts are kept above)
+    if (j < no) {
+        s_ifill[j] = pstart >> 16;
+        s_pfill[j] = (int16_t)(pstart & 0xffff);
     }
     __syncthreads();
     // node slots: grouped by outlet, in the order the cells were reached
@@ -835,18 +836,10 @@ __global__ void __launch_bounds__(256, 5)
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
         if (!s_node[l]) continue;
-        const int pos = s_pos[l];
-        const int first = s_pstart[s_oslot[s_ptr[l]]];
-        int nin = 0;
-#pragma unroll
-        for (int d = 0; d < 8; ++d) {
-            const int nlx = lx + dir_dx(d), nly = ly + dir_dy(d);
-            const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-            if (!donates(s_code[nh], d) || s_cls[nh] != kCellIn) continue;
-            if (!in_tile(nlx, nly) || (s_flag[nly * kTile + nlx] & kFTaint)) ++nin;
-        }
-        const int start = atomicAdd(&s_pool, nin);
-        if (start + nin > kPool) {
+        const int pos = s_pos[l], slot = s_oslot[s_ptr[l]];
+        const int first = s_pstart[slot] & 0xffff;
+        const int start = atomicAdd(&s_ifill[slot], s_node[l]);
+        if (start + s_node[l] > kPool) {
             raise_error(&sc->err, ErrFlags::kCapacity);
             continue;
         }
@@ -899,200 +892,309 @@ __global__ void __launch_bounds__(256, 5)
         f_map[fbase + fslot[q]] = node ? map_identity() : make_float4(s_A[l], s_B[l], s_dep[l], s_stn[l]);
     }
     if (threadIdx.x == 0) t_fcnt[t] = second_wave ? -1 : s_fn;
-    const int j = threadIdx.x;
-    bool ready = false;
     int32_t og = 0;
     if (j < no) {
         const int o = s_olist[j];
         const int32_t opend = ((s_flag[o] & kFDone) ? 0 : kBlocked) + s_ocnt[j];
         og = (ty0 + o / kTile) * W + tx0 + (o & (kTile - 1));
-        t_orng[og] = ((int)s_pstart[j] << 16) | s_pcnt[j];
+        // (the coefficients of a waiting outlet, a node, are still in place)
+        t_rec[og] = make_int4((pstart << 16) | (pcnt & 0xffff), (pstart & ~0xffff) | (pcnt >> 16),
+                              __float_as_int(s_dep[o]), __float_as_int(s_stn[o]));
         t_pend[og] = opend;
-        t_out[og] = make_float2(s_dep[o], s_stn[o]);
-        ready = (opend == 0);
+        if (opend == 0) og = ~og;  // settled here: a source of the coarse wave
     }
-    block_append(ready, og, srcs, &sc->tile_src, W * H, &sc->err, s_wcnt);
+    block_append(j < no, og, outs, &sc->tile_src, W * H, &sc->err, s_wcnt);
     done = wsum(done);
     if ((threadIdx.x & 31) == 0 && done) atomicAdd(&s_done, done);
     __syncthreads();
     if (threadIdx.x == 0 && s_done && s_dem >= 0) atomicAdd(&dc.out[s_dem].sed_done, s_done);
 }
 
-// One outlet of the coarse sediment wave, a warp per outlet: its program
-// level by level (nodes of one tile-wave round depend only on earlier rounds,
-// and the program lists them by round), then its own stores by lane 0.
-// Gathered program of one outlet, per warp: the nodes' coefficients, the
-// first slot of each node's inputs, and per input either its mapped value
-// (an input from another tile, final when the outlet is ready) or its map and
-// the feeding node.  Programs larger than this take the inputs from memory.
-constexpr int kGatherNodes = 64;
-constexpr int kGatherInputs = 96;
+// The coarse sediment wave over the tile outlets.  The sources (settled in
+// their tiles) release their receivers in one parallel pass, which also links
+// every outlet to the one it drains to; then each warp takes a released outlet,
+// runs its program and walks downstream for as long as its outlet is the last
+// inflow to arrive (an outlet has one receiver, so each is reached once).
+//
+// Bound by the longest chain of tile crossings (about 240 at 4096 x 4096
+// cells, with 9 dependent nodes of a program each), so by the latency of one
+// crossing.  A program is static but for the values from other tiles: it is
+// copied to shared memory (cp.async) while the outlet above it is computed, and
+// the records further down are read one outlet earlier still.  Each lane then
+// holds one node with its first inputs in registers; a step computes every node
+// whose input nodes are done, and the values pass between lanes by shuffles.
+// Reading coefficients, references and maps level by level took 2150 cycles a
+// level, 2.3 ms in all; a quarter of the outlets on the longest chains have more
+// than 64 nodes, and such programs run from memory took 70000 cycles each.  The
+// outlet's other outputs are stored behind the release.
+constexpr int kGatherNodes = 64;   // larger programs are gathered 32 nodes at a time, when their turn comes
+constexpr int kGatherInputs = 88;  //   (two buffers for each of the block's warps fit 48 KB)
+constexpr int kGatherTurns = (kGatherInputs + 31) / 32;
+constexpr int kHeldInputs = 3;     // inputs of a node held in registers (the others stay in shared memory)
 
-struct SedCoarse {
-    const uint8_t* fd;
-    const int32_t* t_orng;
-    const int32_t* t_dst;
-    const float2* t_out;
-    const float4* p_abc;
-    const int32_t* p_ref;
-    const float4* p_map;
-    float* p_val;
-    float* depo;
-    float* stone;
-    float* fines;
-    float* soilT;
-    float* s_vals;    // kProgLocal values per warp of the block
-    float4* s_abc;    // kGatherNodes per warp
-    int16_t* s_ib;    // kGatherNodes per warp: first input slot of the node
-    float4* s_imap;   // kGatherInputs per warp: mapped value (.x) or map
-    int32_t* s_iref;  // kGatherInputs per warp: 0 (mapped value) or the feeding node (negative)
-    int W, TW;
-    __device__ __forceinline__ void cell_warp(int32_t o, int x, int y, int lane) const {
-        const int rng = __ldg(t_orng + o);
-        const int cnt = rng & 0xffff;
-        if (cnt == 0) return;  // settled inside its tile
-        const int t = (y / kTile) * TW + x / kTile;
-        const size_t nbase = (size_t)t * kTile * kTile + (rng >> 16);
-        const size_t pool = (size_t)t * kPool;
-        const int wq = threadIdx.x >> 5;
-        float* vals = s_vals + wq * kProgLocal;
-        float4* abc = s_abc + wq * kGatherNodes;
-        int16_t* ib = s_ib + wq * kGatherNodes;
-        float4* imap = s_imap + wq * kGatherInputs;
-        int32_t* iref = s_iref + wq * kGatherInputs;
-        // Gather: every node's coefficients and inputs in one batch of loads,
-        // instead of a chain of loads per level of the program.
-        bool gathered = cnt <= kGatherNodes;
-        for (int c0 = 0, in0 = 0; gathered && c0 < cnt; c0 += 32) {
-            const int j = c0 + lane;
-            int nin = 0, start = 0;
-            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (j < cnt) {
-                r = __ldg(p_abc + nbase + j);
-                const int meta = __float_as_int(r.w);
-                start = meta & 2047;
-                nin = (meta >> 11) & 15;
-            }
-            int incl = nin;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int v = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += v;
-            }
-            const int total = __shfl_sync(0xffffffffu, incl, 31);
-            if (in0 + total > kGatherInputs) {
-                gathered = false;  // warp-uniform
-                break;
-            }
-            const int b0 = in0 + incl - nin;
-            if (j < cnt) {
-                abc[j] = r;
-                ib[j] = (int16_t)b0;
-            }
-            for (int jr = 0; jr < nin; ++jr) {
-                const int32_t ref = __ldg(p_ref + pool + start + jr);
-                const float4 mp = __ldg(p_map + pool + start + jr);
-                if (ref >= 0) {
-                    imap[b0 + jr] = make_float4(map_apply(mp, __ldcg(stone + ref)), 0.f, 0.f, 0.f);
-                    iref[b0 + jr] = 0;
-                } else {
-                    imap[b0 + jr] = mp;
-                    iref[b0 + jr] = ref;
-                }
-            }
-            in0 += total;
-        }
-        __syncwarp();
-        for (int i = 0; i < cnt;) {
-            const int j = i + lane;
-            float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
-            int meta = -1;
-            if (j < cnt) {
-                r = gathered ? abc[j] : __ldg(p_abc + nbase + j);
-                meta = __float_as_int(r.w);
-            }
-            const int lvl0 = __shfl_sync(0xffffffffu, meta >> 16, 0);
-            // the run: the nodes from i on that share i's level (independent of one another)
-            const unsigned same = __ballot_sync(0xffffffffu, j < cnt && (meta >> 16) == lvl0);
-            const int run = same == 0xffffffffu ? 32 : __ffs(~same) - 1;
-            const bool act = lane < run;
-            if (act) {
-                const int start = meta & 2047, nin = (meta >> 11) & 15;
-                const bool nz = (meta >> 15) & 1;
-                float from = r.z;
-                if (gathered) {
-                    const int b0 = ib[j];
-                    for (int jr = 0; jr < nin; ++jr) {
-                        const int32_t ref = iref[b0 + jr];
-                        const float4 mp = imap[b0 + jr];
-                        const float v = ref == 0 ? mp.x : map_apply(mp, vals[-ref - 1]);
-                        from = __fadd_rn(from, __fmul_rn(1.0f, v));
-                    }
-                } else {
-                    for (int jr = 0; jr < nin; ++jr) {
-                        const int32_t ref = __ldg(p_ref + pool + start + jr);
-                        const float4 mp = __ldg(p_map + pool + start + jr);
-                        float v;
-                        if (ref >= 0)
-                            v = __ldcg(stone + ref);
-                        else if (-ref - 1 < kProgLocal)
-                            v = vals[-ref - 1];
-                        else
-                            v = __ldcg(p_val + nbase - ref - 1);
-                        from = __fadd_rn(from, __fmul_rn(1.0f, map_apply(mp, v)));
-                    }
-                }
-                const float sn = nz ? sed_mix(r.x, r.y, from) : r.x;
-                if (j < kProgLocal) vals[j] = sn;
-                __stcg(p_val + nbase + j, sn);  // the final pass maps every node's value onto its chain
-            }
-            __syncwarp();
-            i += run;
-        }
-        if (lane == 0) {
-            // the outlet is the last node of its program
-            const int j = cnt - 1;
-            const float sn = j < kProgLocal ? vals[j] : __ldcg(p_val + nbase + j);
-            const int meta = __float_as_int(__ldg(p_abc + nbase + j).w);
-            const float2 out = __ldg(t_out + o);
-            depo[o] = out.x;
-            if ((meta >> 15) & 1) {
-                __stcg(stone + o, sn);
-                fines[o] = __fsub_rn(100.0f, sn);
-            }
-            soilT[o] = out.y;
-        }
-        __syncwarp();  // the gather buffers are reused by the warp's next node
-    }
-    __device__ __forceinline__ int receivers(int32_t o, int x, int y, int32_t* r) const {
-        const int d = bit_dir(__ldg(fd + o));
-        const int32_t rc = (y + dir_dy(d)) * W + x + dir_dx(d);
-        const int32_t dst = __ldg(t_dst + rc);
-        r[0] = dst;
-        return dst >= 0 ? 1 : 0;
-    }
-    // the receiving outlet's record, read first when this warp carries on with it
-    __device__ __forceinline__ void prefetch(int32_t o) const {
-        if (o >= 0) prefetch_l2(t_orng + o);
-    }
+struct SedProg {
+    float4 abc[kGatherNodes];    // the nodes' coefficients
+    float4 map[kGatherInputs];   // their inputs' maps; once the outlet is ready, the mapped value (.x) of an
+    int32_t ref[kGatherInputs];  //   input from another tile, its ref 0; below 0 the feeding node
 };
 
-__global__ void __launch_bounds__(256)
-    k_sedt_coarse(const uint8_t* __restrict__ fd, const int32_t* __restrict__ t_orng,
-                  const int32_t* __restrict__ t_dst, const float2* __restrict__ t_out,
-                  const float4* __restrict__ p_abc, const int32_t* __restrict__ p_ref,
-                  const float4* __restrict__ p_map, float* p_val, float* depo, float* stone, float* fines,
-                  float* soilT, int32_t* t_pend, int32_t* list_a, int32_t* list_b, ModelConsts k, DevScalars* sc) {
+__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+__global__ void __launch_bounds__(256, 4)
+    k_sedt_coarse(const uint8_t* __restrict__ fd, const int4* __restrict__ t_rec, int32_t* t_nxt,
+                  const int32_t* __restrict__ t_dst, const float4* __restrict__ p_abc,
+                  const int32_t* __restrict__ p_ref, const float4* __restrict__ p_map, float* p_val, float* depo,
+                  float* stone, float* fines, float* soilT, int32_t* t_pend, const int32_t* __restrict__ outs,
+                  int32_t* ready, ModelConsts k, DevScalars* sc) {
     if (!sc->sed_tiled_ok) return;
-    __shared__ float s_vals[8 * kProgLocal];
-    __shared__ float4 s_abc[8 * kGatherNodes];
-    __shared__ int16_t s_ib[8 * kGatherNodes];
-    __shared__ float4 s_imap[8 * kGatherInputs];
-    __shared__ int32_t s_iref[8 * kGatherInputs];
-    if (blockIdx.x == 0 && threadIdx.x == 0) sc->counters[0] = sc->tile_src;
-    const SedCoarse op{fd,    t_orng, t_dst, t_out,  p_abc, p_ref,  p_map,  p_val,  depo,          stone,
-                       fines, soilT,  s_vals, s_abc, s_ib,  s_imap, s_iref, k.W,    (k.W + kTile - 1) / kTile};
-    wave_walk_warp(op, t_pend, list_a, list_b, k.W, k.H, sc);
+    cg::grid_group grid = cg::this_grid();
+    __shared__ SedProg s_prog[8][2];
+    __shared__ float s_vals[8][kGatherNodes];
+    __shared__ int s_cnt[9];
+    const int W = k.W, TW = (W + kTile - 1) / kTile;
+    const size_t N = (size_t)W * k.H;
+    const int n = sc->tile_src;
+    int32_t* const n_ready = &sc->counters[0];
+    int32_t* const head = &sc->counters[1];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *n_ready = *head = 0;
+    grid.sync();
+    for (size_t base = (size_t)blockIdx.x * blockDim.x; base < (size_t)n; base += (size_t)gridDim.x * blockDim.x) {
+        const size_t i = base + threadIdx.x;
+        int32_t nx = -1;
+        bool rdy = false;
+        if (i < (size_t)n) {
+            const int32_t e = outs[i], o = e < 0 ? ~e : e;
+            const int d = bit_dir(fd[o]);  // the receiver is a routed cell of another tile
+            nx = t_dst[o + dir_dy(d) * W + dir_dx(d)];
+            t_nxt[o] = nx;
+            if (e < 0 && nx >= 0) rdy = atomicSub(t_pend + nx, 1) == 1;
+        }
+        block_append(rdy, nx, ready, n_ready, (int)N, &sc->err, s_cnt);
+    }
+    grid.sync();
+    const int nin = *((volatile int32_t*)n_ready);
+    const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+    float* const vals = s_vals[wq];
+    auto tile_of = [&](int32_t o) {
+        const int y = o / W, x = o - y * W;
+        return (y / kTile) * TW + x / kTile;
+    };
+    auto held = [](int4 r) { return (r.x & 0xffff) <= kGatherNodes && (r.y & 0xffff) <= kGatherInputs; };
+    // starts copying the program of an outlet of tile t
+    auto fetch = [&](SedProg& b, int t, int4 r) {
+        const int cnt = r.x & 0xffff, ni = r.y & 0xffff;
+        const float4* abc = p_abc + (size_t)t * kTile * kTile + (r.x >> 16);
+        const size_t in0 = (size_t)t * kPool + (r.y >> 16);
+        if (!held(r)) {  // a line of 128 bytes per lane
+#pragma unroll 1
+            for (int j = 8 * lane; j < cnt; j += 256) prefetch_l2(abc + j);
+#pragma unroll 1
+            for (int j = 8 * lane; j < ni; j += 256) {
+                prefetch_l2(p_map + in0 + j);
+                prefetch_l2(p_ref + in0 + j);
+            }
+            return;
+        }
+#pragma unroll 1
+        for (int j = lane; j < cnt; j += 32) cp_async16(&b.abc[j], abc + j);
+#pragma unroll 1
+        for (int j = lane; j < ni; j += 32) {
+            cp_async16(&b.map[j], p_map + in0 + j);
+            cp_async4(&b.ref[j], p_ref + in0 + j);
+        }
+    };
+    for (size_t guard = 0; guard <= N; ++guard) {
+        int32_t o = -1;
+        if (lane == 0) {
+            const int it = atomicAdd(head, 1);
+            if (it < nin) o = __ldcg(ready + it);
+        }
+        o = __shfl_sync(0xffffffffu, o, 0);
+        if (o < 0) break;
+        int4 r = __ldg(t_rec + o);
+        int32_t d = __ldcg(t_nxt + o);
+        int buf = 0, t = tile_of(o);
+        fetch(s_prog[wq][0], t, r);
+        int4 rd = make_int4(0, 0, 0, 0);  // the record of d and the outlet d drains to
+        int32_t e = -1;
+        if (d >= 0) {
+            rd = __ldg(t_rec + d);
+            e = __ldcg(t_nxt + d);
+        }
+        for (size_t chain = 0; o >= 0 && chain <= N; ++chain) {
+            SedProg& pr = s_prog[wq][buf];
+            const int cnt = r.x & 0xffff, ni = r.y & 0xffff;
+            const size_t nbase = (size_t)t * kTile * kTile + (r.x >> 16);
+            const size_t pool = (size_t)t * kPool;
+            const int in0 = r.y >> 16;
+            const bool gathered = held(r);
+            cp_async_wait();
+            __syncwarp();
+            // the values from other tiles, final now that the outlet is ready
+            if (gathered)
+#pragma unroll 1
+                for (int j = lane; j < ni; j += 32) {
+                    const int32_t ref = pr.ref[j];
+                    if (ref < 0) continue;
+                    pr.map[j].x = map_apply(pr.map[j], __ldcg(stone + ref));
+                    pr.ref[j] = 0;
+                }
+            // ahead of their use: the next outlet's program, the record after it
+            int4 re = make_int4(0, 0, 0, 0);
+            int32_t f = -1;
+            if (d >= 0) {
+                t = tile_of(d);
+                fetch(s_prog[wq][buf ^ 1], t, rd);
+                if (e >= 0) {
+                    re = __ldg(t_rec + e);
+                    f = __ldcg(t_nxt + e);
+                }
+            }
+            __syncwarp();
+            float sn = 0.f;  // the outlet's new stone: the last node of its program
+            bool snz = false;
+#pragma unroll 1
+            for (int i = 0, m; i < cnt; i += m) {
+                // The nodes i .. i + m - 1, one per lane.  An input from a node
+                // among these is its lane's value through the map (bits of
+                // need); one whose value is known becomes a constant map of
+                // the lane's own value, still 0.
+                const int j = i + lane;
+                m = min(32, cnt - i);
+                float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (lane < m) c = gathered ? pr.abc[j] : __ldg(p_abc + nbase + j);
+                const int meta = __float_as_int(c.w);
+                int nj = lane < m ? (meta >> 11) & 15 : 0;
+                const bool nz = (meta >> 15) & 1;
+                int b0 = (meta & 2047) - in0;
+                if (!gathered) {
+                    int incl = nj;
+#pragma unroll
+                    for (int d2 = 1; d2 < 32; d2 <<= 1) {
+                        const int w = __shfl_up_sync(0xffffffffu, incl, d2);
+                        if (lane >= d2) incl += w;
+                    }
+                    // as many nodes as have room for their inputs (at most 8 each)
+                    m = min(m, __popc(__ballot_sync(0xffffffffu, incl <= kGatherInputs)));
+                    b0 = incl - nj;
+                    if (lane >= m) nj = 0;
+                    // their places in the pool, then every input by its own lane
+#pragma unroll 1
+                    for (int q = 0; q < nj; ++q) pr.ref[b0 + q] = (meta & 2047) + q;
+                    const int total = __shfl_sync(0xffffffffu, incl, m - 1);
+                    __syncwarp();
+                    int32_t ref[kGatherTurns];
+                    float4 g[kGatherTurns];
+#pragma unroll
+                    for (int q = 0; q < kGatherTurns; ++q) {
+                        const int at = lane + 32 * q;
+                        if (at >= total) continue;
+                        const size_t from = pool + pr.ref[at];
+                        ref[q] = __ldg(p_ref + from);
+                        g[q] = __ldg(p_map + from);
+                    }
+#pragma unroll
+                    for (int q = 0; q < kGatherTurns; ++q) {
+                        const int at = lane + 32 * q;
+                        if (at >= total) continue;
+                        if (ref[q] >= 0) g[q].x = map_apply(g[q], __ldcg(stone + ref[q]));
+                        pr.map[at] = g[q];
+                        pr.ref[at] = ref[q] >= 0 ? 0 : ref[q];
+                    }
+                    __syncwarp();
+                }
+                uint32_t need = 0;
+                auto input = [&](int q, float4& f, int& src) {
+                    const bool mine = q < nj;
+                    const float4 g = pr.map[mine ? b0 + q : 0];
+                    const int32_t ref = mine ? pr.ref[b0 + q] : 0;
+                    bool known = ref == 0 || g.z > g.w;  // another tile's value, mapped; a constant map
+                    float val = !mine ? 0.f : (ref == 0 ? g.x : g.y);
+                    if (!known && -ref - 1 < i) {  // a node of an earlier turn
+                        val = map_apply(g, gathered ? vals[-ref - 1] : __ldcg(p_val + nbase - ref - 1));
+                        known = true;
+                    }
+                    f = make_float4(known ? 0.f : g.x, known ? val : g.y, known ? -INFINITY : g.z,
+                                    known ? INFINITY : g.w);
+                    src = known ? lane : -ref - 1 - i;
+                    need |= known ? 0u : 1u << src;
+                };
+                auto through = [](const float4 f, float x) {  // map_apply of a map that is no constant
+                    const float y = __fadd_rn(__fmul_rn(f.x, x), f.y);
+                    return y < f.z ? f.z : (y > f.w ? f.w : y);
+                };
+                float4 f[kHeldInputs];
+                int src[kHeldInputs];
+#pragma unroll
+                for (int q = 0; q < kHeldInputs; ++q) input(q, f[q], src[q]);
+                const int most = __reduce_max_sync(0xffffffffu, nj);
+#pragma unroll 1
+                for (int q = kHeldInputs; q < most; ++q) {  // read again in each step
+                    float4 f2;
+                    int s2;
+                    input(q, f2, s2);
+                }
+                uint32_t todo = m == 32 ? 0xffffffffu : (1u << m) - 1u;
+                float v = 0.f;
+#pragma unroll 1
+                for (int step = 0; todo && step < 32; ++step) {
+                    const bool act = ((todo >> lane) & 1u) && !(need & todo);
+                    float from = c.z;
+#pragma unroll
+                    for (int q = 0; q < kHeldInputs; ++q)
+                        from = __fadd_rn(from, through(f[q], __shfl_sync(0xffffffffu, v, src[q])));
+#pragma unroll 1
+                    for (int q = kHeldInputs; q < most; ++q) {
+                        float4 f2;
+                        int s2;
+                        input(q, f2, s2);
+                        from = __fadd_rn(from, through(f2, __shfl_sync(0xffffffffu, v, s2)));
+                    }
+                    const float sn2 = sed_mix(c.x, c.y, from);
+                    v = act ? (nz ? sn2 : c.x) : v;
+                    todo &= ~__ballot_sync(0xffffffffu, act);
+                }
+                if (lane < m) {
+                    if (gathered)
+                        vals[j] = v;
+                    else
+                        __stcg(p_val + nbase + j, v);
+                }
+                sn = __shfl_sync(0xffffffffu, v, m - 1);
+                snz = __shfl_sync(0xffffffffu, (int)nz, m - 1) != 0;
+                __syncwarp();
+            }
+            int32_t next = -1;
+            if (lane == 0) {
+                if (snz) __stcg(stone + o, sn);
+                if (d >= 0 && dec_acq_rel(t_pend + d) == 1) next = d;
+                depo[o] = __int_as_float(r.z);
+                if (snz) fines[o] = __fsub_rn(100.0f, sn);
+                soilT[o] = __int_as_float(r.w);
+            }
+            // the final pass maps every node's value onto its chain
+            if (gathered)
+#pragma unroll 1
+                for (int j = lane; j < cnt; j += 32) p_val[nbase + j] = vals[j];
+            o = __shfl_sync(0xffffffffu, next, 0);
+            r = rd;
+            d = e;
+            rd = re;
+            e = f;
+            buf ^= 1;
+        }
+        cp_async_wait();  // the buffers are refilled for the next outlet
+        __syncwarp();
+    }
 }
 
 constexpr uint8_t kStatNz = 4;  // k_sedt_final: flag in a waiting cell's status
@@ -1474,12 +1576,12 @@ lem_status launch_erosion(const DevState& s, const ModelConsts& k, uint32_t flag
     if (tiled) {
         const int tiles = ts.n;
         LEM_LAUNCH(L, k_sedt_local, tiles, 256, s.mask, s.fd, s.ero, s.inci, s.geli, s.depo, s.stone, s.fines,
-                   s.soilT, s.t_dst, s.t_pend, s.t_orng, s.t_la, s.p_abc, s.p_ref, s.p_map, s.t_stat, s.f_idx,
-                   s.f_map, s.f_ds, s.t_fcnt, s.list_b, k, s.sc, s.dems, ts);
+                   s.soilT, s.t_dst, s.t_pend, s.t_rec, s.p_abc, s.p_ref, s.p_map, s.t_stat, s.f_idx, s.f_map,
+                   s.f_ds, s.t_fcnt, s.list_b, k, s.sc, s.dems, ts);
         const uint8_t* fd = s.fd;
-        const int32_t* torng = s.t_orng;
+        const int4* trec = s.t_rec;
+        int32_t* tnxt = s.t_nxt;
         const int32_t* tdst = s.t_dst;
-        const float2* tout = s.t_la;
         const float4* pabc = s.p_abc;
         const int32_t* pref = s.p_ref;
         const float4* pmap = s.p_map;
@@ -1489,13 +1591,13 @@ lem_status launch_erosion(const DevState& s, const ModelConsts& k, uint32_t flag
         float* fines = s.fines;
         float* soilT = s.soilT;
         int32_t* tpend = s.t_pend;
-        int32_t* la = s.list_b;  // the outlets k_sedt_local found ready
-        int32_t* lb = s.list_a;
+        const int32_t* outs = s.list_b;  // the outlets, listed by k_sedt_local
+        int32_t* ready = s.list_a;
         ModelConsts kk = k;
         DevScalars* sc = s.sc;
-        void* args[] = {(void*)&fd,    (void*)&torng, (void*)&tdst,  (void*)&tout, (void*)&pabc, (void*)&pref,
-                        (void*)&pmap,  (void*)&pval,  (void*)&depo,  (void*)&stone, (void*)&fines, (void*)&soilT, (void*)&tpend,
-                        (void*)&la,    (void*)&lb,    (void*)&kk,    (void*)&sc};
+        void* args[] = {(void*)&fd,    (void*)&trec, (void*)&tnxt, (void*)&tdst,  (void*)&pabc, (void*)&pref,
+                        (void*)&pmap,  (void*)&pval, (void*)&depo, (void*)&stone, (void*)&fines, (void*)&soilT,
+                        (void*)&tpend, (void*)&outs, (void*)&ready, (void*)&kk,   (void*)&sc};
         L.pre("k_sedt_coarse");
         LEM_CUDA_TRY(coop_launch((const void*)k_sedt_coarse, s.coop_blocks[kCkSedCoarse], args, L.st));
         L.post();

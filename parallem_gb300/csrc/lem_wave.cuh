@@ -145,7 +145,6 @@ __device__ int wave_walk(const Op& op, int32_t* pending, int32_t* list_a, int32_
                 // loads overlap the cell's own chain of loads
                 int32_t rcv[8];
                 const int nr = op.receivers(cur, x, y, rcv);
-                for (int j = 0; j < nr; ++j) op.prefetch(rcv[j]);
                 op.cell(cur, x, y);
                 ++done;
                 int32_t next = -1;
@@ -216,6 +215,24 @@ __device__ __forceinline__ void list_outlets(const uint8_t* s_kind, int16_t* s_o
     if (threadIdx.x == 255) *s_no = base;  // the last warp's end is the total
 }
 
+// Exclusive prefix sums over a tile's outlets (at most kTileEnt), by warp 0.
+// Each count packs two numbers, one per 16-bit half, whose sums fit in theirs.
+__device__ __forceinline__ void outlet_starts(const int32_t* s_count, int32_t* s_start, int no) {
+    const int lane = threadIdx.x & 31;
+    int carry = 0;
+    for (int b = 0; b < no; b += 32) {
+        const int v = b + lane < no ? s_count[b + lane] : 0;
+        int incl = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += u;
+        }
+        if (b + lane < no) s_start[b + lane] = carry + incl - v;
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+}
+
 // The halo ring in a fixed order: top row, bottom row, left column, right column.
 constexpr int kRing = 4 * kTH - 4;
 constexpr int kRingChunks = (kRing + 31) / 32;
@@ -279,81 +296,6 @@ __device__ __forceinline__ void tile_wave(const Op& op, int32_t* s_pend, int16_t
     }
     __syncthreads();
 }
-
-// The wave of wave_walk with a whole warp per node: lane 0 takes a ready node,
-// Op::cell_warp(c, x, y, lane) computes it with every lane, lane 0 releases its
-// receivers and the warp carries on with the first it made ready.  For nodes
-// whose own computation has parallel parts (the sediment programs).
-template <class Op>
-__device__ void wave_walk_warp(const Op& op, int32_t* pending, int32_t* list_a, int32_t* list_b, int W, int H,
-                               DevScalars* sc) {
-    namespace cg = cooperative_groups;
-    cg::grid_group grid = cg::this_grid();
-    const size_t N = (size_t)W * H;
-    const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int lane = threadIdx.x & 31;
-    int32_t* cnt = sc->counters;  // [0..2] list sizes by round % 3, [3..5] take heads by round % 3
-    if (gtid == 0) {
-        cnt[1] = cnt[2] = 0;
-        cnt[3] = cnt[4] = cnt[5] = 0;
-    }
-    grid.sync();
-    for (int round = 0;; ++round) {
-        const int32_t* in = (round & 1) ? list_b : list_a;
-        int32_t* out = (round & 1) ? list_a : list_b;
-        const int nin = *((volatile int32_t*)&cnt[round % 3]);
-        if (nin == 0) break;
-        if (round >= round_cap_of(sc)) {
-            if (gtid == 0) raise_error(&sc->err, ErrFlags::kNoConverge);
-            break;
-        }
-        if (gtid == 0) {
-            cnt[(round + 2) % 3] = 0;
-            cnt[3 + (round + 1) % 3] = 0;
-        }
-        int32_t* head = &cnt[3 + round % 3];
-        for (size_t guard = 0; guard <= N; ++guard) {
-            int32_t cur = -1;
-            if (lane == 0) {
-                const int it = atomicAdd(head, 1);
-                if (it < nin) cur = __ldcg(in + it);
-            }
-            cur = __shfl_sync(0xffffffffu, cur, 0);
-            if (cur < 0) break;
-            for (size_t chain = 0; cur >= 0 && chain <= N; ++chain) {
-                const int x = cur % W, y = cur / W;
-                // the receivers first (static data): their loads overlap the node's
-                int32_t rcv[8];
-                int nr = 0;
-                if (lane == 0) {
-                    nr = op.receivers(cur, x, y, rcv);
-                    for (int j = 0; j < nr; ++j) op.prefetch(rcv[j]);
-                }
-                __syncwarp();
-                op.cell_warp(cur, x, y, lane);
-                __syncwarp();
-                int32_t next = -1;
-                if (lane == 0) {
-                    for (int j = 0; j < nr; ++j) {
-                        if (dec_acq_rel(pending + rcv[j]) == 1) {
-                            if (next < 0) {
-                                next = rcv[j];
-                            } else {
-                                const int p = atomicAdd(&cnt[(round + 1) % 3], 1);
-                                if (p < (int)N) out[p] = rcv[j];
-                            }
-                        }
-                    }
-                }
-                cur = __shfl_sync(0xffffffffu, next, 0);
-            }
-        }
-        grid.sync();
-    }
-}
-
-// Brings the line holding p into L2 (a hint: no value is read).
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 // Receivers of cell (x, y) by its direction code: in-grid, in-catchment cells.
 __device__ __forceinline__ int code_receivers(const uint8_t* __restrict__ fd, const uint8_t* __restrict__ mask,
