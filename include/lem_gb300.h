@@ -259,7 +259,8 @@ lem_status lem_set_graphs(lem_handle* h, int32_t on);
  * and merge loops routeflow.cu:285-302,314-338, accumulation mfd_simple.cu:
  * 204-226), and its basin-pair hash table overflows silently
  * (newflow.cu:860-872).  Here every loop stops after max_rounds rounds and the
- * next lem_synchronize returns LEM_ERR_NOCONVERGE; the basin-pair table holds
+ * next lem_synchronize returns LEM_ERR_NOCONVERGE (the dependency waves visit
+ * each cell once and end by themselves); the basin-pair table holds
  * at most 2^edge_table_log2 pairs and a full table makes lem_synchronize return
  * LEM_ERR_CAPACITY.  After either error the step's results are incomplete but
  * the handle stays usable.  0 in a field restores its default (65536 rounds;
@@ -352,7 +353,7 @@ lem_status lem_snapshot_load(lem_handle* h, int32_t id, const void* host, size_t
  * everything below one) output their own weight and the call returns
  * LEM_ERR_NOCONVERGE after writing d_fa.
  * Intermediate data lives in one statically allocated device array sized for
- * LEM_NOALLOC_MAX_CELLS cells (about 27 MB, held by every GPU that loads the
+ * LEM_NOALLOC_MAX_CELLS cells (about 17 MB, held by every GPU that loads the
  * library until the process exits); larger grids are rejected with
  * LEM_ERR_CAPACITY before any work.  The call looks up that array's device
  * address on the current device; the first call on a device must come before

@@ -282,6 +282,14 @@ inline cudaError_t coop_launch(const void* fn, int blocks, void** args, cudaStre
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
+// Blocks of the general dependency wave on n cells: a warp for every 256 cells
+// covers the front of a slope (a row or two of the grid); more only watch the
+// list.
+inline int walk_blocks(int coop, size_t n) {
+    const size_t b = (n + 2047) / 2048;
+    return b < (size_t)coop ? (int)b : coop;
+}
+
 #define LEM_LAUNCH(L, kern, grid, block, ...)                  \
     do {                                                       \
         (L).pre(#kern);                                        \

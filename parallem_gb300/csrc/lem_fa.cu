@@ -99,10 +99,10 @@ __global__ void k_fa_prep(const uint8_t* __restrict__ mask, const uint8_t* __res
     if (threadIdx.x == 0 && tot) atomicAdd(&dc.out[ch.d].n_active, tot);
 }
 
-// In-degrees and sources of the global accumulation wave, for the steps that
+// Words and sources of the general accumulation wave, for the steps that
 // take it (MFD, contributing area, or a step k_fa_prep sent off the tiled path).
 __global__ void k_fa_pend(const double* __restrict__ z, const uint8_t* __restrict__ mask,
-                          const uint8_t* __restrict__ fd, int32_t* __restrict__ pending, int32_t* __restrict__ contrib,
+                          const uint8_t* __restrict__ fd, int32_t* __restrict__ word, int32_t* __restrict__ contrib,
                           int32_t* ready, const int32_t* __restrict__ chunk_start, ModelConsts k, DemCtx dc,
                           DevScalars* sc, int gate) {
     if (gate && sc->tiled_ok) return;  // the tiled path accumulates this step
@@ -120,22 +120,28 @@ __global__ void k_fa_pend(const double* __restrict__ z, const uint8_t* __restric
             if (mask[i]) {
                 if (contrib) contrib[i] = 1;
                 int32_t pend = 0;
+                uint32_t donors = 0, receivers = 0;
+                const uint8_t code = fd[i];
 #pragma unroll
                 for (int d = 0; d < 8; ++d) {
                     const int nx = x + dir_dx(d), ny = y + dir_dy(d);
                     if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
                     const size_t n = (size_t)ny * W + nx;
+                    const bool in = mask[n];
+                    if (in) receivers |= code & dir_bit(d);
                     if (!donates(fd[n], d)) continue;
-                    if (mask[n])
+                    if (in) {
                         ++pend;
-                    else if (z[n] != kNoData)
+                        donors |= 1u << scan_index(d);
+                    } else if (z[n] != kNoData) {
                         pend |= kBlocked;
+                    }
                 }
-                pending[i] = pend;
+                word[i] = wave_word(pend, donors, receivers);
                 src = (pend == 0);
             } else {
                 if (contrib) contrib[i] = 0;
-                pending[i] = kBlocked;
+                word[i] = kBlocked;
             }
         }
         wave_append(src, (int32_t)i, ready, &sc->counters[0], (int)N, &sc->err);
@@ -171,56 +177,57 @@ __global__ void k_calcprops(const uint8_t* __restrict__ mask, const uint8_t* __r
     }
 }
 
-__device__ __forceinline__ float prop_of(const float* prop, const uint8_t* mask, size_t n, int slot) {
-    return prop ? prop[8 * n + slot] : (mask[n] ? 1.0f : 0.0f);
-}
-
 // One cell of correctmfdflow's CalcMFD (mfd_simple.cu:31-171): the weight plus
 // the donors' accumulation in the order E, SE, S, SW, W, NW, N, NE, a negative
-// donor sum clamped to zero.
+// donor sum clamped to zero.  A donor outside the catchment adds nothing, and
+// the accumulation of a cell starts at its weight.
 struct FaCell {
-    const uint8_t* mask;
-    const uint8_t* fd;
-    const float* w;
     const float* prop;
     float2* fa;
     int32_t* contrib;
     DemCtx dc;
-    int W, H;
-    __device__ __forceinline__ void cell(int32_t cur, int x, int y) const {
-        if (dc.of) atomicAdd(&dc.out[dc.of[cur]].fa_done, 1);  // a batch: count per DEM
-        float2 acc = make_float2(0.f, 0.f);
-        int32_t cacc = 1;
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-            const int d = scan_dir(kk);
-            const int nx = x + dir_dx(d), ny = y + dir_dy(d);
-            if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
-            const int32_t n = ny * W + nx;
-            if (!donates(__ldg(fd + n), d)) continue;
+    int W;
+    struct Part {
+        float2 v;  // the donor's accumulation, its share taken
+        int32_t cnt;
+    };
+    __device__ __forceinline__ Part donor(int32_t cur, int kk, bool on) const {
+        Part part{make_float2(0.f, 0.f), 0};
+        const int d = scan_dir(kk);
+        const int32_t n = cur + grid_step(d, W);
+        if (on) {
+            const float p = prop ? __ldg(prop + 8 * (size_t)n + ((d + 4) & 7)) : 1.0f;
             const float2 v = __ldcg(fa + n);
-            const float p = prop_of(prop, mask, n, (d + 4) & 7);
-            acc = ff_add(acc, p == 1.0f ? v : ff_scale(v, p));
-            if (contrib && __ldg(mask + n)) cacc += __ldcg(contrib + n);
+            part.v = p == 1.0f ? v : ff_scale(v, p);
+            if (contrib) part.cnt = __ldcg(contrib + n);
+        }
+        return part;
+    }
+    __device__ __forceinline__ void cell(int32_t cur, uint32_t donors, Part part) const {
+        const float2 w = __ldcg(fa + cur);
+        float2 acc = make_float2(0.f, 0.f);
+        for (uint32_t m = donors; m; m &= m - 1) {
+            const int k = __ffs(m) - 1;
+            acc = ff_add(acc, make_float2(__shfl_sync(0xffffffffu, part.v.x, k), __shfl_sync(0xffffffffu, part.v.y, k)));
         }
         if (acc.x < 0.0f) acc = make_float2(0.f, 0.f);
-        __stcg(fa + cur, ff_add(make_float2(__ldg(w + cur), 0.f), acc));
-        if (contrib) __stcg(contrib + cur, cacc);
-    }
-    __device__ __forceinline__ int receivers(int32_t cur, int x, int y, int32_t* r) const {
-        return code_receivers(fd, mask, cur, x, y, W, H, r);
+        const int cnt = contrib ? wsum(part.cnt) : 0;
+        if ((threadIdx.x & 31) == 0) {
+            __stcg(fa + cur, ff_add(w, acc));
+            if (contrib) __stcg(contrib + cur, 1 + cnt);
+            if (dc.of) atomicAdd(&dc.out[dc.of[cur]].fa_done, 1);  // a batch: count per DEM
+        }
     }
 };
 
-// The accumulation wave: every source starts it; cells follow as their last
-// donor finishes.  With gate set it runs only when the tiled path is off.
-__global__ void k_fa_walk(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
-                          const float* __restrict__ w, const float* __restrict__ prop, float2* fa, int32_t* pending,
-                          int32_t* contrib, int32_t* list_a, int32_t* list_b, ModelConsts k, DevScalars* sc,
-                          DemCtx dc, int gate) {
+// The general accumulation wave.  With gate set it runs only when the tiled
+// path is off.
+__global__ void __launch_bounds__(256, 4)
+    k_fa_walk(const float* __restrict__ prop, float2* fa, int32_t* word, int32_t* contrib, int32_t* list,
+              ModelConsts k, DevScalars* sc, DemCtx dc, int gate) {
     if (gate && sc->tiled_ok) return;  // the tiled kernels did this step
-    const FaCell op{mask, fd, w, prop, fa, contrib, dc, k.W, k.H};
-    int done = wave_walk(op, pending, list_a, list_b, k.W, k.H, sc);
+    const FaCell op{prop, fa, contrib, dc, k.W};
+    int done = wave_walk(op, word, list, k.W, k.H, sc);
     done = wsum(done);
     if (!dc.of && (threadIdx.x & 31) == 0 && done) atomicAdd(&dc.out[0].fa_done, done);
 }
@@ -1008,22 +1015,17 @@ lem_status launch_flow_accumulation(const DevState& s, const ModelConsts& k, uin
                    s.f_ds, s.t_fcnt, k, s.sc, s.dems, ts);
     }
     {
-        const uint8_t* mask = s.mask;
-        const uint8_t* fd = s.fd;
-        const float* w = s.w;
         float2* fa = s.fa;
-        int32_t* pending = s.pending;
-        int32_t* la = s.list_a;
-        int32_t* lb = s.list_b;
+        int32_t* word = s.pending;
+        int32_t* list = s.list_a;
         ModelConsts kk = k;
         DevScalars* sc = s.sc;
         DemCtx dc = s.dems;
         int gate = tiled;
-        void* args[] = {(void*)&mask,    (void*)&fd, (void*)&w,  (void*)&prop, (void*)&fa,  (void*)&pending,
-                        (void*)&contrib, (void*)&la, (void*)&lb, (void*)&kk,   (void*)&sc,  (void*)&dc,
-                        (void*)&gate};
+        void* args[] = {(void*)&prop, (void*)&fa, (void*)&word, (void*)&contrib, (void*)&list,
+                        (void*)&kk,   (void*)&sc, (void*)&dc,   (void*)&gate};
         L.pre("k_fa_walk");
-        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, s.coop_blocks[kCkFaWalk], args, L.st));
+        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, walk_blocks(s.coop_blocks[kCkFaWalk], N), args, L.st));
         L.post();
     }
     if (flags & LEM_STEP_SET_OUTLET_FROM_FA) {  // some DEM moves its outlet this step
@@ -1044,13 +1046,9 @@ constexpr size_t kNaCells = LEM_NOALLOC_MAX_CELLS;
 constexpr size_t kNaHead = 1024;  // DevScalars and one DemOut, rounded up
 constexpr size_t kNaOffDem = 512;
 static_assert(sizeof(DevScalars) <= kNaOffDem && kNaOffDem + sizeof(DemOut) <= kNaHead, "scalar block");
-constexpr size_t kNaOffCode = kNaHead;
-constexpr size_t kNaOffMask = kNaOffCode + kNaCells;
-constexpr size_t kNaOffPend = kNaOffMask + kNaCells;          // int32
-constexpr size_t kNaOffListA = kNaOffPend + 4 * kNaCells;     // int32
-constexpr size_t kNaOffListB = kNaOffListA + 4 * kNaCells;    // int32
-constexpr size_t kNaOffW = kNaOffListB + 4 * kNaCells;        // float
-constexpr size_t kNaOffFa = kNaOffW + 4 * kNaCells;           // float2
+constexpr size_t kNaOffWord = kNaHead;                        // int32
+constexpr size_t kNaOffList = kNaOffWord + 4 * kNaCells;      // int32
+constexpr size_t kNaOffFa = kNaOffList + 4 * kNaCells;        // float2
 constexpr size_t kNaBytes = kNaOffFa + 8 * kNaCells;
 
 // Scratch of the no-allocation entry point (every call shares it).
@@ -1071,11 +1069,10 @@ __global__ void k_na_reset(DevScalars* sc, DemOut* dem) {
     sc->err_first = 0;
 }
 
-// Codes, mask, weights, initial accumulation and in-degrees from the caller's
-// int32 codes and DEM (cells at -9999 are outside and complete with zero flow).
+// Initial accumulation (the weight) and the wave's words from the caller's int32
+// codes and DEM (cells at -9999 are outside and complete with zero flow).
 __global__ void k_na_prep(const int32_t* __restrict__ fd_in, const double* __restrict__ w_in,
-                          const double* __restrict__ dem, uint8_t* __restrict__ code, uint8_t* __restrict__ mask,
-                          float* __restrict__ w, float2* __restrict__ fa, int32_t* __restrict__ pending,
+                          const double* __restrict__ dem, float2* __restrict__ fa, int32_t* __restrict__ word,
                           int32_t* ready, int W, int H, DevScalars* sc, DemOut* dem_out) {
     const size_t N = (size_t)W * H;
     for (size_t base = (size_t)blockIdx.x * blockDim.x; base < N; base += (size_t)gridDim.x * blockDim.x) {
@@ -1084,19 +1081,23 @@ __global__ void k_na_prep(const int32_t* __restrict__ fd_in, const double* __res
         if (i < N) {
             const int x = (int)(i % W), y = (int)(i / W);
             const bool in = dem[i] != kNoData;
-            code[i] = (uint8_t)(fd_in[i] & 0xff);
-            mask[i] = in ? 1 : 0;
-            const float wi = (float)w_in[i];
-            w[i] = wi;
-            fa[i] = make_float2(in ? wi : 0.0f, 0.0f);
+            const uint32_t code = (uint32_t)(fd_in[i] & 0xff);
+            fa[i] = make_float2(in ? (float)w_in[i] : 0.0f, 0.0f);
             int32_t pend = in ? 0 : kBlocked;
-            for (int d = 0; in && d < 8; ++d) {
+            uint32_t donors = 0, receivers = 0;
+#pragma unroll
+            for (int d = 0; d < 8; ++d) {
                 const int nx = x + dir_dx(d), ny = y + dir_dy(d);
-                if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
+                if (!in || nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
                 const size_t n = (size_t)ny * W + nx;
-                if (donates((uint8_t)(fd_in[n] & 0xff), d) && dem[n] != kNoData) ++pend;
+                if (dem[n] == kNoData) continue;
+                receivers |= code & dir_bit(d);
+                if (donates((uint8_t)(fd_in[n] & 0xff), d)) {
+                    ++pend;
+                    donors |= 1u << scan_index(d);
+                }
             }
-            pending[i] = pend;
+            word[i] = wave_word(pend, donors, receivers);
             src = in && pend == 0;
             act = in;
         }
@@ -1148,22 +1149,15 @@ extern "C" lem_status lem_accumulate_flow_noalloc(const int32_t* d_fd, const dou
     }
     DevScalars* sc = reinterpret_cast<DevScalars*>(nd.base);
     DemOut* dem = reinterpret_cast<DemOut*>(nd.base + kNaOffDem);
-    uint8_t* code = nd.base + kNaOffCode;
-    uint8_t* mask = nd.base + kNaOffMask;
-    int32_t* pending = reinterpret_cast<int32_t*>(nd.base + kNaOffPend);
-    int32_t* la = reinterpret_cast<int32_t*>(nd.base + kNaOffListA);
-    int32_t* lb = reinterpret_cast<int32_t*>(nd.base + kNaOffListB);
-    float* w = reinterpret_cast<float*>(nd.base + kNaOffW);
+    int32_t* word = reinterpret_cast<int32_t*>(nd.base + kNaOffWord);
+    int32_t* list = reinterpret_cast<int32_t*>(nd.base + kNaOffList);
     float2* fa = reinterpret_cast<float2*>(nd.base + kNaOffFa);
     const int T = 256;
     const int blocks = (int)std::min<size_t>((N + T - 1) / T, 152 * 32);
     k_na_reset<<<1, 1, 0, st>>>(sc, dem);  // the array keeps the previous call's contents
-    k_na_prep<<<blocks, T, 0, st>>>(d_fd, d_weight, d_dem, code, mask, w, fa, pending, la, width, height, sc, dem);
+    k_na_prep<<<blocks, T, 0, st>>>(d_fd, d_weight, d_dem, fa, word, list, width, height, sc, dem);
     LEM_CUDA_TRY(cudaGetLastError());
     {
-        const uint8_t* m = mask;
-        const uint8_t* c = code;
-        const float* ww = w;
         const float* prop = nullptr;
         int32_t* contrib = nullptr;
         ModelConsts k{};
@@ -1171,9 +1165,9 @@ extern "C" lem_status lem_accumulate_flow_noalloc(const int32_t* d_fd, const dou
         k.H = height;
         int gate = 0;
         DemCtx dc{nullptr, nullptr, dem, 1};
-        void* args[] = {(void*)&m, (void*)&c, (void*)&ww, (void*)&prop, (void*)&fa, (void*)&pending,
-                        (void*)&contrib, (void*)&la, (void*)&lb, (void*)&k, (void*)&sc, (void*)&dc, (void*)&gate};
-        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, nd.blocks, args, st));
+        void* args[] = {(void*)&prop, (void*)&fa, (void*)&word, (void*)&contrib, (void*)&list,
+                        (void*)&k,    (void*)&sc, (void*)&dc,   (void*)&gate};
+        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, walk_blocks(nd.blocks, N), args, st));
     }
     k_na_out<<<blocks, T, 0, st>>>(fa, d_fa, N);
     LEM_CUDA_TRY(cudaGetLastError());

@@ -201,46 +201,6 @@ __global__ void __launch_bounds__(256, 5)
     }
 }
 
-// In-degrees and sources of the global sediment wave, for the steps that take
-// it (MFD, or a multi-direction code found by k_erosion): cells in row 0 or
-// column 0 are never processed (mfd_accum.cu:42) and masked cells never
-// complete, so a donor of either kind blocks its receiver for good.
-__global__ void k_sed_prep(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
-                           float* __restrict__ depo, int32_t* __restrict__ pending, int32_t* ready, ModelConsts k,
-                           DevScalars* sc, TileSet ts) {
-    if (sc->sed_tiled_ok) return;  // the tiled path routes this step
-    const int W = k.W, H = k.H;
-    const size_t N = (size_t)W * H;
-    for (size_t base = (size_t)blockIdx.x * blockDim.x; base < ts.span(); base += (size_t)gridDim.x * blockDim.x) {
-        int x, y;
-        const bool in = ts.cell(base + threadIdx.x, W, H, x, y);
-        const size_t i = (size_t)y * W + x;
-        bool src = false;
-        if (in) {
-            int32_t pend = kBlocked;
-            if (mask[i]) {
-                if (x != 0 && y != 0) {
-                    pend = 0;
-#pragma unroll
-                    for (int d = 0; d < 8; ++d) {
-                        const int nx = x + dir_dx(d), ny = y + dir_dy(d);
-                        if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
-                        const size_t n = (size_t)ny * W + nx;
-                        if (!donates(fd[n], d)) continue;
-                        if (mask[n] && nx != 0 && ny != 0)
-                            ++pend;
-                        else
-                            pend |= kBlocked;
-                    }
-                    src = (pend == 0);
-                }
-            }
-            pending[i] = pend;
-        }
-        wave_append(src, (int32_t)i, ready, &sc->counters[0], (int)N, &sc->err);
-    }
-}
-
 // The per-cell arithmetic of MFDsedbud (mfd_accum.cu:222-249), rounded the same
 // way wherever it is evaluated (no contraction): deposition, the stone mix
 // coefficients (stone = A + B * from, clamped, when the sediment column is not
@@ -284,58 +244,113 @@ __device__ __forceinline__ void sed_store(size_t g, const SedLocal& L, float sn,
     soilT[g] = L.stn;
 }
 
-// One cell of MFDsedbud (mfd_accum.cu:32-254): deposition from the donors'
-// erosion, stone mixing with the donors' updated stone, new soil thickness.
+// Words and sources of the general sediment wave, for the steps that take it
+// (MFD, or a multi-direction code found by k_erosion): cells in row 0 or column
+// 0 are never processed (mfd_accum.cu:42) and masked cells never complete, so a
+// donor of either kind blocks its receiver for good.  Only the stone mix waits
+// on the donors: every other part of a cell (MFDsedbud, mfd_accum.cu:32-254:
+// deposition from the donors' erosion, new soil thickness, mix coefficients) is
+// computed here.
+__global__ void k_sed_prep(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
+                           const float* __restrict__ prop, const float* __restrict__ ero,
+                           const float* __restrict__ inci, const float* __restrict__ geli,
+                           const float* __restrict__ stone, const float* __restrict__ soilT, float4* __restrict__ coef,
+                           uint8_t* __restrict__ nonzero, int32_t* __restrict__ word, int32_t* ready, ModelConsts k,
+                           DevScalars* sc, TileSet ts) {
+    if (sc->sed_tiled_ok) return;  // the tiled path routes this step
+    const int W = k.W, H = k.H;
+    const size_t N = (size_t)W * H;
+    const float omd = 1.0f - k.ddk, omc = 1.0f - k.dck, omg = 1.0f - k.dgk;
+    for (size_t base = (size_t)blockIdx.x * blockDim.x; base < ts.span(); base += (size_t)gridDim.x * blockDim.x) {
+        int x, y;
+        const bool in = ts.cell(base + threadIdx.x, W, H, x, y);
+        const size_t i = (size_t)y * W + x;
+        bool src = false;
+        if (in) {
+            int32_t pend = kBlocked;
+            uint32_t donors = 0, receivers = 0;
+            if (mask[i] && x != 0 && y != 0) {
+                pend = 0;
+                const uint8_t code = fd[i];
+                float ad = 0.f, ac = 0.f, ag = 0.f;
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk) {
+                    const int d = scan_dir(kk);
+                    const int nx = x + dir_dx(d), ny = y + dir_dy(d);
+                    if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
+                    const size_t n = (size_t)ny * W + nx;
+                    const bool live = mask[n] && nx != 0 && ny != 0;
+                    if (live) receivers |= code & dir_bit(d);
+                    if (!donates(fd[n], d)) continue;
+                    if (live) {
+                        ++pend;
+                        donors |= 1u << kk;
+                    } else {
+                        pend |= kBlocked;
+                    }
+                    const float p = prop ? __ldg(prop + 8 * n + ((d + 4) & 7)) : 1.0f;
+                    ad = __fadd_rn(ad, __fmul_rn(p, __fmul_rn(__ldg(ero + n), omd)));
+                    ac = __fadd_rn(ac, __fmul_rn(p, __fmul_rn(__ldg(inci + n), omc)));
+                    ag = __fadd_rn(ag, __fmul_rn(p, __fmul_rn(__ldg(geli + n), omg)));
+                }
+                const SedLocal L = sed_local(ad, ac, ag, __ldg(ero + i), __ldg(inci + i), __ldg(geli + i), soilT[i],
+                                             stone[i], k.ddk, k.dck, k.dgk);
+                coef[i] = make_float4(L.A, L.B, L.dep, L.stn);
+                nonzero[i] = L.nz;
+                src = (pend == 0);
+            }
+            word[i] = wave_word(pend, donors, receivers);
+        }
+        wave_append(src, (int32_t)i, ready, &sc->counters[0], (int)N, &sc->err);
+    }
+}
+
+// A cell of the general sediment wave: its stone mixed with the donors' updated
+// stone, by the coefficients of k_sed_prep.
 struct SedCell {
-    const uint8_t* mask;
-    const uint8_t* fd;
     const float* prop;
-    const float* ero;
-    const float* inci;
-    const float* geli;
+    const float4* coef;
+    const uint8_t* nonzero;
     float* depo;
     float* stone;
     float* fines;
     float* soilT;
     DemCtx dc;
-    int W, H;
-    float ddk, dck, dgk;
-    __device__ __forceinline__ void cell(int32_t cur, int x, int y) const {
-        if (dc.of) atomicAdd(&dc.out[dc.of[cur]].sed_done, 1);  // a batch: count per DEM
-        const float omd = 1.0f - ddk, omc = 1.0f - dck, omg = 1.0f - dgk;
-        float ad = 0.f, ac = 0.f, ag = 0.f, from = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-            const int d = scan_dir(kk);
-            const int nx = x + dir_dx(d), ny = y + dir_dy(d);
-            if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
-            const int32_t n = ny * W + nx;
-            if (!donates(__ldg(fd + n), d)) continue;
-            const float p = prop ? __ldg(prop + 8 * (size_t)n + ((d + 4) & 7)) : 1.0f;
-            ad = __fadd_rn(ad, __fmul_rn(p, __fmul_rn(__ldg(ero + n), omd)));
-            ac = __fadd_rn(ac, __fmul_rn(p, __fmul_rn(__ldg(inci + n), omc)));
-            ag = __fadd_rn(ag, __fmul_rn(p, __fmul_rn(__ldg(geli + n), omg)));
-            from = __fadd_rn(from, __fmul_rn(p, __ldcg(stone + n)));
-        }
-        const SedLocal L = sed_local(ad, ac, ag, __ldg(ero + cur), __ldg(inci + cur), __ldg(geli + cur), soilT[cur],
-                                     __ldcg(stone + cur), ddk, dck, dgk);
-        sed_store(cur, L, L.nz ? sed_mix(L.A, L.B, from) : 0.0f, depo, stone, fines, soilT);
+    int W;
+    __device__ __forceinline__ float donor(int32_t cur, int kk, bool on) const {
+        const int d = scan_dir(kk);
+        const int32_t n = cur + grid_step(d, W);
+        if (!on) return 0.f;
+        const float p = prop ? __ldg(prop + 8 * (size_t)n + ((d + 4) & 7)) : 1.0f;
+        return __fmul_rn(p, __ldcg(stone + n));
     }
-    __device__ __forceinline__ int receivers(int32_t cur, int x, int y, int32_t* r) const {
-        return code_receivers(fd, mask, cur, x, y, W, H, r);
+    __device__ __forceinline__ void cell(int32_t cur, uint32_t donors, float part) const {
+        const float4 c = __ldg(coef + cur);
+        SedLocal L;
+        L.A = c.x;
+        L.B = c.y;
+        L.dep = c.z;
+        L.stn = c.w;
+        L.nz = __ldg(nonzero + cur) != 0;
+        float from = 0.f;
+        for (uint32_t m = donors; m; m &= m - 1)
+            from = __fadd_rn(from, __shfl_sync(0xffffffffu, part, __ffs(m) - 1));
+        if ((threadIdx.x & 31) == 0) {
+            sed_store(cur, L, L.nz ? sed_mix(L.A, L.B, from) : 0.0f, depo, stone, fines, soilT);
+            if (dc.of) atomicAdd(&dc.out[dc.of[cur]].sed_done, 1);  // a batch: count per DEM
+        }
     }
 };
 
-// The sediment wave: every source starts it; cells follow as their last donor
-// finishes.  With gate set it runs only when the tiled path is off.
-__global__ void k_sed_walk(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
-                           const float* __restrict__ prop, const float* __restrict__ ero,
-                           const float* __restrict__ inci, const float* __restrict__ geli, float* depo, float* stone,
-                           float* fines, float* soilT, int32_t* pending, int32_t* list_a, int32_t* list_b,
-                           ModelConsts k, DevScalars* sc, DemCtx dc, int gate) {
+// The general sediment wave.  With gate set it runs only when the tiled path is
+// off.
+__global__ void __launch_bounds__(256, 4)
+    k_sed_walk(const float* __restrict__ prop, const float4* __restrict__ coef, const uint8_t* __restrict__ nonzero,
+               float* depo, float* stone, float* fines, float* soilT, int32_t* word, int32_t* list, ModelConsts k,
+               DevScalars* sc, DemCtx dc, int gate) {
     if (gate && sc->sed_tiled_ok) return;
-    const SedCell op{mask, fd, prop, ero, inci, geli, depo, stone, fines, soilT, dc, k.W, k.H, k.ddk, k.dck, k.dgk};
-    int done = wave_walk(op, pending, list_a, list_b, k.W, k.H, sc);
+    const SedCell op{prop, coef, nonzero, depo, stone, fines, soilT, dc, k.W};
+    int done = wave_walk(op, word, list, k.W, k.H, sc);
     done = wsum(done);
     if (!dc.of && (threadIdx.x & 31) == 0 && done) atomicAdd(&dc.out[0].sed_done, done);
 }
@@ -1570,8 +1585,8 @@ lem_status launch_erosion(const DevState& s, const ModelConsts& k, uint32_t flag
     const TileSet ts = tiles_of(s, k.W);
     {
         const size_t vb = (ts.span() + T - 1) / T;
-        LEM_LAUNCH(L, k_sed_prep, (int)(vb > 152 * 32 ? 152 * 32 : vb), T, s.mask, s.fd, s.depo, s.pending, s.list_a,
-                   k, s.sc, ts);
+        LEM_LAUNCH(L, k_sed_prep, (int)(vb > 152 * 32 ? 152 * 32 : vb), T, s.mask, s.fd, prop, s.ero, s.inci, s.geli,
+                   s.stone, s.soilT, s.p_abc, s.t_stat, s.pending, s.list_a, k, s.sc, ts);
     }
     if (tiled) {
         const int tiles = ts.n;
@@ -1606,28 +1621,23 @@ lem_status launch_erosion(const DevState& s, const ModelConsts& k, uint32_t flag
                    ts);
     }
     {
-        const uint8_t* mask = s.mask;
-        const uint8_t* fd = s.fd;
-        const float* ero = s.ero;
-        const float* inci = s.inci;
-        const float* geli = s.geli;
+        const float4* coef = s.p_abc;  // per cell (a tile has kTile * kTile of them)
+        const uint8_t* nonzero = s.t_stat;
         float* depo = s.depo;
         float* stone = s.stone;
         float* fines = s.fines;
         float* soilT = s.soilT;
-        int32_t* pending = s.pending;
-        int32_t* la = s.list_a;
-        int32_t* lb = s.list_b;
+        int32_t* word = s.pending;
+        int32_t* list = s.list_a;
         ModelConsts kk = k;
         DevScalars* sc = s.sc;
         DemCtx dc = s.dems;
         int gate = tiled;
-        void* args[] = {(void*)&mask, (void*)&fd,    (void*)&prop,  (void*)&ero,     (void*)&inci,
-                        (void*)&geli, (void*)&depo,  (void*)&stone, (void*)&fines,   (void*)&soilT,
-                        (void*)&pending, (void*)&la, (void*)&lb,    (void*)&kk,      (void*)&sc, (void*)&dc,
-                        (void*)&gate};
+        void* args[] = {(void*)&prop, (void*)&coef, (void*)&nonzero, (void*)&depo, (void*)&stone, (void*)&fines, (void*)&soilT,
+                        (void*)&word, (void*)&list, (void*)&kk,      (void*)&sc,   (void*)&dc,    (void*)&gate};
         L.pre("k_sed_walk");
-        LEM_CUDA_TRY(coop_launch((const void*)k_sed_walk, s.coop_blocks[kCkSedWalk], args, L.st));
+        LEM_CUDA_TRY(coop_launch((const void*)k_sed_walk, walk_blocks(s.coop_blocks[kCkSedWalk], (size_t)k.W * k.H), args,
+                                 L.st));
         L.post();
     }
     const bool diag = (flags & LEM_STEP_KEEP_DIAGNOSTICS) != 0;

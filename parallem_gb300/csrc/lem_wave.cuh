@@ -69,105 +69,116 @@ __device__ __forceinline__ int32_t dec_acq_rel(int32_t* p) {
     return old;
 }
 
-constexpr int kWaveStack = 8;      // receivers a lane keeps for itself before spilling to the next round
+// The general dependency wave (several receivers, contributing counts, steps the
+// tiled waves cannot take), run by every thread of a cooperative launch.  Each
+// cell's word counts its donors still to come in the low four bits (kBlocked:
+// one never comes), and carries its donors that take part (bit k: direction
+// scan_dir(k)) and its receivers that do (bits of its code), so that lowering a
+// receiver's count brings all that is needed to go on with it.
+//
+// The ready cells stand in one list in which every cell appears once.  A warp
+// without a cell holds a ticket, a place of the list, and watches it; a warp
+// that finishes a cell lowers its receivers' counts, goes on with the first that
+// became ready and appends the others, so a front spreads over all warps however
+// few cells start ready.  inflight counts the cells ready and unfinished; the
+// wave ends when it is 0.
+//
+// Bound by the chain of cells on the longest path: the last donor's release, the
+// donors' values and the sum in order.  A warp takes one cell at a time, so no
+// cell waits for another's turn (a lane per cell: 1.4 times as long), a lane
+// reads each donor and lowers each receiver's count.  When each lane walked cells
+// of its own and kept the ones it made ready, a smooth slope with few sources
+// ran on as many lanes: 5 us a cell over all cells.
+constexpr int32_t kWordReady = kBlocked | 15;  // the bits that are 0 in a ready cell's word
+__device__ __forceinline__ int32_t wave_word(int count_and_block, uint32_t donors, uint32_t receivers) {
+    return count_and_block | (int32_t)(donors << 8) | (int32_t)(receivers << 16);
+}
+constexpr int kWaveSpin = 1 << 26;  // polls of an idle warp before it gives up
 
-// The dependency wave shared by flow accumulation and sediment routing, run by
-// every thread of a cooperative launch.  A cell is ready once all its donors
-// are finished (pending[c] counts them; kBlocked marks a donor that never
-// finishes).  Lanes take ready cells from the round's list through one atomic
-// head per warp request, so no lane idles while work is left.  A lane that
-// finishes a cell decrements its receivers and carries on with the first one
-// it made ready (it was that cell's last donor); further receivers made ready
-// at the same time (MFD) go on the lane's own stack, and only when that is full
-// to the next round's list.  Op::cell(c, x, y) computes and stores cell c,
-// reading finished donors with ld.global.cg; Op::receivers(c, x, y, r) lists
-// the nodes whose pending count c's completion decrements.  Returns the nodes
-// this thread finished.
+// index step of direction d in a grid of width W
+__device__ __forceinline__ int32_t grid_step(int d, int W) { return dir_dy(d) * W + dir_dx(d); }
+
+// Op::donor(c, k, on) is called by every lane: lane k < 8 with its bit of the
+// donors set (on) reads its donor's part; Op::cell(c, donors, part) combines the
+// parts in scan order and stores cell c from lane 0.  The list starts with
+// counters[0] cells.  Returns the cells this warp finished, in lane 0.
 template <class Op>
-__device__ int wave_walk(const Op& op, int32_t* pending, int32_t* list_a, int32_t* list_b, int W, int H,
-                         DevScalars* sc) {
+__device__ int wave_walk(const Op& op, int32_t* word, int32_t* list, int W, int H, DevScalars* sc) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    const size_t N = (size_t)W * H;
+    const int32_t N = W * H;
     const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t gstride = (size_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    int32_t* cnt = sc->counters;  // [0..2] list sizes by round % 3, [3..5] take heads by round % 3
+    int32_t* const tail = &sc->counters[0];
+    int32_t* const head = &sc->counters[1];
+    int32_t* const inflight = &sc->counters[2];
+    int32_t* const stop = &sc->counters[3];
+    const int nin = *tail;
+    if (nin == 0) return 0;  // the same in every thread
+    for (size_t i = nin + gtid; i < (size_t)N; i += gstride) list[i] = -1;
     if (gtid == 0) {
-        cnt[1] = cnt[2] = 0;
-        cnt[3] = cnt[4] = cnt[5] = 0;
+        *head = *stop = 0;
+        *inflight = nin;
     }
     grid.sync();
+    const int b = lane & 7;  // a lane's receiver: bit b of the code
+    const int32_t to = grid_step((b + 2) & 7, W);
     int done = 0;
-    for (int round = 0;; ++round) {
-        const int32_t* in = (round & 1) ? list_b : list_a;
-        int32_t* out = (round & 1) ? list_a : list_b;
-        const int nin = *((volatile int32_t*)&cnt[round % 3]);
-        if (nin == 0) break;
-        if (round >= round_cap_of(sc)) {
-            if (gtid == 0) raise_error(&sc->err, ErrFlags::kNoConverge);
-            break;
-        }
-        if (gtid == 0) {
-            cnt[(round + 2) % 3] = 0;      // size of the list after next (read before the last sync)
-            cnt[3 + (round + 1) % 3] = 0;  // head of the next round
-        }
-        int32_t* head = &cnt[3 + round % 3];
-        int32_t stack[kWaveStack];
-        int sp = 0;
+    for (;;) {
+        int32_t ticket = 0;
+        if (lane == 0) ticket = atomicAdd(head, 1);
+        ticket = __shfl_sync(0xffffffffu, ticket, 0);
         int32_t cur = -1;
-        bool more = true;  // warp-uniform: the round's list may still hold cells
-        for (size_t guard = 0;; ++guard) {
-            if (cur < 0 && sp > 0) cur = stack[--sp];
-            const bool need = cur < 0;
-            const unsigned m = __ballot_sync(0xffffffffu, need && more);
-            if (m) {
-                const int leader = __ffs(m) - 1;
-                int base = 0;
-                if (lane == leader) base = atomicAdd(head, __popc(m));
-                base = __shfl_sync(0xffffffffu, base, leader);
-                if (need) {
-                    const int it = base + __popc(m & below);
-                    if (it < nin) cur = __ldcg(in + it);
+        for (int spin = 0;; ++spin) {
+            if (lane == 0 && ticket < N) cur = *((volatile int32_t*)(list + ticket));
+            cur = __shfl_sync(0xffffffffu, cur, 0);
+            if (cur >= 0) break;
+            int end = 0;
+            if (lane == 0 && (spin & 15) == 15) {  // seldom: every waiting warp reads this one word
+                end = *((volatile int32_t*)inflight) == 0 || *((volatile int32_t*)stop);
+                if (!end && spin > kWaveSpin) {
+                    raise_error(&sc->err, ErrFlags::kNoConverge);
+                    atomicExch(stop, 1);
+                    end = 1;
                 }
-                if (base + __popc(m) >= nin) more = false;
             }
-            if (!__any_sync(0xffffffffu, cur >= 0)) break;
-            if (guard > 2 * N + 64) {  // every cell is finished at most once
-                if (lane == 0) raise_error(&sc->err, ErrFlags::kNoConverge);
-                break;
-            }
-            int32_t spill[8];
-            int nspill = 0;
-            if (cur >= 0) {
-                const int x = cur % W, y = cur / W;
-                // the receivers first: they read static data only, so their
-                // loads overlap the cell's own chain of loads
-                int32_t rcv[8];
-                const int nr = op.receivers(cur, x, y, rcv);
-                op.cell(cur, x, y);
-                ++done;
-                int32_t next = -1;
-                for (int j = 0; j < nr; ++j) {
-                    const int32_t r = rcv[j];
-                    if (dec_acq_rel(pending + r) == 1) {
-                        if (next < 0)
-                            next = r;
-                        else if (sp < kWaveStack)
-                            stack[sp++] = r;
-                        else
-                            spill[nspill++] = r;
-                    }
-                }
-                cur = next;
-            }
-            if (__any_sync(0xffffffffu, nspill > 0))
-                for (int j = 0; j < 8; ++j)
-                    wave_append(j < nspill, j < nspill ? spill[j] : 0, out, &cnt[(round + 1) % 3], (int)N, &sc->err);
+            if (__shfl_sync(0xffffffffu, end, 0)) break;
+            __nanosleep(32);
         }
-        grid.sync();
+        if (cur < 0) break;
+        __threadfence();  // the donors' values, after the cell
+        int32_t info = __ldcg(word + cur);
+        while (cur >= 0) {
+            const uint32_t donors = (uint32_t)(info >> 8) & 255u;
+            op.cell(cur, donors, op.donor(cur, b, lane < 8 && ((donors >> b) & 1u)));
+            ++done;
+            __syncwarp();
+            __threadfence();  // the finished cell, before its receivers' counts
+            const bool on = lane < 8 && ((info >> (16 + b)) & 1);
+            int32_t old = 0;
+            if (on) old = atomicSub(word + cur + to, 1);
+            const unsigned rdy = __ballot_sync(0xffffffffu, on && (old & kWordReady) == 1);
+            __threadfence();  // the other donors' values, after the counts
+            if (!rdy) break;
+            const int first = __ffs(rdy) - 1, rest = __popc(rdy) - 1;
+            if (rest) {
+                int base = 0;
+                if (lane == 0) {
+                    atomicAdd(inflight, rest);
+                    base = atomicAdd(tail, rest);
+                    __threadfence();
+                }
+                base = __shfl_sync(0xffffffffu, base, 0);
+                if (((rdy >> lane) & 1u) && lane != first)
+                    *((volatile int32_t*)(list + base + __popc(rdy & ((1u << lane) - 1u)) - 1)) = cur + to;
+            }
+            cur += grid_step((first + 2) & 7, W);
+            info = __shfl_sync(0xffffffffu, old, first);
+        }
+        if (lane == 0) atomicSub(inflight, 1);
     }
-    return done;
+    return lane == 0 ? done : 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -295,21 +306,6 @@ __device__ __forceinline__ void tile_wave(const Op& op, int32_t* s_pend, int16_t
         if (threadIdx.x == 0) *s_qn = qn;
     }
     __syncthreads();
-}
-
-// Receivers of cell (x, y) by its direction code: in-grid, in-catchment cells.
-__device__ __forceinline__ int code_receivers(const uint8_t* __restrict__ fd, const uint8_t* __restrict__ mask,
-                                              int32_t cur, int x, int y, int W, int H, int32_t* r) {
-    const uint8_t code = __ldg(fd + cur);
-    int nr = 0;
-    for (int d = 0; d < 8; ++d) {
-        if (!(code & dir_bit(d))) continue;
-        const int rx = x + dir_dx(d), ry = y + dir_dy(d);
-        if (rx < 0 || rx >= W || ry < 0 || ry >= H) continue;
-        const int32_t n = ry * W + rx;
-        if (__ldg(mask + n)) r[nr++] = n;
-    }
-    return nr;
 }
 
 }  // namespace lem

@@ -1,0 +1,88 @@
+"""The tile waves at the sizes where their tables end, against the FP64 oracle.
+
+* Coarse waves: a comb of trunk channels whose tiles give one outlet a program
+  of fewer than 32, of 32 to 64 and of more than 64 nodes, with more inputs than
+  a warp gathers at once.
+* The general wave (several receivers, the stateless accumulation): slopes on
+  which few cells start ready, on grids of a few cells and of many blocks.
+* Spill heights: boundaries that tie, on few edges (one block) and on many.
+
+The tolerances are those of tests/test_gpu_parity.py.
+"""
+import numpy as np
+import pytest
+
+from parallem_gb300 import scenario as S
+from tests.helpers import NODATA, ringed
+from tests.test_gpu_parity import libs, run_steps  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def comb(h, w, spacing):
+    """Trunk channels flowing south every `spacing` columns, fed row by row from both sides."""
+    y, x = np.mgrid[0:h, 0:w]
+    off = np.abs((x + 5) % spacing - spacing // 2)
+    z = 900.0 - 0.3 * y + 1.0 * off + 1e-3 * np.random.default_rng(3).random((h, w))
+    return ringed(z, 2)
+
+
+@pytest.mark.parametrize("spacing", [8, 32, 64, 200])
+def test_programs_of_every_size_class(libs, spacing):
+    run_steps(libs, comb(150, 170, spacing), 2, np.full(2, 900.0), np.full(2, 9.0), False)
+
+
+def tilted(h, w, dy, dx):
+    """A plane with a gentle undulation: no pits, few sources, several receivers per cell."""
+    y, x = np.mgrid[0:h, 0:w]
+    z = 500.0 + dy * y + dx * x + 3.0 * np.sin(x / 17.0) * np.cos(y / 23.0)
+    return ringed(z, 2)
+
+
+@pytest.mark.parametrize("shape,slope", [((30, 30), (1.0, 0.7)), ((97, 65), (-1.0, 1.2)), ((64, 131), (0.8, -1.0))])
+@pytest.mark.parametrize("props", [0, 1])
+def test_general_wave_with_several_receivers(libs, shape, slope, props):
+    if props == 0 and max(shape) > 30:
+        pytest.skip("every receiver takes the whole flow: it overflows on long paths")
+    run_steps(libs, tilted(*shape, *slope), 1, np.full(1, 900.0), np.full(1, 9.0), False,
+              params=dict(flow_direction_type=1, mfd_proportions=props))
+
+
+@pytest.mark.parametrize("shape", [(1, 40), (33, 31), (257, 130)])
+def test_stateless_accumulation_on_ragged_grids(libs, shape):
+    torch = pytest.importorskip("torch")
+    from parallem_gb300 import lem
+    rng = np.random.default_rng(shape[0])
+    h, w = shape
+    dem = rng.random(shape) + 500.0
+    dem[rng.random(shape) < 0.05] = NODATA
+    inside = dem != NODATA
+    weight = np.where(inside, rng.random(shape) + 0.1, -9999.0)
+    # every cell drains east or south-east (to a cell inside, or off the grid): a forest
+    step = {1: (0, 1), 2: (1, 1)}
+    code = np.where(rng.random(shape) < 0.7, 1, 2).astype(np.int32)
+    code[~inside] = -9999
+    want = np.where(inside, weight, 0.0)
+    for x in range(w):
+        for y in range(h):
+            if not inside[y, x]:
+                continue
+            dy, dx = step[int(code[y, x])]
+            if y + dy < h and x + dx < w and inside[y + dy, x + dx]:
+                want[y + dy, x + dx] += want[y, x]
+    t = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (code, weight, dem)]
+    out = torch.full(shape, -1.0, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    rc = lem.load().lem_accumulate_flow_noalloc(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), out.data_ptr(), w,
+                                                h, None)
+    assert rc == 0
+    # fp32 weights summed as float pairs: the accumulation tolerance of the parity tests
+    np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("n", [40, 300])
+def test_spill_heights_of_tied_boundaries(libs, n):
+    z = S.make_dem(n, 0.6, 60.0, 0.02, n, 2, 5, depressions=n // 4)
+    # whole metres: many boundaries tie; above zero, since the reference takes a spill height of 0 for none
+    z = np.where(z == NODATA, NODATA, np.floor(z) + 100.0)
+    run_steps(libs, z, 1, np.full(1, 900.0), np.full(1, 9.0), False)
