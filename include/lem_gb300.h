@@ -353,7 +353,7 @@ lem_status lem_snapshot_load(lem_handle* h, int32_t id, const void* host, size_t
  * everything below one) output their own weight and the call returns
  * LEM_ERR_NOCONVERGE after writing d_fa.
  * Intermediate data lives in one statically allocated device array sized for
- * LEM_NOALLOC_MAX_CELLS cells (about 17 MB, held by every GPU that loads the
+ * LEM_NOALLOC_MAX_CELLS cells (about 78 MB, held by every GPU that loads the
  * library until the process exits); larger grids are rejected with
  * LEM_ERR_CAPACITY before any work.  The call looks up that array's device
  * address on the current device; the first call on a device must come before

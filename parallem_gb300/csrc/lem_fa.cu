@@ -12,6 +12,7 @@
 
 #include <cooperative_groups.h>
 
+#include <cstring>
 #include <mutex>
 
 #include "lem_wave.cuh"
@@ -26,7 +27,7 @@ namespace {
 // inflow from another tile somewhere upstream (its final value needs the
 // coarse wave)
 constexpr uint8_t kLaDone = 1, kLaWaits = 2;
-constexpr int kLaOutlet = 1;  // final-pass entry: an outlet (stored by the coarse wave; counted only)
+constexpr int32_t kLaOutlet = -1;  // final-pass entry in the place of the node: an outlet (the coarse wave's; counted only)
 
 // calcrunoffweight (runoffweight.cu:21-58) plus the in-degrees of the wave.
 // A donor outside the catchment is complete from the start when its DEM is
@@ -272,9 +273,9 @@ __global__ void __launch_bounds__(256, 8)
     k_fat_local(const double* __restrict__ z, const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
                 const float* __restrict__ w, int4* __restrict__ t_rec, int32_t* __restrict__ t_dst,
                 int32_t* __restrict__ t_pend, int32_t* __restrict__ t_ent, float2* __restrict__ fa,
-                int32_t* __restrict__ n_meta, int32_t* __restrict__ n_ref, int4* __restrict__ f_idx,
-                float2* __restrict__ f_la, int32_t* __restrict__ t_fcnt, int32_t* outs,
-                ModelConsts k, DevScalars* sc, DemCtx dc, TileSet ts) {
+                int32_t* __restrict__ n_meta, int32_t* __restrict__ n_ref, int2* __restrict__ f_idx,
+                float2* __restrict__ f_la, int32_t* __restrict__ t_fcnt, int32_t* outs, ModelConsts k,
+                DevScalars* sc, DemCtx dc, TileSet ts, int count) {
     if (!sc->tiled_ok) return;
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
@@ -299,7 +300,7 @@ __global__ void __launch_bounds__(256, 8)
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int gx = tx0 + lx, gy = ty0 + ly0 + 8 * q;
-        wq[q] = (gx < W && gy < H) ? w[(size_t)gy * W + gx] : 0.f;
+        wq[q] = !w ? 1.0f : (gx < W && gy < H) ? w[(size_t)gy * W + gx] : 0.f;
     }
     tile_load(z, mask, fd, W, H, tx0, ty0, s_code, s_cls);
     if (threadIdx.x == 0) s_fn = s_pool = 0;
@@ -523,7 +524,7 @@ __global__ void __launch_bounds__(256, 8)
     }
     done = wsum(done);
     dem = __reduce_max_sync(0xffffffffu, dem);  // one DEM per tile
-    if ((threadIdx.x & 31) == 0 && done && dem >= 0) atomicAdd(&dc.out[dem].fa_done, done);
+    if (count && (threadIdx.x & 31) == 0 && done && dem >= 0) atomicAdd(&dc.out[dem].fa_done, done);
     __syncthreads();
     // pointer jumping: every cell between nodes finds the node at the top of its run
     for (int it = 0; it < 10; ++it) {  // in-tile runs are shorter than 2^10 cells
@@ -585,10 +586,10 @@ __global__ void __launch_bounds__(256, 8)
         const bool waits = s_done[l] == (kLaDone | kLaWaits), outlet = s_kind[l] == kKindOutlet;
         const int e = warp_slot(waits || outlet, &s_fn);
         if (outlet) {  // counted once the coarse wave stored it
-            f_idx[tb + e] = make_int4((int)g, 0, kLaOutlet, 0);
+            f_idx[tb + e] = make_int2((int)g, kLaOutlet);
         } else if (waits) {
             const int node = (v & 0xffff) ? (v & 0xffff) - 1 : (s_nd[v >> 16] & 0xffff) - 1;
-            f_idx[tb + e] = make_int4((int)g, node, 0, 0);
+            f_idx[tb + e] = make_int2((int)g, node);
             f_la[tb + e] = s_la[l];
         }
         if (!waits || !(v & 0xffff)) continue;
@@ -723,9 +724,9 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_fat_final(const double* __restrict__ z, const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
                 const float* __restrict__ w, const int32_t* __restrict__ t_pend, float2* fa,
-                const int32_t* __restrict__ n_meta, const int32_t* __restrict__ n_ref, const int4* __restrict__ f_idx,
+                const int32_t* __restrict__ n_meta, const int32_t* __restrict__ n_ref, const int2* __restrict__ f_idx,
                 const float2* __restrict__ f_la, const int32_t* __restrict__ t_fcnt, ModelConsts k, DevScalars* sc,
-                DemCtx dc, TileSet ts) {
+                DemCtx dc, TileSet ts, int count) {
     if (!sc->tiled_ok) return;
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
@@ -812,9 +813,9 @@ __global__ void __launch_bounds__(256)
         __syncthreads();
         int done = 0, dem = -1;
         for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-            const int4 id = f_idx[tb + e];
+            const int2 id = f_idx[tb + e];
             dem = dem_at(dc, (size_t)id.x);
-            if (id.z & kLaOutlet) {
+            if (id.y == kLaOutlet) {
                 done += t_pend[id.x] == 0;
                 continue;
             }
@@ -824,7 +825,7 @@ __global__ void __launch_bounds__(256)
         }
         done = wsum(done);
         dem = __reduce_max_sync(0xffffffffu, dem);
-        if ((threadIdx.x & 31) == 0 && done && dem >= 0) atomicAdd(&dc.out[dem].fa_done, done);
+        if (count && (threadIdx.x & 31) == 0 && done && dem >= 0) atomicAdd(&dc.out[dem].fa_done, done);
         return;
     }
     const int tx0 = (t % TW) * kTile, ty0 = (t / TW) * kTile;
@@ -877,7 +878,7 @@ __global__ void __launch_bounds__(256)
                 outlet[q] = true;
                 if (t_pend[(size_t)(ty0 + ly) * W + tx0 + lx] == 0) ++done;
             }
-            wl = w[(size_t)(ty0 + ly) * W + tx0 + lx];
+            wl = w ? w[(size_t)(ty0 + ly) * W + tx0 + lx] : 1.0f;
             if (dem < 0) dem = dem_at(dc, (size_t)(ty0 + ly) * W + tx0 + lx);
         }
         s_pend[l] = pend;
@@ -921,7 +922,81 @@ __global__ void __launch_bounds__(256)
     done = wsum(done);
     if ((threadIdx.x & 31) == 0 && done) atomicAdd(&s_done, done);
     __syncthreads();
-    if (threadIdx.x == 0 && s_done && s_dem >= 0) atomicAdd(&dc.out[s_dem].fa_done, s_done);
+    if (count && threadIdx.x == 0 && s_done && s_dem >= 0) atomicAdd(&dc.out[s_dem].fa_done, s_done);
+}
+
+// The contributing-cell counts of a tiled step are the accumulation of unit
+// weights: the float pairs hold the whole numbers exactly (far beyond 2^31), so
+// the same kernels give them, in the place of the int32 counts of the general
+// wave (7.2 ms against 0.4 ms at 1501 x 1501 cells).  A cell the wave never
+// finishes counts itself only.
+__global__ void k_count_init(const uint8_t* __restrict__ mask, float2* __restrict__ cnt,
+                             const int32_t* __restrict__ chunk_start, int W, DemCtx dc, DevScalars* sc) {
+    if (!sc->tiled_ok) return;
+    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc->tile_src = 0;
+    for (int64_t ri = ch.first + threadIdx.x; ri < ch.end; ri += blockDim.x) {
+        int x, y;
+        const size_t i = region_cell(dc.in[ch.d], ri, W, &x, &y);
+        cnt[i] = make_float2(mask[i] ? 1.0f : 0.0f, 0.0f);
+    }
+}
+__global__ void k_count_out(const float2* __restrict__ cnt, int32_t* __restrict__ contrib,
+                            const int32_t* __restrict__ chunk_start, int W, DemCtx dc, DevScalars* sc) {
+    if (!sc->tiled_ok) return;
+    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    for (int64_t ri = ch.first + threadIdx.x; ri < ch.end; ri += blockDim.x) {
+        int x, y;
+        const size_t i = region_cell(dc.in[ch.d], ri, W, &x, &y);
+        const float2 v = cnt[i];
+        contrib[i] = (int32_t)v.x + (int32_t)v.y;  // both are whole
+    }
+}
+
+// The tiled accumulation of weights w (null: one each) into fa.  count: add the
+// finished cells to the DEMs' counters.
+struct FatArgs {
+    const double* z;
+    const uint8_t* mask;
+    const uint8_t* fd;
+    const float* w;
+    float2* fa;
+    int4* t_rec;
+    int32_t* t_dst;
+    int32_t* t_pend;
+    int32_t* t_ent;
+    int32_t* n_meta;
+    int32_t* n_ref;
+    int2* f_idx;
+    float2* f_la;
+    int32_t* t_fcnt;
+    int32_t* outs;
+    int32_t* ready;
+    DevScalars* sc;
+    DemCtx dc;
+    int coarse_blocks;
+};
+lem_status launch_fat(const FatArgs& a, const ModelConsts& k, const TileSet& ts, int count, const Launch& L) {
+    LEM_LAUNCH(L, k_fat_local, ts.n, 256, a.z, a.mask, a.fd, a.w, a.t_rec, a.t_dst, a.t_pend, a.t_ent, a.fa, a.n_meta,
+               a.n_ref, a.f_idx, a.f_la, a.t_fcnt, a.outs, k, a.sc, a.dc, ts, count);
+    const uint8_t* fd = a.fd;
+    int4* trec = a.t_rec;
+    const int32_t* tent = a.t_ent;
+    const int32_t* tdst = a.t_dst;
+    float2* fa = a.fa;
+    int32_t* tpend = a.t_pend;
+    const int32_t* outs = a.outs;  // the outlets, listed by k_fat_local
+    int32_t* ready = a.ready;
+    ModelConsts kk = k;
+    DevScalars* sc = a.sc;
+    void* args[] = {(void*)&fd,    (void*)&trec, (void*)&tent,  (void*)&tdst, (void*)&fa,
+                    (void*)&tpend, (void*)&outs, (void*)&ready, (void*)&kk,   (void*)&sc};
+    L.pre("k_fat_coarse");
+    LEM_CUDA_TRY(coop_launch((const void*)k_fat_coarse, a.coarse_blocks, args, L.st));
+    L.post();
+    LEM_LAUNCH(L, k_fat_final, ts.n, 256, a.z, a.mask, a.fd, a.w, a.t_pend, a.fa, a.n_meta, a.n_ref, a.f_idx, a.f_la,
+               a.t_fcnt, k, a.sc, a.dc, ts, count);
+    return LEM_OK;
 }
 
 // correctmfdflow's first-iteration branch (mfd_simple.cu:336-349): the outlet
@@ -980,7 +1055,7 @@ lem_status launch_flow_accumulation(const DevState& s, const ModelConsts& k, uin
     const int blocks = (int)(nb > 152 * 32 ? 152 * 32 : nb);
     const int dem_blocks = (s.dems.n + 127) / 128;
     int32_t* contrib = (flags & LEM_STEP_CONTRIB) ? s.contrib : nullptr;
-    const int tiled = (k.flow_type == 0 && !contrib) ? 1 : 0;
+    const int tiled = k.flow_type == 0 ? 1 : 0;
     LEM_LAUNCH(L, k_fa_reset, dem_blocks, 128, s.sc, s.dems, tiled);
     const float* prop = nullptr;
     if (k.flow_type != 0 && k.mfd_props) {
@@ -993,26 +1068,18 @@ lem_status launch_flow_accumulation(const DevState& s, const ModelConsts& k, uin
                s.sc, tiled);
     if (tiled) {
         const TileSet ts = tiles_of(s, k.W);
-        const int tiles = ts.n;
-        LEM_LAUNCH(L, k_fat_local, tiles, 256, s.z, s.mask, s.fd, s.w, s.t_rec, s.t_dst, s.t_pend, s.t_ent, s.fa,
-                   s.n_meta, s.p_ref, s.f_idx, s.f_ds, s.t_fcnt, s.list_b, k, s.sc, s.dems, ts);
-        const uint8_t* fd = s.fd;
-        int4* trec = s.t_rec;
-        const int32_t* tent = s.t_ent;
-        const int32_t* tdst = s.t_dst;
-        float2* fa = s.fa;
-        int32_t* tpend = s.t_pend;
-        const int32_t* outs = s.list_b;  // the outlets, listed by k_fat_local
-        int32_t* ready = s.list_a;
-        ModelConsts kk = k;
-        DevScalars* sc = s.sc;
-        void* args[] = {(void*)&fd,    (void*)&trec, (void*)&tent,  (void*)&tdst, (void*)&fa,
-                        (void*)&tpend, (void*)&outs, (void*)&ready, (void*)&kk,   (void*)&sc};
-        L.pre("k_fat_coarse");
-        LEM_CUDA_TRY(coop_launch((const void*)k_fat_coarse, s.coop_blocks[kCkFatCoarse], args, L.st));
-        L.post();
-        LEM_LAUNCH(L, k_fat_final, tiles, 256, s.z, s.mask, s.fd, s.w, s.t_pend, s.fa, s.n_meta, s.p_ref, s.f_idx,
-                   s.f_ds, s.t_fcnt, k, s.sc, s.dems, ts);
+        FatArgs a{s.z, s.mask, s.fd, s.w, s.fa, s.t_rec, s.t_dst, s.t_pend, s.t_ent, s.n_meta, s.p_ref,
+                  reinterpret_cast<int2*>(s.f_idx), s.f_ds, s.t_fcnt, s.list_b, s.list_a, s.sc, s.dems,
+                  s.coop_blocks[kCkFatCoarse]};
+        lem_status r = launch_fat(a, k, ts, 1, L);
+        if (r != LEM_OK) return r;
+        if (contrib) {
+            a.w = nullptr;
+            a.fa = reinterpret_cast<float2*>(s.p_map);  // free until the sediment programs: one pair per cell
+            LEM_LAUNCH(L, k_count_init, s.n_chunks, T, s.mask, a.fa, s.chunk_start, k.W, s.dems, s.sc);
+            if ((r = launch_fat(a, k, ts, 0, L)) != LEM_OK) return r;
+            LEM_LAUNCH(L, k_count_out, s.n_chunks, T, a.fa, contrib, s.chunk_start, k.W, s.dems, s.sc);
+        }
     }
     {
         float2* fa = s.fa;
@@ -1043,46 +1110,90 @@ lem_status launch_flow_accumulation(const DevState& s, const ModelConsts& k, uin
 namespace {
 
 constexpr size_t kNaCells = LEM_NOALLOC_MAX_CELLS;
+// The tiled accumulation's tables hold this many tiles, an eighth more than the
+// cells fill: grids a few columns or rows over a multiple of 32 fit, narrow
+// strips take the general wave.
+constexpr size_t kNaTiles = kNaCells / (kTile * kTile) * 9 / 8;
+constexpr size_t kNaSlots = kNaTiles * kTile * kTile;
 constexpr size_t kNaHead = 1024;  // DevScalars and one DemOut, rounded up
 constexpr size_t kNaOffDem = 512;
 static_assert(sizeof(DevScalars) <= kNaOffDem && kNaOffDem + sizeof(DemOut) <= kNaHead, "scalar block");
-constexpr size_t kNaOffWord = kNaHead;                        // int32
-constexpr size_t kNaOffList = kNaOffWord + 4 * kNaCells;      // int32
-constexpr size_t kNaOffFa = kNaOffList + 4 * kNaCells;        // float2
-constexpr size_t kNaBytes = kNaOffFa + 8 * kNaCells;
+constexpr size_t kNaOffFa = kNaHead;                          // float2 per cell
+constexpr size_t kNaOffRec = kNaOffFa + 8 * kNaCells;         // int4
+constexpr size_t kNaOffDst = kNaOffRec + 16 * kNaCells;       // int32
+constexpr size_t kNaOffPend = kNaOffDst + 4 * kNaCells;       // int32 (the general wave's words)
+constexpr size_t kNaOffOuts = kNaOffPend + 4 * kNaCells;      // int32 (and its list)
+constexpr size_t kNaOffReady = kNaOffOuts + 4 * kNaCells;     // int32
+constexpr size_t kNaOffW = kNaOffReady + 4 * kNaCells;        // float
+constexpr size_t kNaOffFd = kNaOffW + 4 * kNaCells;           // u8
+constexpr size_t kNaOffMask = kNaOffFd + kNaCells;            // u8
+constexpr size_t kNaOffIdx = kNaOffMask + kNaCells;           // int2 per slot
+constexpr size_t kNaOffLa = kNaOffIdx + 8 * kNaSlots;         // float2
+constexpr size_t kNaOffMeta = kNaOffLa + 8 * kNaSlots;        // int32
+constexpr size_t kNaOffRef = kNaOffMeta + 4 * kNaSlots;       // int32, kTilePool per tile
+constexpr size_t kNaOffEnt = kNaOffRef + 4 * kTilePool * kNaTiles;  // int32, kTileEnt per tile
+constexpr size_t kNaOffCnt = kNaOffEnt + 4 * kTileEnt * kNaTiles;   // int32 per tile
+constexpr size_t kNaBytes = kNaOffCnt + 4 * kNaTiles;
 
 // Scratch of the no-allocation entry point (every call shares it).
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
 
 struct NaDevice {
     unsigned char* base = nullptr;  // device address of g_noalloc_scratch
-    int blocks = 0;                 // co-resident blocks of k_fa_walk
+    int walk_blocks = 0;            // co-resident blocks of k_fa_walk
+    int coarse_blocks = 0;          //   and of k_fat_coarse
 };
 std::mutex g_na_mutex;
 NaDevice g_na[64];
 
-__global__ void k_na_reset(DevScalars* sc, DemOut* dem) {
+__global__ void k_na_reset(DevScalars* sc, DemOut* dem, int tiled) {
     dem->fa_done = 0;
     dem->n_active = 0;
-    sc->counters[0] = sc->counters[1] = sc->counters[2] = 0;
+    sc->counters[0] = 0;
+    sc->tile_src = 0;
+    sc->tiled_ok = tiled;
     sc->err = 0;
     sc->err_first = 0;
 }
 
-// Initial accumulation (the weight) and the wave's words from the caller's int32
-// codes and DEM (cells at -9999 are outside and complete with zero flow).
-__global__ void k_na_prep(const int32_t* __restrict__ fd_in, const double* __restrict__ w_in,
-                          const double* __restrict__ dem, float2* __restrict__ fa, int32_t* __restrict__ word,
-                          int32_t* ready, int W, int H, DevScalars* sc, DemOut* dem_out) {
+// Codes, mask, weights and the initial accumulation (the weight) from the
+// caller's int32 codes and DEM (cells at -9999 are outside and complete with
+// zero flow).  As in a step, a negative weight or a multi-direction code sends
+// the call to the general wave.
+__global__ void __launch_bounds__(256)
+    k_na_prep(const int32_t* __restrict__ fd_in, const double* __restrict__ w_in, const double* __restrict__ dem,
+              uint8_t* __restrict__ fd, uint8_t* __restrict__ mask, float* __restrict__ w, float2* __restrict__ fa,
+              size_t N, DevScalars* sc, DemOut* dem_out) {
+    int nact = 0;
+    bool untiled = false;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
+        const bool in = dem[i] != kNoData;
+        const uint32_t code = (uint32_t)fd_in[i] & 0xffu;
+        const float wi = (float)w_in[i];
+        fd[i] = (uint8_t)code;
+        mask[i] = in ? 1 : 0;
+        w[i] = wi;
+        fa[i] = make_float2(in ? wi : 0.0f, 0.0f);
+        nact += in;
+        untiled |= in && (wi < 0.0f || (code & (code - 1)));
+    }
+    if (__syncthreads_or(untiled) && threadIdx.x == 0) sc->tiled_ok = 0;
+    const int tot = block_sum_i(nact);
+    if (threadIdx.x == 0 && tot) atomicAdd(&dem_out->n_active, tot);
+}
+
+// The general wave's words and sources.
+__global__ void k_na_words(const uint8_t* __restrict__ fd, const uint8_t* __restrict__ mask,
+                           int32_t* __restrict__ word, int32_t* ready, int W, int H, DevScalars* sc) {
+    if (sc->tiled_ok) return;
     const size_t N = (size_t)W * H;
     for (size_t base = (size_t)blockIdx.x * blockDim.x; base < N; base += (size_t)gridDim.x * blockDim.x) {
         const size_t i = base + threadIdx.x;
-        bool src = false, act = false;
+        bool src = false;
         if (i < N) {
             const int x = (int)(i % W), y = (int)(i / W);
-            const bool in = dem[i] != kNoData;
-            const uint32_t code = (uint32_t)(fd_in[i] & 0xff);
-            fa[i] = make_float2(in ? (float)w_in[i] : 0.0f, 0.0f);
+            const bool in = mask[i];
+            const uint32_t code = fd[i];
             int32_t pend = in ? 0 : kBlocked;
             uint32_t donors = 0, receivers = 0;
 #pragma unroll
@@ -1090,19 +1201,16 @@ __global__ void k_na_prep(const int32_t* __restrict__ fd_in, const double* __res
                 const int nx = x + dir_dx(d), ny = y + dir_dy(d);
                 if (!in || nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
                 const size_t n = (size_t)ny * W + nx;
-                if (dem[n] == kNoData) continue;
+                if (!mask[n]) continue;
                 receivers |= code & dir_bit(d);
-                if (donates((uint8_t)(fd_in[n] & 0xff), d)) {
+                if (donates(fd[n], d)) {
                     ++pend;
                     donors |= 1u << scan_index(d);
                 }
             }
             word[i] = wave_word(pend, donors, receivers);
             src = in && pend == 0;
-            act = in;
         }
-        const unsigned nact = __ballot_sync(0xffffffffu, act);  // in-catchment cells, one atomic per warp
-        if ((threadIdx.x & 31) == 0 && nact) atomicAdd(&dem_out->n_active, __popc(nact));
         wave_append(src, (int32_t)i, ready, &sc->counters[0], (int)N, &sc->err);
     }
 }
@@ -1137,11 +1245,9 @@ extern "C" lem_status lem_accumulate_flow_noalloc(const int32_t* d_fd, const dou
             // call on this device is used.
             void* ptr = nullptr;
             LEM_CUDA_TRY(cudaGetSymbolAddress(&ptr, g_noalloc_scratch));
-            if (!g_na[dev].blocks) {
-                int per = 0, sms = 0;
-                LEM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fa_walk, 256, 0));
-                LEM_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-                g_na[dev].blocks = (per < 1 ? 1 : per) * sms;
+            if (!g_na[dev].walk_blocks) {
+                g_na[dev].walk_blocks = coop_blocks_for((const void*)k_fa_walk, 256, 0);
+                g_na[dev].coarse_blocks = coop_blocks_for((const void*)k_fat_coarse, 256, 0);
             }
             g_na[dev].base = static_cast<unsigned char*>(ptr);
         }
@@ -1149,33 +1255,54 @@ extern "C" lem_status lem_accumulate_flow_noalloc(const int32_t* d_fd, const dou
     }
     DevScalars* sc = reinterpret_cast<DevScalars*>(nd.base);
     DemOut* dem = reinterpret_cast<DemOut*>(nd.base + kNaOffDem);
-    int32_t* word = reinterpret_cast<int32_t*>(nd.base + kNaOffWord);
-    int32_t* list = reinterpret_cast<int32_t*>(nd.base + kNaOffList);
-    float2* fa = reinterpret_cast<float2*>(nd.base + kNaOffFa);
+    auto at = [&](size_t off) { return static_cast<void*>(nd.base + off); };
+    uint8_t* const fd = static_cast<uint8_t*>(at(kNaOffFd));
+    uint8_t* const mask = static_cast<uint8_t*>(at(kNaOffMask));
+    float* const w = static_cast<float*>(at(kNaOffW));
+    float2* fa = static_cast<float2*>(at(kNaOffFa));
+    int32_t* word = static_cast<int32_t*>(at(kNaOffPend));
+    int32_t* list = static_cast<int32_t*>(at(kNaOffOuts));
     const int T = 256;
     const int blocks = (int)std::min<size_t>((N + T - 1) / T, 152 * 32);
-    k_na_reset<<<1, 1, 0, st>>>(sc, dem);  // the array keeps the previous call's contents
-    k_na_prep<<<blocks, T, 0, st>>>(d_fd, d_weight, d_dem, fa, word, list, width, height, sc, dem);
+    const int tw = (width + kTile - 1) / kTile, tiles = tw * ((height + kTile - 1) / kTile);
+    const int tiled = (size_t)tiles <= kNaTiles;
+    ModelConsts k{};
+    k.W = width;
+    k.H = height;
+    const DemCtx dc{nullptr, nullptr, dem, 1};
+    uint64_t launches = 0;
+    const Launch L{st, &launches, nullptr};
+    k_na_reset<<<1, 1, 0, st>>>(sc, dem, tiled);  // the array keeps the previous call's contents
+    k_na_prep<<<blocks, T, 0, st>>>(d_fd, d_weight, d_dem, fd, mask, w, fa, N, sc, dem);
+    if (tiled) {
+        const FatArgs a{d_dem, mask, fd, w, fa, static_cast<int4*>(at(kNaOffRec)), static_cast<int32_t*>(at(kNaOffDst)),
+                        word, static_cast<int32_t*>(at(kNaOffEnt)), static_cast<int32_t*>(at(kNaOffMeta)),
+                        static_cast<int32_t*>(at(kNaOffRef)), static_cast<int2*>(at(kNaOffIdx)),
+                        static_cast<float2*>(at(kNaOffLa)), static_cast<int32_t*>(at(kNaOffCnt)), list,
+                        static_cast<int32_t*>(at(kNaOffReady)), sc, dc, std::min(nd.coarse_blocks, tiles)};
+        const lem_status r = launch_fat(a, k, TileSet{nullptr, tiles, tw}, 1, L);
+        if (r != LEM_OK) return r;
+    }
+    k_na_words<<<blocks, T, 0, st>>>(fd, mask, word, list, width, height, sc);
     LEM_CUDA_TRY(cudaGetLastError());
     {
         const float* prop = nullptr;
         int32_t* contrib = nullptr;
-        ModelConsts k{};
-        k.W = width;
-        k.H = height;
-        int gate = 0;
-        DemCtx dc{nullptr, nullptr, dem, 1};
+        int gate = tiled;
+        DemCtx d = dc;
         void* args[] = {(void*)&prop, (void*)&fa, (void*)&word, (void*)&contrib, (void*)&list,
-                        (void*)&k,    (void*)&sc, (void*)&dc,   (void*)&gate};
-        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, walk_blocks(nd.blocks, N), args, st));
+                        (void*)&k,    (void*)&sc, (void*)&d,    (void*)&gate};
+        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, walk_blocks(nd.walk_blocks, N), args, st));
     }
     k_na_out<<<blocks, T, 0, st>>>(fa, d_fa, N);
     LEM_CUDA_TRY(cudaGetLastError());
-    uint32_t err[2] = {0, 0};  // err and err_first
-    DemOut counts{};
-    LEM_CUDA_TRY(cudaMemcpyAsync(err, &sc->err, sizeof err, cudaMemcpyDeviceToHost, st));
-    LEM_CUDA_TRY(cudaMemcpyAsync(&counts, dem, sizeof counts, cudaMemcpyDeviceToHost, st));
+    unsigned char head[kNaHead];  // the scalars and the counts in one copy
+    LEM_CUDA_TRY(cudaMemcpyAsync(head, nd.base, sizeof head, cudaMemcpyDeviceToHost, st));
     LEM_CUDA_TRY(cudaStreamSynchronize(st));
+    uint32_t err[2];  // err and err_first
+    DemOut counts;
+    std::memcpy(err, head + offsetof(DevScalars, err), sizeof err);
+    std::memcpy(&counts, head + kNaOffDem, sizeof counts);
     if (err[1] == ErrFlags::kCapacity || (err[0] & ErrFlags::kCapacity && err[1] != ErrFlags::kNoConverge))
         return LEM_ERR_CAPACITY;
     if (err[0]) return LEM_ERR_NOCONVERGE;

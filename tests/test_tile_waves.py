@@ -3,8 +3,10 @@
 * Coarse waves: a comb of trunk channels whose tiles give one outlet a program
   of fewer than 32, of 32 to 64 and of more than 64 nodes, with more inputs than
   a warp gathers at once.
-* The general wave (several receivers, the stateless accumulation): slopes on
-  which few cells start ready, on grids of a few cells and of many blocks.
+* The general wave (several receivers): slopes on which few cells start ready,
+  on grids of a few cells and of many blocks.
+* The stateless accumulation, tiled and by the general wave, and the tiled
+  contributing counts.
 * Spill heights: boundaries that tie, on few edges (one block) and on many.
 
 The tolerances are those of tests/test_gpu_parity.py.
@@ -14,7 +16,7 @@ import pytest
 
 from parallem_gb300 import scenario as S
 from tests.helpers import NODATA, ringed
-from tests.test_gpu_parity import libs, run_steps  # noqa: F401
+from tests.test_gpu_parity import check_fa, libs, pair, run_steps  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -48,8 +50,10 @@ def test_general_wave_with_several_receivers(libs, shape, slope, props):
               params=dict(flow_direction_type=1, mfd_proportions=props))
 
 
-@pytest.mark.parametrize("shape", [(1, 40), (33, 31), (257, 130)])
-def test_stateless_accumulation_on_ragged_grids(libs, shape):
+# a strip whose tiles the tables do not hold (the general wave), ragged grids, a code with two receivers
+@pytest.mark.parametrize("shape,double", [((1, 40), False), ((3, 40000), False), ((33, 31), False), ((257, 130), False),
+                                          ((65, 97), True)])
+def test_stateless_accumulation_on_ragged_grids(libs, shape, double):
     torch = pytest.importorskip("torch")
     from parallem_gb300 import lem
     rng = np.random.default_rng(shape[0])
@@ -61,15 +65,17 @@ def test_stateless_accumulation_on_ragged_grids(libs, shape):
     # every cell drains east or south-east (to a cell inside, or off the grid): a forest
     step = {1: (0, 1), 2: (1, 1)}
     code = np.where(rng.random(shape) < 0.7, 1, 2).astype(np.int32)
+    if double:
+        code[h // 2, w // 3] = 3
     code[~inside] = -9999
     want = np.where(inside, weight, 0.0)
     for x in range(w):
         for y in range(h):
-            if not inside[y, x]:
-                continue
-            dy, dx = step[int(code[y, x])]
-            if y + dy < h and x + dx < w and inside[y + dy, x + dx]:
-                want[y + dy, x + dx] += want[y, x]
+            for bit, (dy, dx) in step.items():
+                if not inside[y, x] or not code[y, x] & bit:
+                    continue
+                if y + dy < h and x + dx < w and inside[y + dy, x + dx]:
+                    want[y + dy, x + dx] += want[y, x]
     t = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (code, weight, dem)]
     out = torch.full(shape, -1.0, dtype=torch.float64, device="cuda")
     torch.cuda.synchronize()
@@ -78,6 +84,19 @@ def test_stateless_accumulation_on_ragged_grids(libs, shape):
     assert rc == 0
     # fp32 weights summed as float pairs: the accumulation tolerance of the parity tests
     np.testing.assert_allclose(out.cpu().numpy(), want, rtol=1e-5, atol=0)
+
+
+@pytest.mark.parametrize("n", [31, 97, 300])
+def test_contributing_counts_of_tiled_steps(libs, n):
+    from parallem_gb300 import lem
+    dem = S.make_dem(n, 0.7, 800.0, 0.03, n, 2, 17)
+    o, g, mask = pair(libs, dem, 900.0, 9.0, None, None)
+    g.flow_direction()
+    g.flow_accumulation(lem.STEP_CONTRIB)
+    g.synchronize()
+    o.flow_direction()
+    o.flow_accumulation()
+    check_fa(o, g, mask, contrib=True)
 
 
 @pytest.mark.parametrize("n", [40, 300])
