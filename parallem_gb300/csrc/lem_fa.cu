@@ -23,10 +23,11 @@ namespace lem {
 
 namespace {
 
-// k_fat_local's cell status: finished inside the tile, and waiting on an
-// inflow from another tile somewhere upstream (its final value needs the
-// coarse wave)
-constexpr uint8_t kLaDone = 1, kLaWaits = 2;
+// k_fat_local's cell status: a donor in another tile, finished inside the tile,
+// and waiting on an inflow from another tile somewhere upstream (its final value
+// needs the coarse wave)
+constexpr uint8_t kLaKind = 3, kLaEntry = 4, kLaDone = 8, kLaWaits = 16;  // (below them the cell's kind)
+constexpr int32_t kRun = 1 << 30;  // k_fat_local: a waiting cell between nodes
 constexpr int32_t kLaOutlet = -1;  // final-pass entry in the place of the node: an outlet (the coarse wave's; counted only)
 
 // calcrunoffweight (runoffweight.cu:21-58) plus the in-degrees of the wave.
@@ -269,7 +270,7 @@ __device__ __forceinline__ void tile_load(const double* __restrict__ z, const ui
     }
 }
 
-__global__ void __launch_bounds__(256, 8)
+__global__ void __launch_bounds__(256, 6)
     k_fat_local(const double* __restrict__ z, const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
                 const float* __restrict__ w, int4* __restrict__ t_rec, int32_t* __restrict__ t_dst,
                 int32_t* __restrict__ t_pend, int32_t* __restrict__ t_ent, float2* __restrict__ fa,
@@ -279,18 +280,20 @@ __global__ void __launch_bounds__(256, 8)
     if (!sc->tiled_ok) return;
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
-    __shared__ int32_t s_pend[kTile * kTile];
-    __shared__ float2 s_la[kTile * kTile];
-    __shared__ int16_t s_ptr[kTile * kTile];
-    __shared__ uint8_t s_kind[kTile * kTile];
-    __shared__ uint8_t s_ext[kTile * kTile];
-    __shared__ uint8_t s_done[kTile * kTile];
-    __shared__ int16_t s_oslot[kTile * kTile];
-    __shared__ int16_t s_q[kTile * kTile];
+    __shared__ int32_t s_pd[kTile * kTile];  // the in-tile path (tile_paths): where it ends
+    __shared__ int32_t s_h[kTile * kTile + 1];  // levels
+    __shared__ float2 s_la[kTile * kTile + 1];
+    __shared__ uint8_t s_info[kTile * kTile];  // kind, and kLa flags
+    // donors, bit k for direction scan_dir(k): in the low byte those in the tile,
+    // in the high byte those in other tiles, then with the waiting ones in the tile
+    __shared__ __align__(4) uint16_t s_dm[kTile * kTile + 1];
+    __shared__ uint32_t s_ent[kTile * kTile];  // the finished cells by level
+    __shared__ uint32_t s_bins[kTile * kTile / 2];
+    __shared__ uint32_t s_wait[kTile], s_bad[kTile];
     __shared__ int16_t s_olist[kTileEnt];
     __shared__ int32_t s_ocnt[kTileEnt];
     __shared__ int32_t s_ofill[kTileEnt];
-    __shared__ int s_no, s_qn, s_qend, s_nn, s_fn, s_pool;
+    __shared__ int s_no, s_nn, s_fn, s_pool, s_qn;
     __shared__ int s_wcnt[9];  // per-warp counts of the outlet list and its append
     const int W = k.W, H = k.H, TW = (W + kTile - 1) / kTile;
     const int t = ts.tile(blockIdx.x);
@@ -302,123 +305,132 @@ __global__ void __launch_bounds__(256, 8)
         const int gx = tx0 + lx, gy = ty0 + ly0 + 8 * q;
         wq[q] = !w ? 1.0f : (gx < W && gy < H) ? w[(size_t)gy * W + gx] : 0.f;
     }
-    tile_load(z, mask, fd, W, H, tx0, ty0, s_code, s_cls);
     if (threadIdx.x == 0) s_fn = s_pool = 0;
+    for (int i = threadIdx.x; i < kTile * kTile / 2; i += blockDim.x) {
+        s_bins[i] = 0;
+        reinterpret_cast<uint32_t*>(s_dm)[i] = 0;
+    }
+    if (threadIdx.x < kTile) s_bad[threadIdx.x] = 0;
     __syncthreads();
-    bool src[4];  // chain starts, fixed before any chain runs (a chain may enter them later)
+    tile_stage(
+        fd,
+        [&](size_t g, int, int) {
+            return mask[g] ? kCellIn : (z[g] == kNoData ? kCellOff : kCellBlock);
+        },
+        W, H, tx0, ty0, s_code, s_cls, s_dm, s_bad);
+    __syncthreads();
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        int32_t pend = kBlocked;
-        uint8_t kind = kKindEnd, ext = 0;
-        int16_t ptr = (int16_t)l;
-        float wl = 0.f;
-        int16_t dm = 0;  // the in-tile donors: bit k for direction scan_dir(k)
+        uint32_t dm = 0, kind = kKindEnd;
+        int32_t pd = l;
         if (s_cls[hc] == kCellIn) {
-            pend = 0;
-#pragma unroll
-            for (int d = 0; d < 8; ++d) {
-                const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-                if (!donates(s_code[nh], d)) continue;
-                const uint8_t cl = s_cls[nh];
-                if (cl == kCellBlock)
-                    pend |= kBlocked;
-                else if (cl == kCellIn) {
-                    if (in_tile(lx + dir_dx(d), ly + dir_dy(d))) {
-                        ++pend;
-                        dm |= (int16_t)(1 << scan_index(d));
-                    } else {
-                        ++ext;
-                    }
-                }
-            }
+            dm = s_dm[l];
             const int d = bit_dir(s_code[hc]);
-            if (d >= 0 && s_cls[hc + dir_dy(d) * kTH + dir_dx(d)] == kCellIn) {
-                const int rlx = lx + dir_dx(d), rly = ly + dir_dy(d);
-                if (in_tile(rlx, rly)) {
-                    kind = kKindIn;
-                    ptr = (int16_t)(rly * kTile + rlx);
-                } else {
-                    kind = kKindOutlet;
-                }
-            }
-            wl = wq[q];
-        }
-        s_pend[l] = pend;
-        src[q] = pend == 0;
-        s_kind[l] = kind;
-        s_ext[l] = ext;
-        s_ptr[l] = ptr;
-        s_la[l] = make_float2(wl, 0.f);
-        s_done[l] = 0;
-        s_oslot[l] = dm;  // the outlet slots are listed after the wave
-    }
-    if (threadIdx.x == 0) s_qn = 0;
-    __syncthreads();
-    // accumulation from inside the tile, in dependency order
-    tile_wave(
-        [&](int cur, int rnd) {
-            // the in-tile donors, all loaded before the sum in scan order
-            const uint32_t dm = (uint16_t)s_oslot[cur];
-            float2 v[8];
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-                v[kk] = (dm >> kk) & 1u ? s_la[cur + tile_step(scan_dir(kk))] : make_float2(0.f, 0.f);
-            float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int kk = 0; kk < 8; ++kk)
-                if ((dm >> kk) & 1u) acc = ff_add(acc, v[kk]);
-            if (acc.x < 0.0f) acc = make_float2(0.f, 0.f);
-            s_la[cur] = ff_add(s_la[cur], acc);
-            s_done[cur] = kLaDone;
-            return s_kind[cur] == kKindIn ? (int)s_ptr[cur] : -1;
-        },
-        s_pend, s_q, &s_qn, &s_qend, src, lx, ly0);
-    // The waiting cells: every finished cell downstream of an entry (a cell
-    // with a donor in another tile), marked along each entry's in-tile path.
-    // A walk stops where another walk has passed (it carries on from there).
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        int c = (ly0 + 8 * q) * kTile + lx;
-        if (!s_ext[c]) continue;
-        for (int guard = 0; guard < kTile * kTile; ++guard) {
-            if (s_done[c] != kLaDone) break;  // not finished, or marked already
-            s_done[c] = kLaDone | kLaWaits;
-            if (s_kind[c] != kKindIn) break;
-            c = s_ptr[c];
-        }
-    }
-    __syncthreads();
-    // the end of every in-tile path: pointer jumping (paths are shorter than 2^10 cells)
-    for (int it = 0; it < 10; ++it) {  // in-tile paths are shorter than 2^10 cells
-        bool ch = false;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int l = (ly0 + 8 * q) * kTile + lx;
-            const int16_t nx = s_ptr[s_ptr[l]];
-            if (nx != s_ptr[l]) {
-                s_ptr[l] = nx;
-                ch = true;
+            const int rlx = lx + dir_dx(d < 0 ? 0 : d), rly = ly + dir_dy(d < 0 ? 0 : d);
+            if (d >= 0 && s_cls[(rly + 1) * kTH + rlx + 1] == kCellIn) {
+                kind = in_tile(rlx, rly) ? kKindIn : kKindOutlet;
+                if (kind == kKindIn) pd = (rly * kTile + rlx) | (1 << 10);
             }
         }
-        if (!__syncthreads_or(ch)) break;  // every pointer is at its path's end
+        const float2 wl = make_float2(s_cls[hc] == kCellIn ? wq[q] : 0.f, 0.f);
+        const bool entry = dm >> 8;
+        s_la[l] = dm & 255u ? wl : ff_add(wl, make_float2(0.f, 0.f));  // level 0: final
+        s_pd[l] = pd;
+        s_h[l] = 0;
+        s_info[l] = (uint8_t)(kind | (entry ? kLaEntry : 0));
+        s_dm[l] = (uint16_t)dm;
+        const unsigned wb = __ballot_sync(0xffffffffu, entry);
+        if (lx == 0) s_wait[ly] = wb;
     }
+    __syncthreads();
+    tile_paths(s_pd, s_h, s_wait, s_bad, lx, ly0);
+    // a cell is finished here unless a donor upstream never completes; it waits
+    // when an entry (a cell with a donor in another tile) lies upstream
+    int level[4];
     bool stray = false;  // a waiting cell whose in-tile path ends inside the tile
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx;
-        if (s_ext[l]) {
-            const int e = s_ptr[l];
-            t_dst[(size_t)(ty0 + ly) * W + tx0 + lx] =
-                s_kind[e] == kKindOutlet ? (int32_t)((ty0 + e / kTile) * W + tx0 + (e & (kTile - 1))) : -1;
-        }
-        stray |= s_done[l] == (kLaDone | kLaWaits) && s_kind[s_ptr[l]] != kKindOutlet;
+        uint32_t info = s_info[l];
+        const bool done = s_cls[(ly + 1) * kTH + lx + 1] == kCellIn && !((s_bad[ly] >> lx) & 1u);
+        const bool waits = done && ((s_wait[ly] >> lx) & 1u);
+        level[q] = done ? s_h[l] : -1;
+        info |= (done ? kLaDone : 0) | (waits ? kLaWaits : 0);
+        s_info[l] = (uint8_t)info;
     }
+    tile_sort(
+        level,
+        [&](int q) {
+            const int l = (ly0 + 8 * q) * kTile + lx;
+            return entry_of(l, s_dm[l] & 255u);
+        },
+        s_bins, kTile * kTile / 2, s_ent, &s_qn, lx);  // (its barriers also cover s_info)
+    // What a waiting cell needs of the cells above it: s_nd holds 1 for a node
+    // (an entry, a join of waiting branches, the outlet), else kRun and the cell
+    // at the top of its run of single-input cells in the high half, found in
+    // level order from its waiting donor.
+    int32_t* const s_nd = s_h;  // the levels are spent
+#pragma unroll 1
+    for (int q = 0; q < 4; ++q) {
+        const int ly = ly0 + 8 * q, l = ly * kTile + lx;
+        const uint32_t info = s_info[l];
+        int32_t nd = 0;
+        if (info & kLaWaits) {
+            const uint32_t dm = s_dm[l];
+            uint32_t wm = 0;
+            for (uint32_t m = dm & 255u; m; m &= m - 1)
+                if (s_info[l + scan_step(__ffs(m) - 1)] & kLaWaits) wm |= m & (0u - m);
+            nd = (dm >> 8) || (wm & (wm - 1)) || (info & kLaKind) == kKindOutlet
+                     ? 1
+                     : kRun | ((l + scan_step(__ffs(wm) - 1)) << 16);
+            s_dm[l] = (uint16_t)(dm | (wm << 8));
+        }
+        s_nd[l] = nd;
+        const int e = s_pd[l] & kPtr;
+        const bool out = (s_info[e] & kLaKind) == kKindOutlet;
+        if (info & kLaEntry)
+            t_dst[(size_t)(ty0 + ly) * W + tx0 + lx] =
+                out ? (int32_t)((ty0 + e / kTile) * W + tx0 + (e & (kTile - 1))) : -1;
+        stray |= (info & kLaWaits) && !out;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {  // kNoCell: a cell of nothing, its own donor
+        s_la[kNoCell] = make_float2(0.f, 0.f);
+        s_nd[kNoCell] = 0;
+        s_dm[kNoCell] = 0;
+    }
+    __syncthreads();
+    // accumulation from inside the tile, level by level; adding the zero of
+    // kNoCell changes no pair
+    struct Cell {
+        float2 w;
+        uint32_t e;
+        int32_t nd;
+    };
+    tile_levels(
+        [&](uint32_t e) { return Cell{s_la[entry_cell(e)], e, s_nd[entry_cell(e)]}; },
+        [&](const Cell& f) {
+            const int c = entry_cell(f.e);
+            float2 acc = ff_add(s_la[entry_d0(f.e)], s_la[entry_d1(f.e)]);
+            const int32_t top = s_nd[f.nd & kRun ? (f.nd >> 16) & kPtr : kNoCell];
+            if (__any_sync(0xffffffffu, f.e & kMoreDonors) && (f.e & kMoreDonors)) {
+                uint32_t m = s_dm[c] & 255u;
+                m &= m - 1;
+                for (m &= m - 1; m; m &= m - 1) acc = ff_add(acc, s_la[c + scan_step(__ffs(m) - 1)]);
+            }
+            const bool neg = acc.x < 0.0f;
+            s_la[c] = ff_add(f.w, make_float2(neg ? 0.f : acc.x, neg ? 0.f : acc.y));
+            s_nd[c] = top & kRun ? top : f.nd;
+        },
+        1, kTile * kTile, s_bins, s_ent);
+    int16_t* const s_oslot = reinterpret_cast<int16_t*>(s_bins);  // the bins are spent
+    const int qn = s_qn;                                          // finished cells
     // Such a tile keeps the second wave; every other tile writes its settled
     // cells here and leaves the final pass a program of nodes (see below).
     const bool second_wave = __syncthreads_or(stray);
     // outlets in cell order (they lie on the border: at most 124)
-    list_outlets(s_kind, s_olist, s_oslot, &s_no, s_wcnt);
+    list_outlets(s_info, kLaKind, s_olist, s_oslot, &s_no, s_wcnt);
     if (threadIdx.x < kTileEnt) s_ocnt[threadIdx.x] = 0;
     __syncthreads();
     // inflows: ring cells of the halo that flow into the tile, grouped by the
@@ -437,8 +449,8 @@ __global__ void __launch_bounds__(256, 8)
                 const int hx = h % kTH + dir_dx(d), hy = h / kTH + dir_dy(d);
                 if (hx >= 1 && hx <= kTile && hy >= 1 && hy <= kTile && s_cls[hy * kTH + hx] == kCellIn) {
                     const int e = (hy - 1) * kTile + hx - 1;
-                    const int o = s_ptr[e];
-                    if (s_kind[o] == kKindOutlet) {
+                    const int o = s_pd[e] & kPtr;
+                    if ((s_info[o] & kLaKind) == kKindOutlet) {
                         key[c] = s_oslot[o];
                         donor[c] = (ty0 - 1 + h / kTH) * W + tx0 - 1 + h % kTH;
                         atomicAdd(&s_ocnt[key[c]], 1);
@@ -471,7 +483,7 @@ __global__ void __launch_bounds__(256, 8)
     int32_t og = 0;
     if (j < no) {
         const int o = s_olist[j];
-        const int32_t opend = ((s_done[o] & kLaDone) ? 0 : kBlocked) + s_ocnt[j];
+        const int32_t opend = ((s_info[o] & kLaDone) ? 0 : kBlocked) + s_ocnt[j];
         og = (ty0 + o / kTile) * W + tx0 + (o & (kTile - 1));
         const float2 la = s_la[o];
         t_rec[og] = make_int4(__float_as_int(la.x), __float_as_int(la.y), (ostart << 16) | s_ocnt[j], -1);
@@ -487,70 +499,26 @@ __global__ void __launch_bounds__(256, 8)
 
     // The final pass's program.  A waiting cell's accumulation is its local
     // one plus the inflows of every entry upstream of it.  That sum is the same
-    // along a run of single-input cells, so it is kept per node (an entry, a
-    // join of two waiting branches, or the outlet): the inflows the node takes
-    // from other tiles plus the sums of the nodes at the top of its waiting
-    // inputs.  s_nd: node index + 1 in the low half (0: not a node), the cell
-    // above in the high half (a cell between nodes: its waiting donor, then
-    // the node at the top of its run).
-    int32_t* s_nd = s_pend;  // the in-degrees are spent
+    // along a run of single-input cells, so it is kept per node: the inflows the
+    // node takes from other tiles plus the sums of the nodes at the top of its
+    // waiting inputs.  s_nd: from here on a node's index + 1.
     int done = 0, dem = -1;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
         const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
-        int32_t nd = 0;
         if (dem < 0 && s_cls[hc] == kCellIn) dem = dem_at(dc, g);
-        if (s_done[l] == kLaDone) {
-            if (s_kind[l] != kKindOutlet) {  // the coarse wave stores the outlets
-                fa[g] = s_la[l];
-                ++done;
-            }
-        } else if (s_done[l] == (kLaDone | kLaWaits)) {
-            int ntd = 0, up = l;
-#pragma unroll
-            for (int d = 0; d < 8; ++d) {
-                const int nlx = lx + dir_dx(d), nly = ly + dir_dy(d);
-                const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-                if (in_tile(nlx, nly) && donates(s_code[nh], d) && s_cls[nh] == kCellIn &&
-                    (s_done[nly * kTile + nlx] & kLaWaits)) {
-                    ++ntd;
-                    up = nly * kTile + nlx;
-                }
-            }
-            nd = (s_ext[l] != 0 || ntd >= 2 || s_kind[l] == kKindOutlet) ? 1 : (up << 16);
+        if ((s_info[l] & (kLaDone | kLaWaits)) == kLaDone && (s_info[l] & kLaKind) != kKindOutlet) {
+            fa[g] = s_la[l];  // (the coarse wave stores the outlets)
+            ++done;
         }
-        s_nd[l] = nd;
     }
     done = wsum(done);
     dem = __reduce_max_sync(0xffffffffu, dem);  // one DEM per tile
     if (count && (threadIdx.x & 31) == 0 && done && dem >= 0) atomicAdd(&dc.out[dem].fa_done, done);
-    __syncthreads();
-    // pointer jumping: every cell between nodes finds the node at the top of its run
-    for (int it = 0; it < 10; ++it) {  // in-tile runs are shorter than 2^10 cells
-        int32_t nu[4];
-        bool ch = false;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int l = (ly0 + 8 * q) * kTile + lx;
-            nu[q] = -1;
-            const int32_t v = s_nd[l];
-            if (s_done[l] != (kLaDone | kLaWaits) || (v & 0xffff)) continue;
-            const int32_t vp = s_nd[v >> 16];
-            if (vp & 0xffff) continue;  // at the top
-            nu[q] = vp & ~0xffff;
-            ch = true;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (nu[q] >= 0) s_nd[(ly0 + 8 * q) * kTile + lx] = nu[q];
-        if (!__syncthreads_or(ch)) break;
-    }
-    // node indices in the order the wave reached the cells (inputs first):
-    // warp w numbers the nodes among queue entries 128 w .. 128 w + 127
+    // node indices in level order (inputs first): warp w numbers the nodes among queue entries 128 w .. 128 w + 127
     {
-        const int qn = s_qn, wq = threadIdx.x >> 5;
+        const int wq = threadIdx.x >> 5;
         const unsigned below = (1u << lx) - 1u;
         unsigned b[4];
         int cnt = 0;
@@ -559,8 +527,7 @@ __global__ void __launch_bounds__(256, 8)
             const int i = wq * 128 + r * 32 + lx;
             bool isn = false;
             if (i < qn) {
-                const int c = s_q[i];
-                isn = s_done[c] == (kLaDone | kLaWaits) && (s_nd[c] & 0xffff);
+                isn = (s_nd[entry_cell(s_ent[i])] & 0xffff) != 0;
             }
             b[r] = __ballot_sync(0xffffffffu, isn);
             cnt += __popc(b[r]);
@@ -571,7 +538,7 @@ __global__ void __launch_bounds__(256, 8)
         for (int i = 0; i < wq; ++i) base += s_wcnt[i];
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
-            if ((b[r] >> lx) & 1u) s_nd[s_q[wq * 128 + r * 32 + lx]] = base + __popc(b[r] & below) + 1;
+            if ((b[r] >> lx) & 1u) s_nd[entry_cell(s_ent[wq * 128 + r * 32 + lx])] = base + __popc(b[r] & below) + 1;
             base += __popc(b[r]);
         }
         if (threadIdx.x == 255) s_nn = base;  // the last warp's end is the total
@@ -580,28 +547,23 @@ __global__ void __launch_bounds__(256, 8)
     const size_t tb = (size_t)t * kTile * kTile, pool = (size_t)t * kTilePool;
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
-        const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
+        const int ly = ly0 + 8 * q, l = ly * kTile + lx;
         const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
         const int32_t v = s_nd[l];
-        const bool waits = s_done[l] == (kLaDone | kLaWaits), outlet = s_kind[l] == kKindOutlet;
+        const bool waits = (s_info[l] & kLaWaits) != 0, outlet = (s_info[l] & kLaKind) == kKindOutlet;
         const int e = warp_slot(waits || outlet, &s_fn);
         if (outlet) {  // counted once the coarse wave stored it
             f_idx[tb + e] = make_int2((int)g, kLaOutlet);
         } else if (waits) {
-            const int node = (v & 0xffff) ? (v & 0xffff) - 1 : (s_nd[v >> 16] & 0xffff) - 1;
+            const int node = (v & 0xffff) ? (v & 0xffff) - 1 : (s_nd[(v >> 16) & kPtr] & 0xffff) - 1;
             f_idx[tb + e] = make_int2((int)g, node);
             f_la[tb + e] = s_la[l];
         }
         if (!waits || !(v & 0xffff)) continue;
-        // the node's inputs, in the donors' scan order: cells of other tiles, then node indices (negated)
-        int nin = 0;
-#pragma unroll
-        for (int d = 0; d < 8; ++d) {
-            const int nlx = lx + dir_dx(d), nly = ly + dir_dy(d);
-            const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-            if (!donates(s_code[nh], d) || s_cls[nh] != kCellIn) continue;
-            if (!in_tile(nlx, nly) || (s_done[nly * kTile + nlx] & kLaWaits)) ++nin;
-        }
+        // the node's inputs, in the donors' scan order: cells of other tiles and
+        // node indices (negated)
+        const uint32_t dm = s_dm[l];
+        const int nin = __popc(dm >> 8);
         const int start = atomicAdd(&s_pool, nin);
         if (start + nin > kTilePool) {
             raise_error(&sc->err, ErrFlags::kCapacity);
@@ -609,19 +571,15 @@ __global__ void __launch_bounds__(256, 8)
         }
         int m = 0;
 #pragma unroll 1
-        for (int kk = 0; kk < 8; ++kk) {
-            const int d = scan_dir(kk);
-            const int nlx = lx + dir_dx(d), nly = ly + dir_dy(d);
-            const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-            if (!donates(s_code[nh], d) || s_cls[nh] != kCellIn) continue;
+        for (uint32_t b = dm >> 8; b; b &= b - 1) {
+            const int kk = __ffs(b) - 1;
             int32_t ref;
-            if (!in_tile(nlx, nly)) {
-                ref = (ty0 + nly) * W + tx0 + nlx;
+            if ((dm >> kk) & 1u) {
+                const int32_t vu = s_nd[l + scan_step(kk)];
+                ref = -((vu & 0xffff) ? (vu & 0xffff) : (s_nd[(vu >> 16) & kPtr] & 0xffff));
             } else {
-                const int u = nly * kTile + nlx;
-                if (!(s_done[u] & kLaWaits)) continue;
-                const int32_t vu = s_nd[u];
-                ref = -((vu & 0xffff) ? (vu & 0xffff) : (s_nd[vu >> 16] & 0xffff));
+                const int d = scan_dir(kk);
+                ref = (ty0 + ly + dir_dy(d)) * W + tx0 + lx + dir_dx(d);
             }
             n_ref[pool + start + m] = ref;
             ++m;

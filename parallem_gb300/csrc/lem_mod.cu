@@ -713,7 +713,7 @@ __global__ void __launch_bounds__(256, 5)
     // tile each waiting cell's stone is a map of one program node's value,
     // stored by the final pass.
     const bool second_wave = __syncthreads_or(stray);
-    list_outlets(s_kind, s_olist, s_oslot, &s_no, s_wcnt);
+    list_outlets(s_kind, 0xff, s_olist, s_oslot, &s_no, s_wcnt);
     __syncthreads();
     // inflows per outlet (ring cells flowing into the tile)
     if (threadIdx.x < kRing) {

@@ -194,18 +194,18 @@ __device__ __forceinline__ bool in_tile(int lx, int ly) { return lx >= 0 && lx <
 // index step of direction d inside a tile (row-major, kTile cells per row)
 __device__ __forceinline__ int tile_step(int d) { return dir_dy(d) * kTile + dir_dx(d); }
 
-// The outlets of a 32x32 tile (cells whose receiver lies in another tile) in
-// cell order, with each outlet's slot: warp w ballots rows 4w..4w+3, and a
+// The outlets of a 32x32 tile (cells whose receiver lies in another tile: kind
+// kKindOutlet in `bits` of s_kind) in cell order, with each outlet's slot: warp w ballots rows 4w..4w+3, and a
 // prefix over the 8 warps' counts places them.  Called by all 256 threads;
 // s_wcnt holds 8 ints; the caller synchronises before reading the lists.
-__device__ __forceinline__ void list_outlets(const uint8_t* s_kind, int16_t* s_olist, int16_t* s_oslot, int* s_no,
+__device__ __forceinline__ void list_outlets(const uint8_t* s_kind, uint8_t bits, int16_t* s_olist, int16_t* s_oslot, int* s_no,
                                              int* s_wcnt) {
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     unsigned m[4];
     int cnt = 0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-        m[r] = __ballot_sync(0xffffffffu, s_kind[(4 * w + r) * kTile + lane] == kKindOutlet);
+        m[r] = __ballot_sync(0xffffffffu, (s_kind[(4 * w + r) * kTile + lane] & bits) == kKindOutlet);
         cnt += __popc(m[r]);
     }
     if (lane == 0) s_wcnt[w] = cnt;
@@ -254,6 +254,221 @@ __device__ __forceinline__ int ring_halo(int i) {
     return (i - 2 * kTH - kTile + 1) * kTH + kTH - 1;
 }
 
+// Stages the direction codes and classes of a tile and its halo (256 threads; all
+// loads of a thread in flight at once), class_of(grid cell, x, y) called for
+// cells in the grid.  Every cell also announces itself to the cell of the tile it
+// points at: s_dm (zero before, a barrier since) gets bit k of the receiver set
+// when its neighbour in direction scan_dir(k) drains to it, in the low byte for
+// cells of the tile and in the high byte for others; and s_bad the rows of the
+// cells with a donor that never completes (a blocked cell, whose code may have
+// several directions).  One push per cell in the place of eight tests.  Codes of
+// more than one direction occur in blocked cells only.  The caller synchronises.
+template <class ClassOf>
+__device__ __forceinline__ void tile_stage(const uint8_t* __restrict__ fd, const ClassOf& class_of, int W, int H,
+                                           int tx0, int ty0, uint8_t* s_code, uint8_t* s_cls, uint16_t* s_dm,
+                                           uint32_t* s_bad) {
+    constexpr int kTurns = (kTH * kTH + 255) / 256;
+    uint8_t code[kTurns], cls[kTurns];
+#pragma unroll
+    for (int i = 0; i < kTurns; ++i) {
+        const int j = threadIdx.x + 256 * i, hy = j / kTH, hx = j - hy * kTH;
+        const int gx = tx0 - 1 + hx, gy = ty0 - 1 + hy;
+        code[i] = 0;
+        cls[i] = kCellOff;
+        if (j < kTH * kTH && gx >= 0 && gx < W && gy >= 0 && gy < H) {
+            const size_t g = (size_t)gy * W + gx;
+            code[i] = fd[g];
+            cls[i] = class_of(g, gx, gy);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kTurns; ++i) {
+        const int j = threadIdx.x + 256 * i, hy = j / kTH, hx = j - hy * kTH;
+        if (j >= kTH * kTH) continue;
+        s_code[j] = code[i];
+        s_cls[j] = cls[i];
+        if (cls[i] == kCellOff) continue;
+        for (uint32_t m = code[i]; m; m &= m - 1) {
+            const int b = __ffs(m) - 1, d = (b + 2) & 7;  // bit b of a code is direction (b + 2) % 8
+            const int rx = hx - 1 + dir_dx(d), ry = hy - 1 + dir_dy(d);
+            if (!in_tile(rx, ry)) continue;
+            const int r = ry * kTile + rx;
+            if (cls[i] == kCellBlock) {
+                atomicOr(&s_bad[ry], 1u << rx);
+            } else {
+                const int k = scan_index((d + 4) & 7) + (in_tile(hx - 1, hy - 1) ? 0 : 8);
+                atomicOr(reinterpret_cast<uint32_t*>(s_dm) + (r >> 1), 1u << (k + 16 * (r & 1)));
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The in-tile dependency order of one block (256 threads, thread (lx, ly0)
+// holds the cells of column lx in rows ly0 + 8 q).
+//
+// s_pd of a cell: the cell its path reaches after 2^k steps, or where the path
+// ends before that (low 10 bits), and the steps to it (above).  Doubling k
+// takes every cell to its path's end, and on the way each cell hands the cell
+// exactly 2^k steps down what lies above it: the length of the longest path
+// that ends there (s_h, its level: every donor has a smaller one) and two flags
+// (bit sets of 32 words, a row each).  A path that has not ended after 2^10
+// steps runs into a cycle; its cells after as many steps, all of the cycle,
+// join s_bad.  log2 of the longest path rounds, all threads at work, in the place
+// of a queue of released cells whose order costs an atomic and a vote per cell.
+constexpr int kWaveBlockMin = 96;
+constexpr int kPtr = kTile * kTile - 1;  // the pointer bits of s_pd
+__device__ __forceinline__ void tile_paths(int32_t* s_pd, int32_t* s_h, uint32_t* s_wait, uint32_t* s_bad, int lx,
+                                           int ly0) {
+    for (int k = 0;; ++k) {
+        int32_t next[4];
+        int up[4];
+        uint32_t flags = 0;
+        bool any = false;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int l = (ly0 + 8 * q) * kTile + lx;
+            const int32_t v = s_pd[l];
+            up[q] = -1;
+            next[q] = 0;
+            if ((v >> 10) == 1 << k) {
+                const int32_t v2 = s_pd[v & kPtr];
+                next[q] = (v2 & kPtr) | (((v >> 10) + (v2 >> 10)) << 10);
+                up[q] = (v & kPtr) | ((s_h[l] + (1 << k)) << 10);
+                flags |= ((s_wait[l >> 5] >> lx) & 1u) << q | ((s_bad[l >> 5] >> lx) & 1u) << (q + 4);
+                any = true;
+            }
+        }
+        if (!__syncthreads_or(any)) break;
+        if (k == 10) {  // into a cycle
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                if (up[q] >= 0) atomicOr(&s_bad[(up[q] & kPtr) >> 5], 1u << (up[q] & 31));
+            break;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (up[q] < 0) continue;
+            const int p = up[q] & kPtr;
+            s_pd[(ly0 + 8 * q) * kTile + lx] = next[q];
+            atomicMax(&s_h[p], up[q] >> 10);
+            if ((flags >> q) & 1u) atomicOr(&s_wait[p >> 5], 1u << (p & 31));
+            if ((flags >> (q + 4)) & 1u) atomicOr(&s_bad[p >> 5], 1u << (p & 31));
+        }
+        __syncthreads();
+    }
+    __syncthreads();
+}
+
+// Sorts the cells with key[q] >= 0 (below 2 * words) by key and counts them in
+// *s_total: s_ent holds pack(q) of each.  s_bins (`words` words, zero before)
+// then holds where each key's cells end, 16 bits a key, up to the first keys
+// without cells (of 64 in a row none may be empty before the last one used).
+// Every thread calls it.
+__device__ __forceinline__ int bin_end(const uint32_t* s_bins, int key) {
+    return (s_bins[key >> 1] >> (16 * (key & 1))) & 0xffff;
+}
+template <class Pack>
+__device__ __forceinline__ void tile_sort(const int (&key)[4], const Pack& pack, uint32_t* s_bins, int words,
+                                          uint32_t* s_ent, int* s_total, int lx) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (key[q] >= 0) atomicAdd(&s_bins[key[q] >> 1], 1u << (16 * (key[q] & 1)));
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        uint32_t carry = 0;
+        for (int b = lx; b < words; b += 32) {
+            const uint32_t v = s_bins[b], lo = v & 0xffff, n = lo + (v >> 16);
+            uint32_t incl = n;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lx >= d) incl += u;
+            }
+            const uint32_t at = carry + incl - n, all = __shfl_sync(0xffffffffu, incl, 31);
+            s_bins[b] = at | ((at + lo) << 16);
+            if (all == 0) break;
+            carry += all;
+        }
+        if (lx == 0) *s_total = (int)carry;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q)
+        if (key[q] >= 0) {
+            const int sh = 16 * (key[q] & 1);
+            const int at = (atomicAdd(&s_bins[key[q] >> 1], 1u << sh) >> sh) & 0xffff;
+            s_ent[at] = pack(q);
+        }
+    __syncthreads();
+}
+
+// A cell of the sorted list with its first two in-tile donors: the cell in 11
+// bits (kNoCell: a cell that the caller lays out behind the tile's, of no effect),
+// the first donor as a step (7 bits), the second in 11 bits (kNoCell: none), and
+// whether there are more.
+constexpr int kNoCell = kTile * kTile;
+constexpr uint32_t kNoEntry = kNoCell | (64u << 11) | ((uint32_t)kNoCell << 18);
+constexpr uint32_t kMoreDonors = 1u << 29;
+// index step of direction scan_dir(k): +1, +33, +32, +31, then their negatives
+__device__ __forceinline__ int scan_step(int k) {
+    const int v = (0x1F202101 >> (8 * (k & 3))) & 0xff;
+    return k & 4 ? -v : v;
+}
+__device__ __forceinline__ uint32_t entry_of(int c, uint32_t donors) {  // donors: bit k for direction scan_dir(k)
+    const uint32_t m = donors & (donors - 1);
+    const int o0 = donors ? scan_step(__ffs(donors) - 1) : 0;
+    const int d1 = m ? c + scan_step(__ffs(m) - 1) : kNoCell;
+    return (uint32_t)c | (uint32_t)(o0 + 64) << 11 | (uint32_t)d1 << 18 | (m & (m - 1) ? kMoreDonors : 0u);
+}
+__device__ __forceinline__ int entry_cell(uint32_t e) { return e & 2047; }
+__device__ __forceinline__ int entry_d0(uint32_t e) { return (int)(e & 2047) + (int)((e >> 11) & 127) - 64; }
+__device__ __forceinline__ int entry_d1(uint32_t e) { return (e >> 18) & 2047; }
+
+// Runs op(fetch(entry)) on the sorted entries of the keys from `first` on, key by
+// key: a key's cells depend on smaller keys only.  A key has no more cells than
+// the one before (each cell of a level has a donor of its own in the level
+// above): the first keys, of more than 32 cells, run on every thread with a block
+// barrier each, the others on warp 0 alone until one is empty.  There the chain of
+// keys sets the time, and a warp issues in order, so nothing but op stands in it:
+// entries are read two keys ahead and what fetch reads (nothing that op writes for
+// another cell) one key ahead; finding the donors from direction bits in the chain
+// took a third of it.
+template <class Fetch, class Op>
+__device__ __forceinline__ void tile_levels(const Fetch& fetch, const Op& op, int first, int keys,
+                                            const uint32_t* s_bins, const uint32_t* s_ent) {
+    int key = first, start = first ? bin_end(s_bins, first - 1) : 0;
+    for (; key < keys; ++key) {
+        const int end = bin_end(s_bins, key);
+        if (end - start <= 32) break;  // block-uniform
+        for (int i = start + threadIdx.x; i - (int)(threadIdx.x & 31) < end; i += blockDim.x)  // whole warps
+            op(fetch(i < end ? s_ent[i] : kNoEntry));
+        __syncthreads();
+        start = end;
+    }
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        auto end_of = [&](int k) { return k < keys ? bin_end(s_bins, k) : 0; };
+        auto entry_at = [&](int from, int to) { return lane < to - from ? s_ent[from + lane] : kNoEntry; };
+        int end = end_of(key), next = end_of(key + 1), after = end_of(key + 2);
+        auto got = fetch(entry_at(start, end));
+        uint32_t en = entry_at(end, next);
+        while (end > start) {
+            const uint32_t ea = entry_at(next, after);
+            const auto gotn = fetch(en);
+            start = end;
+            end = next;
+            next = after;
+            after = end_of(++key + 2);
+            op(got);
+            __syncwarp();
+            got = gotn;
+            en = ea;
+        }
+    }
+    __syncthreads();
+}
+
 // The in-tile dependency wave of one block, in rounds: a round takes every
 // queued cell (all its donors in the tile finished), computes it with
 // op(c, round), which returns the in-tile receiver it releases (or -1), and
@@ -263,7 +478,6 @@ __device__ __forceinline__ int ring_halo(int i) {
 // block; the narrow rounds after them run on warp 0 alone, with a warp barrier
 // between rounds and the queue appended by ballot, while the block's other
 // warps wait at one block barrier (the SM runs other blocks meanwhile).
-constexpr int kWaveBlockMin = 96;
 template <class Op>
 __device__ __forceinline__ void tile_wave(const Op& op, int32_t* s_pend, int16_t* s_q, int* s_qn, int* s_end,
                                           const bool (&src)[4], int lx, int ly0) {
