@@ -137,7 +137,7 @@ struct lem_handle {
     bool profiling = false;
     bool graphs = false;           // steps replay a captured CUDA graph (lem_set_graphs)
     cudaGraphExec_t gexec = nullptr;
-    int32_t gkey[3] = {-1, -1, -1};  // chunks, visited tiles and step flags the graph was captured for
+    int32_t gkey[4] = {-1, -1, -1, -1};  // chunks, their size, visited tiles and step flags the graph was captured for
     uint64_t glaunches = 0;        // kernel launches in one replay
     int sms = 0;                   // SMs of the handle's device
     Tuner tune;
@@ -296,6 +296,10 @@ lem_status prepare(lem_handle* h) {
     std::vector<DemIn> in(n);
     std::vector<int32_t> chunk(n + 1, 0);
     bool any = false;
+    int64_t cells = 0;
+    for (const HostDem& r : h->dems)
+        if (r.active) cells += (int64_t)r.w * r.h;
+    const int32_t per_block = h->s.dems.chunk = streaming_chunk(cells);
     for (int d = 0; d < n; ++d) {
         const HostDem& r = h->dems[d];
         DemIn& o = in[d];
@@ -317,7 +321,7 @@ lem_status prepare(lem_handle* h) {
         o.rain0 = r.rain0;
         o.temp0 = r.temp0;
         o.rain0_inc = (r.rain0 * 2 - r.rain0) / r.h;
-        chunk[d + 1] += (int32_t)(((int64_t)r.w * r.h + kChunk - 1) / kChunk);
+        chunk[d + 1] += (int32_t)(((int64_t)r.w * r.h + per_block - 1) / per_block);
     }
     if (!any) return LEM_ERR_STATE;
     // pageable sources: the copies take the data before returning
@@ -771,7 +775,7 @@ lem_status create_common(const lem_grid_desc* grid, const lem_params* params, in
     }
 #undef ALLOC
     s.chunk_start = h->chunks;
-    s.dems = DemCtx{h->dem_of, h->dem_in, h->dem_out, max_dems};
+    s.dems = DemCtx{h->dem_of, h->dem_in, h->dem_out, max_dems, kChunkMax};
     s.live = nullptr;  // a single grid visits every tile; a batch lists its DEMs' tiles before each stage
     s.n_live = (int32_t)(((grid->width + kTile - 1) / kTile) * ((grid->height + kTile - 1) / kTile));
     std::vector<float> tab;
@@ -934,7 +938,7 @@ lem_status graph_step(lem_handle* h, uint32_t flags) {
     if (r != LEM_OK) return r;
     uint32_t f = flags & ~LEM_STEP_SET_OUTLET_FROM_FA;
     if (any_flag(h, LEM_STEP_SET_OUTLET_FROM_FA)) f |= LEM_STEP_SET_OUTLET_FROM_FA;
-    const int32_t key[3] = {h->s.n_chunks, h->s.n_live, (int32_t)f};
+    const int32_t key[4] = {h->s.n_chunks, h->s.dems.chunk, h->s.n_live, (int32_t)f};
     if (!h->gexec || std::memcmp(key, h->gkey, sizeof key) != 0) {
         if (h->gexec) {
             cudaGraphExecDestroy(h->gexec);

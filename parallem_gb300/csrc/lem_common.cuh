@@ -159,6 +159,7 @@ struct DemCtx {
     const DemIn* in;
     DemOut* out;
     int32_t n;           // DEM slots
+    int32_t chunk;       // cells of a streaming pass's block (streaming_chunk)
 };
 __device__ __forceinline__ int dem_at(const DemCtx& dc, size_t cell) { return dc.of ? (int)dc.of[cell] : 0; }
 

@@ -168,17 +168,28 @@ inline TileSet tiles_of(const DevState& s, int W) {
     return TileSet{s.live, s.n_live, (W + kTile - 1) / kTile};
 }
 
-// Streaming passes over the DEMs' regions run one block per chunk of kChunk
-// cells, every chunk inside one DEM, so block sums go to that DEM's totals.
-constexpr int kChunk = 4096;
+// Streaming passes over the DEMs' regions run one block per chunk of cells, every
+// chunk inside one DEM, so block sums go to that DEM's totals.  A block takes up
+// to 4096 cells, 16 per thread, one after the other; on grids that would not give
+// every SM two blocks of that size it takes fewer, down to four cells per thread
+// (a 96 x 96 grid: k_final 41 us in blocks of 4096 cells; 512 x 512 cells in
+// blocks of 256: 36 us, most of it the blocks' atomics on the totals).  The sums
+// do not depend on the size (BlockSums).
+constexpr int kChunkMax = 4096, kChunkMin = 1024;
+inline int32_t streaming_chunk(int64_t cells) {
+    int32_t c = kChunkMax;
+    while (c > kChunkMin && cells / c < 2 * 152) c /= 2;
+    return c;
+}
 struct Chunk {
     int d;          // DEM
     int64_t first;  // first region-linear cell of the chunk
     int64_t end;    // one past the last
 };
-__device__ __forceinline__ Chunk chunk_of(const int32_t* chunk_start, int n, const DemIn* in) {
+__device__ __forceinline__ Chunk chunk_of(const int32_t* chunk_start, const DemCtx& dc) {
+    const DemIn* const in = dc.in;
     // the DEM whose chunk range holds blockIdx.x (n is small: binary search)
-    int lo = 0, hi = n;
+    int lo = 0, hi = dc.n;
     const int b = blockIdx.x;
     while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
@@ -186,9 +197,9 @@ __device__ __forceinline__ Chunk chunk_of(const int32_t* chunk_start, int n, con
     }
     Chunk c;
     c.d = lo;
-    c.first = (int64_t)(b - chunk_start[lo]) * kChunk;
+    c.first = (int64_t)(b - chunk_start[lo]) * dc.chunk;
     const int64_t cells = (int64_t)in[lo].w * in[lo].h;
-    c.end = c.first + kChunk < cells ? c.first + kChunk : cells;
+    c.end = c.first + dc.chunk < cells ? c.first + dc.chunk : cells;
     return c;
 }
 // grid index of region-linear cell i of DEM region r

@@ -50,7 +50,7 @@ __global__ void k_fa_prep(const uint8_t* __restrict__ mask, const uint8_t* __res
                           float* __restrict__ w, float2* __restrict__ fa, const int32_t* __restrict__ chunk_start,
                           ModelConsts k, DemCtx dc, DevScalars* sc) {
     const int W = k.W;
-    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    const Chunk ch = chunk_of(chunk_start, dc);
     const DemIn& r = dc.in[ch.d];
     const float rain0 = (float)r.rain, rinc = (float)r.rain_inc;
     int nact = 0;
@@ -110,7 +110,7 @@ __global__ void k_fa_pend(const double* __restrict__ z, const uint8_t* __restric
     if (gate && sc->tiled_ok) return;  // the tiled path accumulates this step
     const int W = k.W, H = k.H;
     const size_t N = (size_t)W * H;
-    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    const Chunk ch = chunk_of(chunk_start, dc);
     const DemIn& r = dc.in[ch.d];
     for (int64_t base = ch.first; base < ch.end; base += blockDim.x) {
         const int64_t ri = base + threadIdx.x;
@@ -891,7 +891,7 @@ __global__ void __launch_bounds__(256)
 __global__ void k_count_init(const uint8_t* __restrict__ mask, float2* __restrict__ cnt,
                              const int32_t* __restrict__ chunk_start, int W, DemCtx dc, DevScalars* sc) {
     if (!sc->tiled_ok) return;
-    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    const Chunk ch = chunk_of(chunk_start, dc);
     if (blockIdx.x == 0 && threadIdx.x == 0) sc->tile_src = 0;
     for (int64_t ri = ch.first + threadIdx.x; ri < ch.end; ri += blockDim.x) {
         int x, y;
@@ -902,7 +902,7 @@ __global__ void k_count_init(const uint8_t* __restrict__ mask, float2* __restric
 __global__ void k_count_out(const float2* __restrict__ cnt, int32_t* __restrict__ contrib,
                             const int32_t* __restrict__ chunk_start, int W, DemCtx dc, DevScalars* sc) {
     if (!sc->tiled_ok) return;
-    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    const Chunk ch = chunk_of(chunk_start, dc);
     for (int64_t ri = ch.first + threadIdx.x; ri < ch.end; ri += blockDim.x) {
         int x, y;
         const size_t i = region_cell(dc.in[ch.d], ri, W, &x, &y);
@@ -961,7 +961,7 @@ lem_status launch_fat(const FatArgs& a, const ModelConsts& k, const TileSet& ts,
 // becomes the first cell holding the largest accumulation.
 __global__ void k_fa_argmax(const float2* __restrict__ fa, const int32_t* __restrict__ chunk_start, int W,
                             DemCtx dc, int phase) {
-    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    const Chunk ch = chunk_of(chunk_start, dc);
     const DemIn& r = dc.in[ch.d];
     DemOut& o = dc.out[ch.d];
     if (!r.outlet_from_fa) return;
@@ -1227,7 +1227,7 @@ extern "C" lem_status lem_accumulate_flow_noalloc(const int32_t* d_fd, const dou
     ModelConsts k{};
     k.W = width;
     k.H = height;
-    const DemCtx dc{nullptr, nullptr, dem, 1};
+    const DemCtx dc{nullptr, nullptr, dem, 1, kChunkMax};
     uint64_t launches = 0;
     const Launch L{st, &launches, nullptr};
     k_na_reset<<<1, 1, 0, st>>>(sc, dem, tiled);  // the array keeps the previous call's contents

@@ -35,22 +35,44 @@ __device__ __forceinline__ float clim_temp(const DemIn& c, const double* z, cons
     return (float)c.temp - ((hi - (float)kMinHeight) + lo) * 0.0065f;
 }
 
-__device__ __forceinline__ double block_sum_d(float v, double* red) {
-    // fp32 warp partials, fp64 across warps
-    v += __shfl_xor_sync(0xffffffffu, v, 16);
-    v += __shfl_xor_sync(0xffffffffu, v, 8);
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    v += __shfl_xor_sync(0xffffffffu, v, 2);
-    v += __shfl_xor_sync(0xffffffffu, v, 1);
-    const int wid = threadIdx.x >> 5;
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[wid] = (double)v;
-    __syncthreads();
-    double t = 0.0;
-    if (threadIdx.x == 0)
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) t += red[i];
-    return t;
-}
+// K sums of fp32 terms over a block of 256 threads: fp32 over a warp's 128 cells
+// (four turns of the loop), fp64 from there on, so the totals depend on the size
+// of the blocks only in the last bits of fp64.  turn() is called by every thread
+// after every cell, finish() by every thread at the end; add_to's thread k < K
+// then holds sum k.
+template <int K>
+struct BlockSums {
+    double (*red)[K];  // [8] in shared memory
+    float v[K];
+    int turns = 0;
+    __device__ __forceinline__ explicit BlockSums(double (*r)[K]) : red(r) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            v[k] = 0.f;
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] = 0.0;
+        }
+    }
+    __device__ __forceinline__ void flush() {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+            if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][k] += (double)v[k];
+            v[k] = 0.f;
+        }
+    }
+    __device__ __forceinline__ void turn() {
+        if ((++turns & 3) == 0) flush();
+    }
+    __device__ __forceinline__ double finish() {
+        if (turns & 3) flush();
+        __syncthreads();
+        double t = 0.0;
+        if (threadIdx.x < K)
+            for (int w = 0; w < 8; ++w) t += red[w][threadIdx.x];
+        return t;
+    }
+};
 
 __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v, unsigned long long* red) {
     for (int o = 16; o > 0; o >>= 1) {
@@ -67,8 +89,8 @@ __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v
     return m;
 }
 
-// five blocks per SM: a few spilled registers, measured faster than four or six
-__global__ void __launch_bounds__(256, 5)
+// six blocks per SM: a few spilled registers, measured faster than four or five
+__global__ void __launch_bounds__(256, 6)
     k_erosion(const double* __restrict__ z, const double* __restrict__ z_init, const uint8_t* __restrict__ mask,
               const float* __restrict__ slopes, const float2* __restrict__ fa, const float* __restrict__ fines,
               const float* __restrict__ nut, const float* __restrict__ soilT, const float* __restrict__ stone,
@@ -76,9 +98,9 @@ __global__ void __launch_bounds__(256, 5)
               float* __restrict__ inci, float* __restrict__ geli, float* __restrict__ depo,
               const uint8_t* __restrict__ fd, const int32_t* __restrict__ chunk_start, ModelConsts k, DemCtx dc,
               DevScalars* sc) {
-    __shared__ double red[8];
+    __shared__ double red[8][3];
     __shared__ unsigned long long redk[8];
-    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    const Chunk ch = chunk_of(chunk_start, dc);
     const DemIn& c = dc.in[ch.d];
     DemOut& o = dc.out[ch.d];
     const int W = k.W;
@@ -86,10 +108,10 @@ __global__ void __launch_bounds__(256, 5)
     const int outlet_clim = o.outlet_clim;  // the cell whose climate elevation is outlet_z_clim
     const double outlet_z = o.outlet_z_clim;
     if (ch.first == 0 && threadIdx.x == 0) o.base_level = z[outlet] - 0.00012;  // updates.cu:151
-    float se = 0.f, si = 0.f, sg = 0.f;
+    BlockSums<3> sums(red);
     unsigned long long famax = 0;
     bool multi = false;
-    for (int64_t ri = ch.first + threadIdx.x; ri < ch.end; ri += blockDim.x) {
+    auto cell = [&](int64_t ri) {
         int x, y;
         const size_t i = region_cell(c, ri, W, &x, &y);
         // every input of the cell in one batch of loads, ahead of the mask test
@@ -105,7 +127,7 @@ __global__ void __launch_bounds__(256, 5)
         if (!mk) {
             ero[i] = inci[i] = geli[i] = 0.0f;
             slopeptr[i] = 0.0f;
-            continue;
+            return;
         }
         // sedmfdaccum set-up (mfd_accum.cu:389-396): depo = 1e-5 in the catchment.
         // A multi-direction code among the routed cells (not row 0 / column 0,
@@ -183,19 +205,19 @@ __global__ void __launch_bounds__(256, 5)
         ero[i] = e;
         inci[i] = in;
         geli[i] = g;
-        se += e;
-        si += in;
-        sg += g;
+        sums.v[0] += e;
+        sums.v[1] += in;
+        sums.v[2] += g;
+    };
+    for (int64_t r0 = ch.first; r0 < ch.end; r0 += blockDim.x) {
+        if (r0 + threadIdx.x < ch.end) cell(r0 + threadIdx.x);
+        sums.turn();
     }
-    const double te = block_sum_d(se, red);
-    const double ti = block_sum_d(si, red);
-    const double tg = block_sum_d(sg, red);
+    const double total = sums.finish();
+    if (threadIdx.x < 3) atomicAdd(threadIdx.x == 0 ? &o.tot_e : threadIdx.x == 1 ? &o.tot_i : &o.tot_g, total);
     const unsigned long long fm = block_max_u64(famax, redk);
     const bool any_multi = __syncthreads_or(multi) != 0;
     if (threadIdx.x == 0) {
-        atomicAdd(&o.tot_e, te);
-        atomicAdd(&o.tot_i, ti);
-        atomicAdd(&o.tot_g, tg);
         atomicMax(&o.fa_max_key, fm);
         if (any_multi) sc->sed_tiled_ok = 0;
     }
@@ -1407,9 +1429,9 @@ __global__ void __launch_bounds__(256, 6)
             float* __restrict__ soilB, float* __restrict__ nut, float* __restrict__ totB, float* __restrict__ dz_out,
             float* __restrict__ wc_out, float* __restrict__ wp_out, const float* __restrict__ tab,
             const int32_t* __restrict__ chunk_start, ModelConsts k, DemCtx dc) {
-    __shared__ double red[8];
+    __shared__ double red[8][4];
     const int W = k.W;
-    const Chunk ch = chunk_of(chunk_start, dc.n, dc.in);
+    const Chunk ch = chunk_of(chunk_start, dc);
     const DemIn& c = dc.in[ch.d];
     DemOut& o = dc.out[ch.d];
     const int outlet = o.outlet;
@@ -1418,8 +1440,8 @@ __global__ void __launch_bounds__(256, 6)
     const double base = o.base_level;
     const float rain0 = (float)c.rain, rinc = (float)c.rain_inc;
     const float dtemp_scalar = (float)(c.temp - c.temp0);
-    float swc = 0.f, swp = 0.f, sbio = 0.f, sd = 0.f;
-    for (int64_t ri = ch.first + threadIdx.x; ri < ch.end; ri += blockDim.x) {
+    BlockSums<4> sums(red);
+    auto cell = [&](int64_t ri) {
         int x, y;
         const size_t i = region_cell(c, ri, W, &x, &y);
         // every input of the cell in one batch of loads, ahead of the mask test
@@ -1430,7 +1452,7 @@ __global__ void __launch_bounds__(256, 6)
         const double zold = z[i], z0 = z_init[i];
         const float2 f2 = fa[i];
         const float st0 = soilT[i], sn0 = stone[i], sm0 = soilM[i], tb = totB[i], sb0 = soilB[i];
-        sd += dp;
+        sums.v[3] += dp;
         if (!mk) {
             totB[i] = 0.0f;  // grow_vegetation (updates.cu:102-105)
             if (dz_out) {
@@ -1438,7 +1460,7 @@ __global__ void __launch_bounds__(256, 6)
                 wc_out[i] = 0.f;
                 wp_out[i] = 0.f;
             }
-            continue;
+            return;
         }
         const float dz = dp - e - ic - gl;  // surface_change (eroincidep.cu:404)
         const double zc = c.from_current_dem ? (((int)i == outlet_clim) ? outlet_z : zold) : z0;
@@ -1542,20 +1564,21 @@ __global__ void __launch_bounds__(256, 6)
             wc_out[i] = wC;
             wp_out[i] = wP;
         }
-        swc += wC;
-        swp += wP;
-        sbio += nb;
+        sums.v[0] += wC;
+        sums.v[1] += wP;
+        sums.v[2] += nb;
+    };
+    for (int64_t r0 = ch.first; r0 < ch.end; r0 += blockDim.x) {
+        if (r0 + threadIdx.x < ch.end) cell(r0 + threadIdx.x);
+        sums.turn();
     }
-    const double t1 = block_sum_d(swc, red);
-    const double t2 = block_sum_d(swp, red);
-    const double t3 = block_sum_d(sbio, red);
-    const double t4 = block_sum_d(sd, red);
-    if (threadIdx.x == 0) {
-        atomicAdd(&o.tot_wc, t1);
-        atomicAdd(&o.tot_wp, t2);
-        atomicAdd(&o.tot_bio, t3);
-        atomicAdd(&o.tot_d, t4);
-    }
+    const double total = sums.finish();
+    if (threadIdx.x < 4)
+        atomicAdd(threadIdx.x == 0   ? &o.tot_wc
+                  : threadIdx.x == 1 ? &o.tot_wp
+                  : threadIdx.x == 2 ? &o.tot_bio
+                                     : &o.tot_d,
+                  total);
 }
 
 __global__ void k_mod_reset(DevScalars* sc, DemCtx dc, int tiled) {
