@@ -293,6 +293,16 @@ inline cudaError_t coop_launch(const void* fn, int blocks, void** args, cudaStre
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
+// Blocks of a cooperative kernel on a grid of that many 32x32 tiles: its schedule's
+// blocks, or `per_tile` for each tile where those are fewer.  A grid-wide barrier of
+// 608 blocks takes about 3 us and one of nine less than half of that, and the
+// blocks beyond the work do nothing else (a 96 x 96 grid: k_plateau_relax 34 us
+// with 608 blocks).
+inline int coop_for(const DevState& s, int kernel, int tiles, int per_tile) {
+    const int64_t b = (int64_t)tiles * per_tile;
+    return b < s.coop_blocks[kernel] ? (b > 0 ? (int)b : 1) : s.coop_blocks[kernel];
+}
+
 // Blocks of the general dependency wave on n cells: a warp for every 256 cells
 // covers the front of a slope (a row or two of the grid); more only watch the
 // list.

@@ -1028,7 +1028,7 @@ lem_status launch_flow_accumulation(const DevState& s, const ModelConsts& k, uin
         const TileSet ts = tiles_of(s, k.W);
         FatArgs a{s.z, s.mask, s.fd, s.w, s.fa, s.t_rec, s.t_dst, s.t_pend, s.t_ent, s.n_meta, s.p_ref,
                   reinterpret_cast<int2*>(s.f_idx), s.f_ds, s.t_fcnt, s.list_b, s.list_a, s.sc, s.dems,
-                  s.coop_blocks[kCkFatCoarse]};
+                  coop_for(s, kCkFatCoarse, ts.n, 2)};
         lem_status r = launch_fat(a, k, ts, 1, L);
         if (r != LEM_OK) return r;
         if (contrib) {
@@ -1237,7 +1237,7 @@ extern "C" lem_status lem_accumulate_flow_noalloc(const int32_t* d_fd, const dou
                         word, static_cast<int32_t*>(at(kNaOffEnt)), static_cast<int32_t*>(at(kNaOffMeta)),
                         static_cast<int32_t*>(at(kNaOffRef)), static_cast<int2*>(at(kNaOffIdx)),
                         static_cast<float2*>(at(kNaOffLa)), static_cast<int32_t*>(at(kNaOffCnt)), list,
-                        static_cast<int32_t*>(at(kNaOffReady)), sc, dc, std::min(nd.coarse_blocks, tiles)};
+                        static_cast<int32_t*>(at(kNaOffReady)), sc, dc, std::min(nd.coarse_blocks, 2 * tiles)};
         const lem_status r = launch_fat(a, k, TileSet{nullptr, tiles, tw}, 1, L);
         if (r != LEM_OK) return r;
     }

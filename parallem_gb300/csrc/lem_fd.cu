@@ -911,10 +911,25 @@ __global__ void k_flood_merge(const double* __restrict__ z, int32_t* ws, const i
     if (gtid == 0) sc->flood_sweeps = round + 1;
 }
 
+// Live capacity of the basin-pair table: 8 slots per label that can own a
+// basin (the sink cells, plus basin 0), rounded up to a power of two, at
+// least 1024, at most the allocated capacity.  A basin borders about three
+// others on average (the basin graph is nearly planar), so the table is at
+// most about half full and linear probing stays short, and the table of a
+// grid with few sinks is small enough to stay in L2.
+__device__ __forceinline__ int edge_logcap(const DevScalars* sc, int logmax) {
+    const long long want = 8ll * ((long long)sc->n_sinks + 1);
+    int l = 10;
+    while (l < logmax && (1ll << l) < want) ++l;
+    const int lim = sc->edge_log_cap;  // lem_set_limits: a smaller table (full tables raise kCapacity)
+    return (lim > 0 && lim < l) ? lim : l;
+}
+
 // identify_watershedMFD loop (newflow.cu:469-487): pointer jumping until every
-// cell holds the label of the sink (or basin 0) its SFD path ends in.
-__global__ void k_flood_jump(int32_t* ws, int32_t* list_a, int32_t* list_b, ModelConsts k, DevScalars* sc,
-                             TileSet ts) {
+// cell holds the label of the sink (or basin 0) its SFD path ends in.  The live
+// part of the basin-pair table is emptied on the way.
+__global__ void k_flood_jump(int32_t* ws, int32_t* list_a, int32_t* list_b, unsigned long long* ekey,
+                             unsigned long long* ewt, int logmax, ModelConsts k, DevScalars* sc, TileSet ts) {
     if (sc->sinkcount_pass1 == 0) return;
     cg::grid_group grid = cg::this_grid();
     __shared__ int s_cnt[9];
@@ -926,6 +941,10 @@ __global__ void k_flood_jump(int32_t* ws, int32_t* list_a, int32_t* list_b, Mode
         cnt[0] = 0;
         cnt[1] = 0;
         cnt[2] = 0;
+    }
+    for (size_t i = gtid; i < (size_t)1 << edge_logcap(sc, logmax); i += gstride) {
+        ekey[i] = ~0ull;
+        ewt[i] = ~0ull;
     }
     grid.sync();
     // round 0 over every visited cell
@@ -978,29 +997,6 @@ __global__ void k_flood_jump(int32_t* ws, int32_t* list_a, int32_t* list_b, Mode
 
 __device__ __forceinline__ uint64_t edge_hash(unsigned long long key, int logcap) {
     return (key * 0x9E3779B97F4A7C15ull) >> (64 - logcap);
-}
-
-// Live capacity of the basin-pair table: 8 slots per label that can own a
-// basin (the sink cells, plus basin 0), rounded up to a power of two, at
-// least 1024, at most the allocated capacity.  A basin borders about three
-// others on average (the basin graph is nearly planar), so the table is at
-// most about half full and linear probing stays short, and the table of a
-// grid with few sinks is small enough to stay in L2.
-__device__ __forceinline__ int edge_logcap(const DevScalars* sc, int logmax) {
-    const long long want = 8ll * ((long long)sc->n_sinks + 1);
-    int l = 10;
-    while (l < logmax && (1ll << l) < want) ++l;
-    const int lim = sc->edge_log_cap;  // lem_set_limits: a smaller table (full tables raise kCapacity)
-    return (lim > 0 && lim < l) ? lim : l;
-}
-
-__global__ void k_edge_clear(unsigned long long* ekey, unsigned long long* ewt, int logmax, DevScalars* sc) {
-    if (sc->sinkcount_pass1 == 0) return;
-    const size_t cap = 1ull << edge_logcap(sc, logmax);
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (size_t)gridDim.x * blockDim.x) {
-        ekey[i] = ~0ull;
-        ewt[i] = ~0ull;
-    }
 }
 
 __device__ __forceinline__ void edge_insert(unsigned long long* ekey, unsigned long long* ewt, int logcap,
@@ -1431,6 +1427,7 @@ __global__ void k_flood_raise(const double* __restrict__ z, const uint8_t* __res
                               const int32_t* __restrict__ ws, const unsigned long long* __restrict__ raise,
                               double* __restrict__ zf, ModelConsts k, DevScalars* sc, DemCtx dc, TileSet ts) {
     if (sc->sinkcount_pass1 == 0) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) sc->n_cand = 0;  // the second pass lists its own candidates
     for (size_t v0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v0 < ts.span();
          v0 += (size_t)gridDim.x * blockDim.x) {
         int x, y;
@@ -1505,8 +1502,6 @@ __global__ void k_fd_reset(DevScalars* sc, DemCtx dc) {
     }
 }
 
-__global__ void k_cand_reset(DevScalars* sc) { sc->n_cand = 0; }
-
 }  // namespace
 
 int coop_blocks_for(const void* kernel, int threads, size_t smem) {
@@ -1557,7 +1552,6 @@ static lem_status direction_pass(const DevState& s, const ModelConsts& k, const 
     const dim3 fdb(FD_BX, FD_BY), fdg(ts.n, kTile / FD_BY);
     const double* zz = pass == 1 ? s.z : s.zf;
     float* slopes = pass == 1 ? s.slopes : nullptr;
-    if (pass == 2) LEM_LAUNCH(L, k_cand_reset, 1, 1, s.sc);
     if (s.fd_tma) {
         lem_status r = LEM_OK;
         switch (s.fd_rows) {
@@ -1581,7 +1575,7 @@ static lem_status direction_pass(const DevState& s, const ModelConsts& k, const 
         DevScalars* sc = s.sc;
         void* args[] = {(void*)&eqm,  (void*)&sp, (void*)&cand, (void*)&tq,  (void*)&tq_cap,
                         (void*)&mark, (void*)&kk, (void*)&sc,   (void*)&pass};
-        lem_status r = coop("k_plateau_relax", (const void*)k_plateau_relax, s.coop_blocks[kCkPlateau], args, L);
+        lem_status r = coop("k_plateau_relax", (const void*)k_plateau_relax, coop_for(s, kCkPlateau, ts.n, 1), args, L);
         if (r != LEM_OK) return r;
     }
     LEM_LAUNCH(L, k_plateau_final, flat_blocks(span, T, big), T, s.eqm, s.sp, s.list_a, s.sfd, s.mfd, slopes, k, s.sc,
@@ -1594,6 +1588,8 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
     const TileSet ts = tiles_of(s, k.W);
     const size_t span = ts.span();
     lem_status r;
+    int logmax = 0;
+    while ((1ll << logmax) < s.ecap) ++logmax;
     LEM_LAUNCH(L, k_fd_reset, (s.dems.n + 127) / 128, 128, s.sc, s.dems);
     if ((r = direction_pass(s, k, L, 1)) != LEM_OK) return r;
     // sink flooding on the pass-1 codes
@@ -1607,7 +1603,7 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
         ModelConsts kk = k;
         DevScalars* sc = s.sc;
         void* args[] = {(void*)&zz, (void*)&ws, (void*)&sinks, (void*)&merging, (void*)&kk, (void*)&sc};
-        if ((r = coop("k_flood_merge", (const void*)k_flood_merge, s.coop_blocks[kCkMerge], args, L)) != LEM_OK) return r;
+        if ((r = coop("k_flood_merge", (const void*)k_flood_merge, coop_for(s, kCkMerge, ts.n, 1), args, L)) != LEM_OK) return r;
     }
     {
         int32_t* ws = s.ws;
@@ -1616,12 +1612,12 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
         ModelConsts kk = k;
         DevScalars* sc = s.sc;
         TileSet tt = ts;
-        void* args[] = {(void*)&ws, (void*)&la, (void*)&lb, (void*)&kk, (void*)&sc, (void*)&tt};
-        if ((r = coop("k_flood_jump", (const void*)k_flood_jump, s.coop_blocks[kCkJump], args, L)) != LEM_OK) return r;
+        unsigned long long* ekey = s.ekey;
+        unsigned long long* ewt = s.ewt;
+        void* args[] = {(void*)&ws,     (void*)&la, (void*)&lb, (void*)&ekey, (void*)&ewt,
+                        (void*)&logmax, (void*)&kk, (void*)&sc, (void*)&tt};
+        if ((r = coop("k_flood_jump", (const void*)k_flood_jump, coop_for(s, kCkJump, ts.n, 1), args, L)) != LEM_OK) return r;
     }
-    int logmax = 0;
-    while ((1ll << logmax) < s.ecap) ++logmax;
-    LEM_LAUNCH(L, k_edge_clear, flat_blocks((size_t)s.ecap, T, big), T, s.ekey, s.ewt, logmax, s.sc);
     {
         const dim3 eb(FE_BX, FE_BY), eg(ts.n, kTile / FE_BY);
         LEM_LAUNCH(L, k_flood_edges, eg, eb, s.z, s.mask, s.ws, s.ekey, s.ewt, logmax, k, s.sc, ts);
@@ -1653,7 +1649,7 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
                         (void*)&cmaxw, (void*)&bidp, (void*)&blab, (void*)&up,    (void*)&wup,  (void*)&uv0,
                         (void*)&uv1,  (void*)&id0,  (void*)&id1,  (void*)&pick,  (void*)&reps, (void*)&list_cap,
                         (void*)&sc};
-        if ((r = coop("k_flood_spill", (const void*)k_flood_spill, s.coop_blocks[kCkSpill], args, L)) != LEM_OK) return r;
+        if ((r = coop("k_flood_spill", (const void*)k_flood_spill, coop_for(s, kCkSpill, ts.n, 1), args, L)) != LEM_OK) return r;
     }
     LEM_LAUNCH(L, k_flood_raise, flat_blocks(span, T, big), T, s.z, s.mask, s.ws, s.raise, s.zf, k, s.sc, s.dems,
                ts);
