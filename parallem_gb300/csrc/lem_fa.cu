@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(256, 6)
         const int gx = tx0 + lx, gy = ty0 + ly0 + 8 * q;
         wq[q] = !w ? 1.0f : (gx < W && gy < H) ? w[(size_t)gy * W + gx] : 0.f;
     }
-    if (threadIdx.x == 0) s_fn = s_pool = 0;
+    if (threadIdx.x == 0) s_fn = s_pool = s_qn = 0;
     for (int i = threadIdx.x; i < kTile * kTile / 2; i += blockDim.x) {
         s_bins[i] = 0;
         reinterpret_cast<uint32_t*>(s_dm)[i] = 0;

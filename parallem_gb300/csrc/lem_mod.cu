@@ -396,7 +396,6 @@ __global__ void __launch_bounds__(256, 4)
 constexpr int kFinNz = 1;      // final-pass slot: the cell's sediment column is not empty
 constexpr int kFinOutlet = 2;  // final-pass slot: an outlet (the coarse wave stored it; counted only)
 constexpr int kPool = kTilePool;
-constexpr uint8_t kFDone = 1, kFTaint = 2;
 
 // Maps of a value through a run of single-input cells: v -> clamp(a*v + b, lo, hi)
 // as float4(a, b, lo, hi); lo > hi encodes the constant b (a cell whose
@@ -448,7 +447,6 @@ struct SedInit {
     SedLocal L;
     int32_t pend;
     int ext;
-    uint32_t dmask;  // the in-tile donors (sed_init_staged): bit k for direction scan_dir(k)
 };
 __device__ __forceinline__ SedInit sed_init(const uint8_t* s_code, const uint8_t* s_cls, int lx, int ly, int tx0,
                                             int ty0, int W, const float* __restrict__ ero,
@@ -459,7 +457,6 @@ __device__ __forceinline__ SedInit sed_init(const uint8_t* s_code, const uint8_t
     SedInit r;
     r.pend = 0;
     r.ext = 0;
-    r.dmask = 0;  // the wave of k_sedt_final derives its donors itself
     float ad = 0.f, ac = 0.f, ag = 0.f;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
@@ -487,43 +484,17 @@ __device__ __forceinline__ SedInit sed_init(const uint8_t* s_code, const uint8_t
     return r;
 }
 
-// sed_init on the tile's erosion terms staged in shared memory (kTH x kTH
-// halo layout): the same sums in the same order.
-__device__ __forceinline__ SedInit sed_init_staged(const uint8_t* s_code, const uint8_t* s_cls, const float* s_e,
-                                                   const float* s_i, const float* s_g, int lx, int ly, float st0,
-                                                   float stone0, const ModelConsts& k) {
-    const float omd = 1.0f - k.ddk, omc = 1.0f - k.dck, omg = 1.0f - k.dgk;
-    const int hc = (ly + 1) * kTH + lx + 1;
-    SedInit r;
-    r.pend = 0;
-    r.ext = 0;
-    r.dmask = 0;
-    float ad = 0.f, ac = 0.f, ag = 0.f;
-#pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-        const int d = scan_dir(kk);
-        const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-        if (!donates(s_code[nh], d)) continue;
-        const uint8_t cl = s_cls[nh];
-        if (cl == kCellBlock) {
-            r.pend |= kBlocked;
-            continue;
-        }
-        if (cl != kCellIn) continue;
-        ad = __fadd_rn(ad, __fmul_rn(1.0f, __fmul_rn(s_e[nh], omd)));
-        ac = __fadd_rn(ac, __fmul_rn(1.0f, __fmul_rn(s_i[nh], omc)));
-        ag = __fadd_rn(ag, __fmul_rn(1.0f, __fmul_rn(s_g[nh], omg)));
-        if (in_tile(lx + dir_dx(d), ly + dir_dy(d))) {
-            ++r.pend;
-            r.dmask |= 1u << kk;
-        } else {
-            ++r.ext;
-        }
-    }
-    r.L = sed_local(ad, ac, ag, s_e[hc], s_i[hc], s_g[hc], st0, stone0, k.ddk, k.dck, k.dgk);
-    return r;
-}
+// Sediment status of a cell in s_info, above its kind: a donor in another tile, a
+// sediment column that is not empty, reached (every donor upstream completes),
+// and downstream of an entry.
+constexpr uint8_t kSedKind = 3, kSedEntry = 4, kSedNz = 8, kSedDone = 16, kSedTaint = 32;
+constexpr int kMaxNodes = 512;  // nodes of a tile: entries (124 border cells), joins of their branches, outlets
 
+// Bound by the chains of its one-warp phases (levels, runs) on few resident tiles
+// rather than by memory.  The cells settle in level order (see tile_levels) in the
+// place of a queue, donors and node inputs come from masks set while the codes are
+// staged, and shared arrays are reused so that five tiles share an SM: 1.55 -> 1.21
+// ms at 4096 x 4096 cells, 53 -> 45 us for a few tiles.
 __global__ void __launch_bounds__(256, 5)
     k_sedt_local(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd, const float* __restrict__ ero,
                  const float* __restrict__ inci, const float* __restrict__ geli, float* depo, float* stone,
@@ -533,28 +504,38 @@ __global__ void __launch_bounds__(256, 5)
                  float4* __restrict__ f_map, float2* __restrict__ f_ds, int32_t* __restrict__ t_fcnt, int32_t* outs,
                  ModelConsts k, DevScalars* sc, DemCtx dc, TileSet ts) {
     if (!sc->sed_tiled_ok) return;
+    constexpr int C = kTile * kTile;
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
-    __shared__ int32_t s_pend[kTile * kTile];
-    __shared__ float s_new[kTile * kTile];  // settled stone (the old stone until then)
+    __shared__ float s_new[C + 1];  // settled stone (the old stone until then)
     // A, B, deposition and soil thickness per cell; before them, the halo's
     // erosion terms (3 kTH x kTH floats) for the set-up
-    __shared__ float s_coef[4 * kTile * kTile];
+    __shared__ float s_coef[4 * C];
     float* const s_A = s_coef;
-    float* const s_B = s_coef + kTile * kTile;
-    float* const s_dep = s_coef + 2 * kTile * kTile;
-    float* const s_stn = s_coef + 3 * kTile * kTile;
+    float* const s_B = s_coef + C;
+    float* const s_dep = s_coef + 2 * C;
+    float* const s_stn = s_coef + 3 * C;
     float* const s_ero = s_coef;
     float* const s_inc = s_coef + kTH * kTH;
     float* const s_gel = s_coef + 2 * kTH * kTH;
-    __shared__ int16_t s_ptr[kTile * kTile];
-    __shared__ int16_t s_topo[kTile * kTile];
-    __shared__ int16_t s_pos[kTile * kTile];
-    __shared__ int16_t s_oslot[kTile * kTile];
-    __shared__ uint8_t s_kind[kTile * kTile];
-    __shared__ uint8_t s_ext[kTile * kTile];
-    __shared__ uint8_t s_flag[kTile * kTile];
-    __shared__ uint8_t s_nz[kTile * kTile];
+    // the in-tile paths (tile_paths), then where each ends, and the outlets' slots
+    __shared__ int32_t s_pd[C];
+    int16_t* const s_end = reinterpret_cast<int16_t*>(s_pd);
+    int16_t* const s_oslot = s_end + C;
+    // levels, then a node's number of inputs (0: not a node)
+    __shared__ int32_t s_h[C];
+    int32_t* const s_node = s_h;
+    // donors, bit k for direction scan_dir(k): in the low byte those in the tile,
+    // in the high byte those in other tiles, then with the waiting ones in the tile
+    __shared__ __align__(4) uint16_t s_dm[C];
+    __shared__ uint8_t s_info[C];
+    // the settled cells by level, then the nodes by level and each node's slot
+    __shared__ uint32_t s_ent[C];
+    int16_t* const s_pos = reinterpret_cast<int16_t*>(s_ent + kMaxNodes);
+    // sorting bins, then the node at the top of a cell's run
+    __shared__ uint32_t s_bins[C / 2];
+    int16_t* const s_up = reinterpret_cast<int16_t*>(s_bins);
+    __shared__ uint32_t s_wait[kTile], s_bad[kTile];
     __shared__ int16_t s_olist[kTileEnt];
     __shared__ int32_t s_ocnt[kTileEnt];
     // per outlet, its program's nodes in the low half and their inputs in the
@@ -562,14 +543,26 @@ __global__ void __launch_bounds__(256, 5)
     __shared__ int32_t s_pcnt[kTileEnt];
     __shared__ int32_t s_pstart[kTileEnt];
     __shared__ int16_t s_pfill[kTileEnt];
-    __shared__ int16_t s_q[kTile * kTile];
-    __shared__ int16_t s_rnd[kTile * kTile];
-    __shared__ int s_no, s_nt, s_done, s_dem, s_qn, s_qend, s_fn;
+    __shared__ int s_no, s_nt, s_done, s_dem, s_fn;
     __shared__ int s_wcnt[9];  // per-warp counts of the outlet list and its append
     const int W = k.W, H = k.H, TW = (W + kTile - 1) / kTile;
     const int t = ts.tile(blockIdx.x);
     const int tx0 = (t % TW) * kTile, ty0 = (t / TW) * kTile;
-    sed_tile_load(mask, fd, W, H, tx0, ty0, s_code, s_cls);
+    const int lx = threadIdx.x & 31, ly0 = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < C / 2; i += blockDim.x) {
+        s_bins[i] = 0;
+        reinterpret_cast<uint32_t*>(s_dm)[i] = 0;
+    }
+    if (threadIdx.x < kTile) s_bad[threadIdx.x] = 0;
+    if (threadIdx.x < kTileEnt) {
+        s_ocnt[threadIdx.x] = 0;
+        s_pcnt[threadIdx.x] = 0;
+    }
+    if (threadIdx.x == 0) s_done = s_fn = s_nt = 0, s_dem = -1, s_new[kNoCell] = 0.f;
+    __syncthreads();
+    tile_stage(
+        fd, [&](size_t g, int x, int y) { return mask[g] && x != 0 && y != 0 ? kCellIn : kCellBlock; }, W, H, tx0, ty0,
+        s_code, s_cls, s_dm, s_bad);
     for (int j = threadIdx.x; j < kTH * kTH; j += blockDim.x) {
         const int gx = tx0 - 1 + j % kTH, gy = ty0 - 1 + j / kTH;
         float e = 0.f, i = 0.f, g = 0.f;
@@ -583,61 +576,53 @@ __global__ void __launch_bounds__(256, 5)
         s_inc[j] = i;
         s_gel[j] = g;
     }
-    if (threadIdx.x < kTileEnt) {
-        s_ocnt[threadIdx.x] = 0;
-        s_pcnt[threadIdx.x] = 0;
-    }
-    if (threadIdx.x == 0) s_nt = s_done = s_fn = 0, s_dem = -1;
     __syncthreads();
-    const int lx = threadIdx.x & 31, ly0 = threadIdx.x >> 5;
-    bool src[4];
     float cA[4], cB[4], cD[4], cS[4];  // the cells' coefficients until the staged terms are spent
-    int dem = -1;  // one DEM per tile
+    int dem = -1;                      // one DEM per tile
+    const float omd = 1.0f - k.ddk, omc = 1.0f - k.dck, omg = 1.0f - k.dgk;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        int32_t pend = kBlocked;
-        uint8_t kind = kKindEnd, ext = 0, nz = 0;
-        int16_t ptr = (int16_t)l, dm = 0;
+        uint32_t info = kKindEnd, dm = 0;
+        int32_t pd = l;
         float snew = 0.f;
         cA[q] = cB[q] = cD[q] = cS[q] = 0.f;
         if (s_cls[hc] == kCellIn) {
             const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
             snew = __ldcg(stone + g);
-            const SedInit in = sed_init_staged(s_code, s_cls, s_ero, s_inc, s_gel, lx, ly, soilT[g], snew, k);
-            pend = in.pend;
-            ext = (uint8_t)in.ext;
-            dm = (int16_t)in.dmask;
-            cA[q] = in.L.A;
-            cB[q] = in.L.B;
-            cD[q] = in.L.dep;
-            cS[q] = in.L.stn;
-            nz = in.L.nz;
-            if (dem < 0) dem = dem_at(dc, (size_t)(ty0 + ly) * W + tx0 + lx);
-            const int d = bit_dir(s_code[hc]);
-            if (d >= 0 && s_cls[hc + dir_dy(d) * kTH + dir_dx(d)] == kCellIn) {
-                const int rlx = lx + dir_dx(d), rly = ly + dir_dy(d);
-                if (in_tile(rlx, rly)) {
-                    kind = kKindIn;
-                    ptr = (int16_t)(rly * kTile + rlx);
-                } else {
-                    kind = kKindOutlet;
-                }
+            const float st0 = soilT[g];
+            dm = s_dm[l];
+            float ad = 0.f, ac = 0.f, ag = 0.f;
+            for (uint32_t m = (dm | (dm >> 8)) & 255u; m; m &= m - 1) {
+                const int d = scan_dir(__ffs(m) - 1), nh = hc + dir_dy(d) * kTH + dir_dx(d);
+                ad = __fadd_rn(ad, __fmul_rn(1.0f, __fmul_rn(s_ero[nh], omd)));
+                ac = __fadd_rn(ac, __fmul_rn(1.0f, __fmul_rn(s_inc[nh], omc)));
+                ag = __fadd_rn(ag, __fmul_rn(1.0f, __fmul_rn(s_gel[nh], omg)));
             }
+            const SedLocal in =
+                sed_local(ad, ac, ag, s_ero[hc], s_inc[hc], s_gel[hc], st0, snew, k.ddk, k.dck, k.dgk);
+            cA[q] = in.A;
+            cB[q] = in.B;
+            cD[q] = in.dep;
+            cS[q] = in.stn;
+            if (dem < 0) dem = dem_at(dc, g);
+            const int d = bit_dir(s_code[hc]);
+            const int rlx = lx + dir_dx(d < 0 ? 0 : d), rly = ly + dir_dy(d < 0 ? 0 : d);
+            if (d >= 0 && s_cls[(rly + 1) * kTH + rlx + 1] == kCellIn) {
+                info = in_tile(rlx, rly) ? kKindIn : kKindOutlet;
+                if (info == kKindIn) pd = (rly * kTile + rlx) | (1 << 10);
+            }
+            info |= (in.nz ? kSedNz : 0) | (dm >> 8 ? kSedEntry : 0);
         }
-        s_pend[l] = pend;
-        src[q] = pend == 0;
-        s_kind[l] = kind;
-        s_ext[l] = ext;
-        s_ptr[l] = ptr;
+        s_pd[l] = pd;
+        s_h[l] = 0;
+        s_info[l] = (uint8_t)info;
         s_new[l] = snew;
-        s_nz[l] = nz;
-        s_flag[l] = 0;
-        s_pos[l] = -1;
-        s_oslot[l] = dm;  // the outlet slots are listed after the wave
+        const unsigned wb = __ballot_sync(0xffffffffu, (info & kSedEntry) != 0);
+        if (lx == 0) s_wait[ly] = wb;
     }
     dem = __reduce_max_sync(0xffffffffu, dem);
-    if ((threadIdx.x & 31) == 0 && dem >= 0) atomicMax(&s_dem, dem);
+    if (lx == 0 && dem >= 0) atomicMax(&s_dem, dem);
     __syncthreads();  // the staged erosion terms are spent
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
@@ -647,95 +632,86 @@ __global__ void __launch_bounds__(256, 5)
         s_dep[l] = cD[q];
         s_stn[l] = cS[q];
     }
-    __syncthreads();
-    // The waiting cells: every cell downstream of an entry (a cell with a donor
-    // in another tile), marked along each entry's in-tile path before the wave.
-    // A walk stops where another walk has passed (it carries on from there).
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        int c = (ly0 + 8 * q) * kTile + lx;
-        if (!s_ext[c]) continue;
-        for (int guard = 0; guard < kTile * kTile; ++guard) {
-            if (s_flag[c] & kFTaint) break;
-            s_flag[c] = kFTaint;
-            if (s_kind[c] != kKindIn) break;
-            c = s_ptr[c];
-        }
-    }
-    // settle what depends on this tile only; order the waiting cells
-    int done = 0;
-    if (threadIdx.x == 0) s_qn = 0;
-    __syncthreads();
-    tile_wave(
-        [&](int cur, int rnd) {
-            const bool taint = (s_flag[cur] & kFTaint) != 0;
-            if (!taint) {
-                // every donor is inside the tile and settled; all of them are
-                // loaded before the sum in scan order
-                const uint32_t dm = (uint16_t)s_oslot[cur];
-                float v[8];
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk) v[kk] = (dm >> kk) & 1u ? s_new[cur + tile_step(scan_dir(kk))] : 0.f;
-                float from = 0.f;
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)
-                    if ((dm >> kk) & 1u) from = __fadd_rn(from, __fmul_rn(1.0f, v[kk]));
-                // the cell's outputs are stored after the wave, coalesced
-                if (s_nz[cur]) s_new[cur] = sed_mix(s_A[cur], s_B[cur], from);
-                s_flag[cur] = kFDone;
-                ++done;
-            } else {
-                s_flag[cur] = kFDone | kFTaint;
-                s_rnd[cur] = (int16_t)rnd;  // a level for the coarse evaluation: inputs come from earlier rounds
-                s_topo[atomicAdd(&s_nt, 1)] = (int16_t)cur;
-            }
-            return s_kind[cur] == kKindIn ? (int)s_ptr[cur] : -1;
-        },
-        s_pend, s_q, &s_qn, &s_qend, src, lx, ly0);
-    // the settled cells' outputs (sed_store), one coalesced pass
+    tile_paths(s_pd, s_h, s_wait, s_bad, lx, ly0);
+    int key[4];
+    int16_t end[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx;
-        if (s_flag[l] != kFDone) continue;
-        const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
-        depo[g] = s_dep[l];
-        if (s_nz[l]) {
-            const float sn = s_new[l];
-            __stcg(stone + g, sn);
-            fines[g] = __fsub_rn(100.0f, sn);
-        }
-        soilT[g] = s_stn[l];
+        const uint32_t info = s_info[l];
+        const bool done = s_cls[(ly + 1) * kTH + lx + 1] == kCellIn && !((s_bad[ly] >> lx) & 1u);
+        const bool taint = (s_wait[ly] >> lx) & 1u;
+        key[q] = done && !taint ? s_h[l] : -1;
+        end[q] = (int16_t)(s_pd[l] & kPtr);
+        s_info[l] = (uint8_t)(info | (done ? kSedDone : 0) | (taint ? kSedTaint : 0));
+        // a settled cell without donors mixes with nothing
+        if (key[q] == 0 && (info & kSedNz)) s_new[l] = sed_mix(s_A[l], s_B[l], 0.0f);
     }
-    for (int it = 0; it < 10; ++it) {  // in-tile paths are shorter than 2^10 cells
-        bool ch = false;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
+    constexpr uint8_t kWaits = kSedDone | kSedTaint;
+    tile_sort(
+        key,
+        [&](int q) {
             const int l = (ly0 + 8 * q) * kTile + lx;
-            const int16_t nx = s_ptr[s_ptr[l]];
-            if (nx != s_ptr[l]) {
-                s_ptr[l] = nx;
-                ch = true;
+            return entry_of(l, s_dm[l] & 255u);
+        },
+        s_bins, C / 2, s_ent, &s_nt, lx);  // (its barriers also cover s_info and the last reads of s_pd)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s_end[(ly0 + 8 * q) * kTile + lx] = end[q];
+    // settle what depends on this tile only: every donor is inside the tile and
+    // settled; the sum in scan order (adding the 0 of kNoCell changes nothing)
+    struct Cell {
+        float A, B;
+        uint32_t e;
+        bool nz;
+    };
+    tile_levels(
+        [&](uint32_t e) {
+            const int c = entry_cell(e) & kPtr;  // (kNoCell's coefficients are not used)
+            return Cell{s_A[c], s_B[c], e, entry_cell(e) != kNoCell && (s_info[c] & kSedNz)};
+        },
+        [&](const Cell& f) {
+            float from = __fadd_rn(__fadd_rn(0.f, s_new[entry_d0(f.e)]), s_new[entry_d1(f.e)]);
+            if (__any_sync(0xffffffffu, f.e & kMoreDonors) && (f.e & kMoreDonors)) {
+                const int c = entry_cell(f.e);
+                uint32_t m = s_dm[c] & 255u;
+                m &= m - 1;
+                for (m &= m - 1; m; m &= m - 1) from = __fadd_rn(from, s_new[c + scan_step(__ffs(m) - 1)]);
             }
-        }
-        if (!__syncthreads_or(ch)) break;  // every pointer is at its path's end
-    }
+            const float sn = sed_mix(f.A, f.B, from);
+            if (f.nz) s_new[entry_cell(f.e)] = sn;
+        },
+        1, C, s_bins, s_ent);
+    // the settled cells' outputs (sed_store), one coalesced pass
     bool stray = false;  // a waiting cell whose in-tile path ends inside the tile (at the DEM's outlet, say)
+    int done = 0;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx;
         const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
-        if (s_ext[l]) {
-            const int e = s_ptr[l];
-            t_dst[g] = s_kind[e] == kKindOutlet ? (int32_t)((ty0 + e / kTile) * W + tx0 + (e & (kTile - 1))) : -1;
+        const uint32_t info = s_info[l];
+        const int e = end[q];
+        const bool out = (s_info[e] & kSedKind) == kKindOutlet;
+        if ((info & kWaits) == kSedDone) {
+            ++done;
+            depo[g] = s_dep[l];
+            if (info & kSedNz) {
+                const float sn = s_new[l];
+                __stcg(stone + g, sn);
+                fines[g] = __fsub_rn(100.0f, sn);
+            }
+            soilT[g] = s_stn[l];
         }
-        stray |= s_flag[l] == (kFDone | kFTaint) && s_kind[s_ptr[l]] != kKindOutlet;
-        if (tx0 + lx < W && ty0 + ly < H) t_stat[g] = (s_flag[l] & kFDone) ? ((s_flag[l] & kFTaint) ? 2 : 1) : 0;
+        if (info & kSedEntry) t_dst[g] = out ? (int32_t)((ty0 + e / kTile) * W + tx0 + (e & (kTile - 1))) : -1;
+        stray |= (info & kWaits) == kWaits && !out;
+        if (tx0 + lx < W && ty0 + ly < H) t_stat[g] = (info & kSedDone) ? ((info & kSedTaint) ? 2 : 1) : 0;
     }
     // Such a tile keeps the second wave for its waiting cells; in every other
     // tile each waiting cell's stone is a map of one program node's value,
     // stored by the final pass.
     const bool second_wave = __syncthreads_or(stray);
-    list_outlets(s_kind, 0xff, s_olist, s_oslot, &s_no, s_wcnt);
+    list_outlets(s_info, kSedKind, s_olist, s_oslot, &s_no, s_wcnt);
+    for (int i = threadIdx.x; i < C / 2; i += blockDim.x) s_bins[i] = 0;  // for the nodes
+    if (threadIdx.x == 0) s_nt = 0;
     __syncthreads();
     // inflows per outlet (ring cells flowing into the tile)
     if (threadIdx.x < kRing) {
@@ -744,8 +720,8 @@ __global__ void __launch_bounds__(256, 5)
         if (d >= 0) {
             const int hx = h % kTH + dir_dx(d), hy = h / kTH + dir_dy(d);
             if (hx >= 1 && hx <= kTile && hy >= 1 && hy <= kTile && s_cls[hy * kTH + hx] == kCellIn) {
-                const int o = s_ptr[(hy - 1) * kTile + hx - 1];
-                if (s_kind[o] == kKindOutlet) atomicAdd(&s_ocnt[s_oslot[o]], 1);
+                const int o = s_end[(hy - 1) * kTile + hx - 1];
+                if ((s_info[o] & kSedKind) == kKindOutlet) atomicAdd(&s_ocnt[s_oslot[o]], 1);
             }
         }
     }
@@ -753,91 +729,78 @@ __global__ void __launch_bounds__(256, 5)
     // from another tile, join two waiting branches, or are the outlet.  The
     // waiting cells between nodes pass one value on; they become the maps of
     // the nodes' inputs.
-    int32_t* s_node = s_pend;  // a node's number of inputs, 0 elsewhere (the in-degrees are spent)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        int node = 0;
-        if (s_flag[l] == (kFDone | kFTaint) && s_kind[s_ptr[l]] == kKindOutlet) {
-            int ntd = 0;
-#pragma unroll
-            for (int d = 0; d < 8; ++d) {
-                const int nlx = lx + dir_dx(d), nly = ly + dir_dy(d);
-                const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-                if (in_tile(nlx, nly) && donates(s_code[nh], d) && s_cls[nh] == kCellIn &&
-                    (s_flag[nly * kTile + nlx] & kFTaint))
-                    ++ntd;
-            }
-            // every input of a node is waiting or comes from another tile
-            if (s_ext[l] != 0 || ntd >= 2 || s_kind[l] == kKindOutlet) node = s_ext[l] + ntd;
-        }
-        s_node[l] = node;
-    }
-    __syncthreads();
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int l = (ly0 + 8 * q) * kTile + lx;
-        if (s_node[l]) atomicAdd(&s_pcnt[s_oslot[s_ptr[l]]], 1 | (s_node[l] << 16));
+        int node = 0;
+        key[q] = -1;
+        if ((s_info[l] & kWaits) == kWaits && (s_info[end[q]] & kSedKind) == kKindOutlet) {
+            const uint32_t dm = s_dm[l];
+            uint32_t wm = 0;
+            for (uint32_t m = dm & 255u; m; m &= m - 1)
+                if (s_info[l + scan_step(__ffs(m) - 1)] & kSedTaint) wm |= m & (0u - m);
+            // every input of a node is waiting or comes from another tile
+            if ((dm >> 8) || (wm & (wm - 1)) || (s_info[l] & kSedKind) == kKindOutlet) {
+                node = __popc(dm >> 8) + __popc(wm);
+                key[q] = s_h[l];
+            }
+            s_dm[l] = (uint16_t)(dm | (wm << 8));
+        }
+        s_node[l] = node;  // (a cell's level is its own thread's to replace)
+        if (node) atomicAdd(&s_pcnt[s_oslot[end[q]]], 1 | (node << 16));
     }
+    tile_sort(
+        key, [&](int q) { return (uint32_t)((ly0 + 8 * q) * kTile + lx); }, s_bins, C / 2, s_ent, &s_nt, lx);
     // Every waiting cell between nodes: its map v -> stone from its one waiting
     // in-tile donor (in place of its own coefficients, which only nodes need
     // from here on).  Every waiting cell of a tile without a second wave also
     // takes a final-pass slot, with its deposition and soil thickness.
-    int16_t* s_up = s_q;  // the node at the top of a cell's run (s_q is spent since the wave)
-    const size_t fbase = (size_t)t * kTile * kTile;
+    const size_t fbase = (size_t)t * C;
     int fslot[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        const bool waits = s_flag[l] == (kFDone | kFTaint) && s_kind[s_ptr[l]] == kKindOutlet;
+        const int l = (ly0 + 8 * q) * kTile + lx;
+        const bool waits = (s_info[l] & kWaits) == kWaits && (s_info[end[q]] & kSedKind) == kKindOutlet;
         fslot[q] = warp_slot(waits && !second_wave, &s_fn);
         if (!waits) continue;
         if (fslot[q] >= 0) f_ds[fbase + fslot[q]] = make_float2(s_dep[l], s_stn[l]);
         if (s_node[l]) continue;
         float Cc = 0.f;
-#pragma unroll
-        for (int k2 = 0; k2 < 8; ++k2) {
-            const int d2 = scan_dir(k2);
-            const int ulx = lx + dir_dx(d2), uly = ly + dir_dy(d2);
-            const int uh = hc + dir_dy(d2) * kTH + dir_dx(d2);
-            if (!in_tile(ulx, uly) || !donates(s_code[uh], d2) || s_cls[uh] != kCellIn) continue;
-            const int u = uly * kTile + ulx;
-            if (!(s_flag[u] & kFTaint)) Cc = __fadd_rn(Cc, __fmul_rn(1.0f, s_new[u]));
-        }
-        const float4 M = map_cell(s_A[l], s_B[l], Cc, s_nz[l] != 0, s_new[l]);
+        const uint32_t dm = s_dm[l];
+        for (uint32_t m = dm & ~(dm >> 8) & 255u; m; m &= m - 1)
+            Cc = __fadd_rn(Cc, __fmul_rn(1.0f, s_new[l + scan_step(__ffs(m) - 1)]));
+        const float4 M = map_cell(s_A[l], s_B[l], Cc, (s_info[l] & kSedNz) != 0, s_new[l]);
         s_A[l] = M.x;
         s_B[l] = M.y;
         s_dep[l] = M.z;
         s_stn[l] = M.w;
     }
+    const int no = s_no, nt = s_nt;
+    if (threadIdx.x < 32) outlet_starts(s_pcnt, s_pstart, no);
     __syncthreads();
     // The maps of the cells between nodes, composed down each run from the node
     // at its top: afterwards s_up of such a cell is that node and its map takes
     // the node's value to its own stone.  One walk per node; no two walks
     // share a cell (a cell between nodes has one waiting donor).
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        const int l = (ly0 + 8 * q) * kTile + lx;
-        if (!s_node[l] || s_kind[l] != kKindIn) continue;
+    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
+        const int l = (int)s_ent[i];
+        if ((s_info[l] & kSedKind) != kKindIn) continue;
         float4 F = map_identity();
         int c = l;
-        for (int guard = 0; guard < kTile * kTile; ++guard) {
+        for (int guard = 0; guard < C; ++guard) {
             const int d = bit_dir(s_code[(c / kTile + 1) * kTH + (c & (kTile - 1)) + 1]);
             c += dir_dy(d) * kTile + dir_dx(d);  // in the tile: c is not an outlet
-            if (s_flag[c] != (kFDone | kFTaint) || s_node[c]) break;
+            const uint32_t info = s_info[c];
+            if ((info & kWaits) != kWaits || s_node[c]) break;
             F = map_compose(make_float4(s_A[c], s_B[c], s_dep[c], s_stn[c]), F);
             s_A[c] = F.x;
             s_B[c] = F.y;
             s_dep[c] = F.z;
             s_stn[c] = F.w;
             s_up[c] = (int16_t)l;
-            if (s_kind[c] != kKindIn) break;
+            if ((info & kSedKind) != kKindIn) break;
         }
     }
-    __syncthreads();
-    const int no = s_no, nt = s_nt;
-    if (threadIdx.x < 32) outlet_starts(s_pcnt, s_pstart, no);
-    __syncthreads();
     const int j = threadIdx.x;
     const int pcnt = j < no ? s_pcnt[j] : 0, pstart = j < no ? s_pstart[j] : 0;
     int32_t* const s_ifill = s_pcnt;  // where the program's next node's inputs go (the counts are kept above)
@@ -846,71 +809,68 @@ __global__ void __launch_bounds__(256, 5)
         s_pfill[j] = (int16_t)(pstart & 0xffff);
     }
     __syncthreads();
-    // node slots: grouped by outlet, in the order the cells were reached
+    // node slots: grouped by outlet, in level order
     if (threadIdx.x < 32) {
         const unsigned below = (1u << lx) - 1u;
         for (int base = 0; base < nt; base += 32) {
             const int i = base + lx;
-            int key = -1, c = 0;
+            int slot = -1, c = 0;
             if (i < nt) {
-                c = s_topo[i];
-                if (s_node[c]) key = s_oslot[s_ptr[c]];
+                c = (int)s_ent[i];
+                slot = s_oslot[s_end[c]];
             }
-            const unsigned peers = __match_any_sync(0xffffffffu, key);
-            const int fill = key >= 0 ? s_pfill[key] : 0;
+            const unsigned peers = __match_any_sync(0xffffffffu, slot);
+            const int fill = slot >= 0 ? s_pfill[slot] : 0;
             __syncwarp();
-            if (key >= 0) {
+            if (slot >= 0) {
                 s_pos[c] = (int16_t)(fill + __popc(peers & below));
-                if ((peers & below) == 0) s_pfill[key] = (int16_t)(fill + __popc(peers));
+                if ((peers & below) == 0) s_pfill[slot] = (int16_t)(fill + __popc(peers));
             }
             __syncwarp();
         }
     }
     __syncthreads();
-    const size_t nbase = (size_t)t * kTile * kTile;
+    const size_t nbase = (size_t)t * C;
     const size_t pool = (size_t)t * kPool;
-#pragma unroll 1
-    for (int q = 0; q < 4; ++q) {
-        const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        if (!s_node[l]) continue;
-        const int pos = s_pos[l], slot = s_oslot[s_ptr[l]];
+    for (int i = threadIdx.x; i < nt; i += blockDim.x) {
+        const int l = (int)s_ent[i], ly = l / kTile, x = l & (kTile - 1);
+        const int pos = s_pos[l], slot = s_oslot[s_end[l]];
         const int first = s_pstart[slot] & 0xffff;
         const int start = atomicAdd(&s_ifill[slot], s_node[l]);
         if (start + s_node[l] > kPool) {
             raise_error(&sc->err, ErrFlags::kCapacity);
             continue;
         }
-        float C = 0.f;
+        const uint32_t dm = s_dm[l];
+        float Cc = 0.f;
         int m = 0;
 #pragma unroll 1
-        for (int kk = 0; kk < 8; ++kk) {
-            const int d = scan_dir(kk);
-            const int nlx = lx + dir_dx(d), nly = ly + dir_dy(d);
-            const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-            if (!donates(s_code[nh], d) || s_cls[nh] != kCellIn) continue;
-            if (!in_tile(nlx, nly)) {
-                p_ref[pool + start + m] = (ty0 + nly) * W + tx0 + nlx;
-                p_map[pool + start + m] = map_identity();
-                ++m;
+        for (uint32_t b = (dm | (dm >> 8)) & 255u; b; b &= b - 1) {
+            const int kk = __ffs(b) - 1;
+            int cur = l + scan_step(kk);
+            if (!((dm >> (8 + kk)) & 1u)) {  // settled in the tile
+                Cc = __fadd_rn(Cc, __fmul_rn(1.0f, s_new[cur]));
                 continue;
             }
-            int cur = nly * kTile + nlx;
-            if (!(s_flag[cur] & kFTaint)) {
-                C = __fadd_rn(C, __fmul_rn(1.0f, s_new[cur]));
-                continue;
-            }
-            // the node that feeds this input, through the single-input cells in between
+            int32_t ref;
             float4 H = map_identity();
-            if (!s_node[cur]) {
-                H = make_float4(s_A[cur], s_B[cur], s_dep[cur], s_stn[cur]);
-                cur = s_up[cur];
+            if (!((dm >> kk) & 1u)) {
+                const int d = scan_dir(kk);
+                ref = (ty0 + ly + dir_dy(d)) * W + tx0 + x + dir_dx(d);
+            } else {
+                // the node that feeds this input, through the single-input cells in between
+                if (!s_node[cur]) {
+                    H = make_float4(s_A[cur], s_B[cur], s_dep[cur], s_stn[cur]);
+                    cur = s_up[cur];
+                }
+                ref = -(s_pos[cur] - first + 1);
             }
-            p_ref[pool + start + m] = -(s_pos[cur] - first + 1);
+            p_ref[pool + start + m] = ref;
             p_map[pool + start + m] = H;
             ++m;
         }
-        p_abc[nbase + pos] =
-            make_float4(s_A[l], s_B[l], C, __int_as_float(start | (m << 11) | (s_nz[l] << 15) | ((int)s_rnd[l] << 16)));
+        p_abc[nbase + pos] = make_float4(s_A[l], s_B[l], Cc,
+                                         __int_as_float(start | (m << 11) | (s_info[l] & kSedNz ? 1 << 15 : 0)));
     }
     // the final pass's slots: a node reads its own value, a cell between nodes
     // maps the value of the node at the top of its chain
@@ -920,19 +880,19 @@ __global__ void __launch_bounds__(256, 5)
         const int ly = ly0 + 8 * q, l = ly * kTile + lx;
         const bool node = s_node[l] != 0;
         const int src_node = node ? l : s_up[l];
-        const int e = s_ptr[l];
-        // (a chain always ends at a node; -1 only guards the final pass's read)
-        const int vref = s_node[src_node] && s_pos[src_node] >= 0 ? (int)(fbase + s_pos[src_node]) : -1;
-        f_idx[fbase + fslot[q]] = make_int4((ty0 + ly) * W + tx0 + lx, vref,
+        const int e = end[q];
+        const uint32_t info = s_info[l];
+        f_idx[fbase + fslot[q]] = make_int4((ty0 + ly) * W + tx0 + lx, (int)(fbase + s_pos[src_node]),
                                             (ty0 + e / kTile) * W + tx0 + (e & (kTile - 1)),
-                                            (s_nz[l] ? kFinNz : 0) | (s_kind[l] == kKindOutlet ? kFinOutlet : 0));
+                                            (info & kSedNz ? kFinNz : 0) |
+                                                ((info & kSedKind) == kKindOutlet ? kFinOutlet : 0));
         f_map[fbase + fslot[q]] = node ? map_identity() : make_float4(s_A[l], s_B[l], s_dep[l], s_stn[l]);
     }
     if (threadIdx.x == 0) t_fcnt[t] = second_wave ? -1 : s_fn;
     int32_t og = 0;
     if (j < no) {
         const int o = s_olist[j];
-        const int32_t opend = ((s_flag[o] & kFDone) ? 0 : kBlocked) + s_ocnt[j];
+        const int32_t opend = ((s_info[o] & kSedDone) ? 0 : kBlocked) + s_ocnt[j];
         og = (ty0 + o / kTile) * W + tx0 + (o & (kTile - 1));
         // (the coefficients of a waiting outlet, a node, are still in place)
         t_rec[og] = make_int4((pstart << 16) | (pcnt & 0xffff), (pstart & ~0xffff) | (pcnt >> 16),
@@ -942,7 +902,7 @@ __global__ void __launch_bounds__(256, 5)
     }
     block_append(j < no, og, outs, &sc->tile_src, W * H, &sc->err, s_wcnt);
     done = wsum(done);
-    if ((threadIdx.x & 31) == 0 && done) atomicAdd(&s_done, done);
+    if (lx == 0 && done) atomicAdd(&s_done, done);
     __syncthreads();
     if (threadIdx.x == 0 && s_done && s_dem >= 0) atomicAdd(&dc.out[s_dem].sed_done, s_done);
 }

@@ -361,23 +361,27 @@ __device__ __forceinline__ void tile_paths(int32_t* s_pd, int32_t* s_h, uint32_t
 }
 
 // Sorts the cells with key[q] >= 0 (below 2 * words) by key and counts them in
-// *s_total: s_ent holds pack(q) of each.  s_bins (`words` words, zero before)
-// then holds where each key's cells end, 16 bits a key, up to the first keys
-// without cells (of 64 in a row none may be empty before the last one used).
-// Every thread calls it.
+// *s_total (0 before): s_ent holds pack(q) of each.  s_bins (`words` words, 0
+// before) then holds where each key's cells end, 16 bits a key, up to the last key
+// used; the words 32 and more behind that one's stay 0.  Every thread calls it.
 __device__ __forceinline__ int bin_end(const uint32_t* s_bins, int key) {
     return (s_bins[key >> 1] >> (16 * (key & 1))) & 0xffff;
 }
 template <class Pack>
 __device__ __forceinline__ void tile_sort(const int (&key)[4], const Pack& pack, uint32_t* s_bins, int words,
                                           uint32_t* s_ent, int* s_total, int lx) {
+    int mine = 0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q)
+    for (int q = 0; q < 4; ++q) {
         if (key[q] >= 0) atomicAdd(&s_bins[key[q] >> 1], 1u << (16 * (key[q] & 1)));
+        mine += __popc(__ballot_sync(0xffffffffu, key[q] >= 0));
+    }
+    if (lx == 0 && mine) atomicAdd(s_total, mine);
     __syncthreads();
     if (threadIdx.x < 32) {
+        const uint32_t total = (uint32_t)*s_total;
         uint32_t carry = 0;
-        for (int b = lx; b < words; b += 32) {
+        for (int b = lx; b < words && carry < total; b += 32) {
             const uint32_t v = s_bins[b], lo = v & 0xffff, n = lo + (v >> 16);
             uint32_t incl = n;
 #pragma unroll
@@ -385,12 +389,10 @@ __device__ __forceinline__ void tile_sort(const int (&key)[4], const Pack& pack,
                 const uint32_t u = __shfl_up_sync(0xffffffffu, incl, d);
                 if (lx >= d) incl += u;
             }
-            const uint32_t at = carry + incl - n, all = __shfl_sync(0xffffffffu, incl, 31);
+            const uint32_t at = carry + incl - n;
             s_bins[b] = at | ((at + lo) << 16);
-            if (all == 0) break;
-            carry += all;
+            carry += __shfl_sync(0xffffffffu, incl, 31);
         }
-        if (lx == 0) *s_total = (int)carry;
     }
     __syncthreads();
 #pragma unroll
