@@ -476,45 +476,54 @@ constexpr int kTileSweeps = 2048;  // sweeps of one tile visit before it is re-q
 // lem_limits.max_rounds times the tiles queued at the start.
 constexpr int kQueueSpin = 1 << 20;  // polls of an empty but busy queue, or of an unwritten slot
 
-// The tile queue is a ring of `cap` slots with a sequence number each (a
-// bounded multi-producer multi-consumer queue): ticket p of the pushes (of the
-// takes) owns slot p % cap, free for it once the slot's number reads p (ready
+// The tile queue is a ring of `cap` slots, each a word of a sequence number and a
+// tile (a bounded multi-producer multi-consumer queue): ticket p of the pushes (of
+// the takes) owns slot p % cap, free for it once the slot's number reads p (ready
 // for it once the number reads p + 1).  Tickets come from one atomicAdd each.
+// Pushes and finished visits are counted in one word; where they are equal nothing
+// is queued and no visit runs, since only visits push.  A chain of visits across a
+// lake pays for every trip to memory between a push and the visit it starts, so
+// there are as few as that takes: three for the push, a poll for the take.
 struct TileQueue {
-    int32_t* val;  // [cap] entries
-    int32_t* seq;  // [cap] sequence numbers
-    int32_t* qc;   // [0] push tickets, [1] take tickets, [2] pending (queued or in a visit), [3] visits, [4] stop
+    unsigned long long* slot;  // [cap] tile << 32 | sequence number
+    int32_t* qc;               // [0] pushes, [1] visits finished, [2] take tickets, [3] stop
     int cap;
+    __device__ static unsigned long long word(int32_t t, int seq) {
+        return (unsigned long long)(uint32_t)t << 32 | (uint32_t)seq;
+    }
+    __device__ volatile unsigned long long* at(int ticket) const { return slot + ticket % cap; }
     __device__ void stop(DevScalars* sc) const {
         raise_error(&sc->err, ErrFlags::kNoConverge);
-        atomicExch(&qc[4], 1);
+        atomicExch(&qc[3], 1);
     }
     __device__ void push(int32_t t, DevScalars* sc) const {
-        atomicAdd(&qc[2], 1);
-        const int p = atomicAdd(&qc[0], 1), slot = p % cap;
+        const int p = atomicAdd(&qc[0], 1);
         int spin = 0;  // the slot's previous entry is taken; its taker may still be reading it
-        while (*((volatile int32_t*)&seq[slot]) != p && ++spin < kQueueSpin) __nanosleep(32);
+        while ((int32_t)*at(p) != p && ++spin < kQueueSpin) __nanosleep(32);
         if (spin >= kQueueSpin) return stop(sc);
-        val[slot] = t;
-        __threadfence();
-        atomicExch(&seq[slot], p + 1);
+        *at(p) = word(t, p + 1);
     }
-    // the next tile, or -1 once nothing is queued and no visit runs (or the queue stopped)
-    __device__ int32_t take(DevScalars* sc) const {
-        const int c = atomicAdd(&qc[1], 1), slot = c % cap;
+    // the next tile, or -1 once nothing is queued and no visit runs (or the queue
+    // stopped, as it does when `visits` have been taken)
+    __device__ int32_t take(long long visits, DevScalars* sc) const {
+        const int c = atomicAdd(&qc[2], 1);
         for (int spin = 0; spin < kQueueSpin; ++spin) {
-            if (*((volatile int32_t*)&seq[slot]) == c + 1) {
-                const int32_t v = *((volatile int32_t*)&val[slot]);
-                atomicExch(&seq[slot], c + cap);  // free for push ticket c + cap
-                return v;
+            const unsigned long long w = *at(c);
+            const unsigned long long n = *reinterpret_cast<volatile unsigned long long*>(qc);
+            const int halt = *((volatile int32_t*)&qc[3]);
+            if ((int32_t)w == c + 1) {
+                *at(c) = word(0, c + cap);  // free for push ticket c + cap
+                if (c < visits) return (int32_t)(w >> 32);
+                break;
             }
-            if (*((volatile int32_t*)&qc[2]) == 0 || *((volatile int32_t*)&qc[4])) return -1;
-            __nanosleep(64);
+            if ((uint32_t)n == (uint32_t)(n >> 32) || halt) return -1;
+            __nanosleep(32);
         }
         stop(sc);
         return -1;
     }
 };
+static_assert(offsetof(DevScalars, counters) % 8 == 0, "the queue's two counts are one word");
 
 __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict__ eqm, float* sp,
                                                        const int32_t* __restrict__ cand, int32_t* tq, int tq_cap,
@@ -522,9 +531,7 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
     if (pass == 2 && sc->sinkcount_pass1 == 0) return;
     cg::grid_group grid = cg::this_grid();
     __shared__ float s_v[kPH * kPH];
-    __shared__ int16_t s_acell[kPT * kPT];  // active cells (halo index)
-    __shared__ uint8_t s_aeq[kPT * kPT];    //   directions of their equal-height neighbours
-    __shared__ float s_av0[kPT * kPT];      //   their values at the start of the visit
+    __shared__ uint32_t s_cell[kPT * kPT];  // active cells: halo index, directions of their equal-height neighbours above
     __shared__ int s_act[9];
     __shared__ int s_na, s_tile;
     const int W = k.W, H = k.H;
@@ -532,11 +539,11 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
     const int n = sc->n_cand;
     const size_t gstride = (size_t)gridDim.x * blockDim.x;
     const size_t gtid = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const TileQueue tqu{tq, tq + tq_cap, sc->counters, tq_cap};
+    const TileQueue tqu{reinterpret_cast<unsigned long long*>(tq), sc->counters, tq_cap};
     int32_t* const qc = tqu.qc;
     const int32_t qid = sc->round_id + 1;  // mark of a queued tile
-    if (gtid == 0) qc[0] = qc[1] = qc[2] = qc[3] = qc[4] = 0;
-    for (size_t i = gtid; i < (size_t)tq_cap; i += gstride) tqu.seq[i] = (int32_t)i;
+    if (gtid == 0) qc[0] = qc[1] = qc[2] = qc[3] = 0;
+    for (size_t i = gtid; i < (size_t)tq_cap; i += gstride) tqu.slot[i] = TileQueue::word(0, (int)i);
     grid.sync();
     for (size_t base = (size_t)blockIdx.x * blockDim.x; base < (size_t)n; base += gstride) {
         const size_t i = base + threadIdx.x;
@@ -556,16 +563,9 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
         const unsigned b = __ballot_sync(0xffffffffu, fresh);
         const int lane = threadIdx.x & 31, leader = b ? __ffs(b) - 1 : 0;
         int at = 0;
-        if (b && lane == leader) {
-            atomicAdd(&qc[2], __popc(b));
-            at = atomicAdd(&qc[0], __popc(b));
-        }
+        if (b && lane == leader) at = atomicAdd(&qc[0], __popc(b));
         at = __shfl_sync(0xffffffffu, at, leader) + __popc(b & ((1u << lane) - 1));
-        if (fresh) {
-            tqu.val[at % tq_cap] = t;
-            __threadfence();
-            atomicExch(&tqu.seq[at % tq_cap], at + 1);
-        }
+        if (fresh) *tqu.at(at) = TileQueue::word(t, at + 1);
     }
     grid.sync();
     const long long visit_cap = (long long)round_cap_of(sc) * max(1, *((volatile int32_t*)&qc[0]));
@@ -573,11 +573,7 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
     const int lx = threadIdx.x & 31, wy = threadIdx.x >> 5;
     for (;;) {
         if (threadIdx.x == 0) {
-            int32_t t = tqu.take(sc);
-            if (t >= 0 && atomicAdd(&qc[3], 1) >= visit_cap) {
-                tqu.stop(sc);
-                t = -1;
-            }
+            const int32_t t = tqu.take(visit_cap, sc);
             if (t >= 0) {
                 atomicExch(mark + t, qid - 1);  // taken: a later improvement queues it again
                 __threadfence();                // before the halo is read
@@ -616,39 +612,48 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
             if (threadIdx.x == 0) s_na = 0;
             __syncthreads();
             // The tile's active cells, listed: candidates (start value above 0)
-            // with an equal-height neighbour (a NaN cell, key 0, has none),
-            // with the directions of those neighbours and their start values.
+            // with an equal-height neighbour (a NaN cell, key 0, has none).
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const int sidx = (4 * wy + q + 1) * kPH + lx + 1;
-                const float v0 = s_v[sidx];
-                const uint32_t m = v0 > 0.f ? m4[q] : 0u;
+                const uint32_t m = s_v[sidx] > 0.f ? m4[q] : 0u;
                 const int slot = warp_slot(m != 0, &s_na);
-                if (slot >= 0) {
-                    s_acell[slot] = (int16_t)sidx;
-                    s_aeq[slot] = (uint8_t)m;
-                    s_av0[slot] = v0;
-                }
+                if (slot >= 0) s_cell[slot] = (uint32_t)sidx | (m << 16);
             }
             __syncthreads();
             const int na = s_na;
-            // Gauss-Seidel sweeps over the list, forward and backward in turn
+            // A thread's cells of the list (at most four), with the directions
+            // of their equal-height neighbours, in registers: only their owner
+            // lowers them.
+            uint32_t own[4];
+            float val[4], val0[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int i = threadIdx.x + 256 * q;
+                own[q] = i < na ? s_cell[i] : 0u;
+                val0[q] = val[q] = i < na ? s_v[own[q] & 0xffff] : 0.f;
+            }
+            // Gauss-Seidel sweeps over them.  All eight neighbours are read and
+            // the ones at another height then left out: tests around the loads
+            // took 1300 cycles a sweep.
             int sweep = 0;
             for (; sweep < kTileSweeps; ++sweep) {
                 bool ch = false;
-                for (int i = threadIdx.x; i < na; i += blockDim.x) {
-                    const int j = (sweep & 1) ? na - 1 - i : i;
-                    const int sidx = s_acell[j];
-                    const uint32_t m = s_aeq[j];
-                    const float cv = s_v[sidx];
-                    float best = cv;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (256 * q >= na) break;  // block-uniform
+                    const int sidx = own[q] ? (int)(own[q] & 0xffff) : kPH + 1;
+                    float nv[8];
+#pragma unroll
+                    for (int d = 0; d < 8; ++d) nv[d] = s_v[sidx + dir_dy(d) * kPH + dir_dx(d)];
+                    float best = val[q];
 #pragma unroll
                     for (int d = 0; d < 8; ++d) {
-                        const float nv = (m >> d) & 1u ? s_v[sidx + dir_dy(d) * kPH + dir_dx(d)] + ((d & 1) ? 1.41f : 1.0f)
-                                                       : cv;
-                        best = nv < best ? nv : best;
+                        const float x = nv[d] + ((d & 1) ? 1.41f : 1.0f);
+                        best = fminf(best, (own[q] & (0x10000u << d)) ? x : kFar);
                     }
-                    if (best < cv) {
+                    if (best < val[q]) {
+                        val[q] = best;
                         s_v[sidx] = best;
                         ch = true;
                     }
@@ -656,12 +661,13 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
                 if (!__syncthreads_or(ch)) break;
             }
             if (sweep == kTileSweeps && threadIdx.x == 0) s_act[4] = 1;  // not settled: visit again
-            for (int i = threadIdx.x; i < na; i += blockDim.x) {
-                const int sidx = s_acell[i];
+#pragma unroll 1
+            for (int q = 0; q < 4; ++q) {
+                const float v = val[q];
+                const int sidx = own[q] & 0xffff;
                 const int ly = sidx / kPH - 1, lx2 = sidx % kPH - 1;
                 const int gx = tx0 + lx2, gy = ty0 + ly;
-                const float v = s_v[sidx];
-                if (gx < W && gy < H && v < s_av0[i] &&
+                if (own[q] && gx < W && gy < H && v < val0[q] &&
                     __int_as_float(atomicMin(reinterpret_cast<int*>(sp) + (size_t)gy * W + gx, __float_as_int(v))) > v) {
                     // (the values are non-negative: their bits order as ints)
                     // a neighbouring tile can improve only through an
@@ -672,7 +678,7 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
                     if (ly == 0) out |= 0x83u;         // NW, N, NE
                     if (ly == kPT - 1) out |= 0x38u;   // SE, S, SW
 #pragma unroll 1
-                    for (uint32_t m = s_aeq[i] & out; m; m &= m - 1) {
+                    for (uint32_t m = (own[q] >> 16) & out; m; m &= m - 1) {
                         const int d = __ffs(m) - 1;
                         const int nx = lx2 + dir_dx(d), ny = ly + dir_dy(d);
                         s_act[3 * (ny < 0 ? 0 : (ny >= kPT ? 2 : 1)) + (nx < 0 ? 0 : (nx >= kPT ? 2 : 1))] = 1;
@@ -689,12 +695,12 @@ __global__ void __launch_bounds__(256) k_plateau_relax(const uint8_t* __restrict
                 }
             }
             __syncthreads();
-            if (threadIdx.x == 0) atomicSub(&qc[2], 1);  // this visit is over (its pushes came first)
+            if (threadIdx.x == 0) atomicAdd(&qc[1], 1);  // this visit is over (its pushes came first)
         }
     }
     grid.sync();
     if (gtid == 0) {
-        sc->plateau_sweeps += qc[3];
+        sc->plateau_sweeps += qc[1];
         sc->round_id = qid + 1;
     }
 }
