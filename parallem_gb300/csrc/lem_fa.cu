@@ -251,25 +251,6 @@ __global__ void __launch_bounds__(256, 4)
 // negative weight or a multi-direction code, and the walk then runs instead.
 
 
-__device__ __forceinline__ void tile_load(const double* __restrict__ z, const uint8_t* __restrict__ mask,
-                                          const uint8_t* __restrict__ fd, int W, int H, int tx0, int ty0,
-                                          uint8_t* s_code, uint8_t* s_cls) {
-    for (int j = threadIdx.x; j < kTH * kTH; j += blockDim.x) {
-        const int gx = tx0 - 1 + j % kTH, gy = ty0 - 1 + j / kTH;
-        uint8_t c = 0, cl = kCellOff;
-        if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-            const size_t g = (size_t)gy * W + gx;
-            c = fd[g];
-            if (mask[g])
-                cl = kCellIn;
-            else if (z[g] != kNoData)
-                cl = kCellBlock;
-        }
-        s_code[j] = c;
-        s_cls[j] = cl;
-    }
-}
-
 __global__ void __launch_bounds__(256, 6)
     k_fat_local(const double* __restrict__ z, const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
                 const float* __restrict__ w, int4* __restrict__ t_rec, int32_t* __restrict__ t_dst,
@@ -688,12 +669,16 @@ __global__ void __launch_bounds__(256)
     if (!sc->tiled_ok) return;
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
-    __shared__ uint8_t s_hok[kTH * kTH];
-    __shared__ float2 s_hval[kTH * kTH];
-    __shared__ int32_t s_pend[kTile * kTile];
-    __shared__ float2 s_val[kTile * kTile];
-    __shared__ int16_t s_q[kTile * kTile];
-    __shared__ int s_done, s_dem, s_qn, s_qend;
+    __shared__ float2 s_hval[kRing];  // the ring's accumulations
+    __shared__ uint8_t s_hok[kRing];  //   and whether they are final
+    __shared__ int32_t s_pd[kTile * kTile];
+    __shared__ int32_t s_h[kTile * kTile];
+    __shared__ float2 s_val[kTile * kTile + 1];
+    __shared__ __align__(4) uint16_t s_dm[kTile * kTile];
+    __shared__ uint32_t s_ent[kTile * kTile];
+    __shared__ uint32_t s_bins[kTile * kTile / 2];
+    __shared__ uint32_t s_wait[kTile], s_bad[kTile];
+    __shared__ int s_done, s_dem, s_qn;
     const int W = k.W, H = k.H, TW = (W + kTile - 1) / kTile;
     const int t = ts.tile(blockIdx.x);
     const int fc = t_fcnt[t];
@@ -704,11 +689,11 @@ __global__ void __launch_bounds__(256)
         const int ne = fc & 0xffff, nn = fc >> 16;
         const size_t tb = (size_t)t * kTile * kTile, pool = (size_t)t * kTilePool;
         float2* s_X = s_val;      // node sums
-        int32_t* s_ok = s_pend;  // node valid
+        int32_t* s_ok = s_pd;    // node valid
         // (the second wave's arrays are free here) per node: its largest input
         // node + 1 and its number of input nodes, and up to four input nodes
-        int16_t* s_nin = s_q;                                     // (largest + 1) | count << 11
-        int16_t* s_in4 = reinterpret_cast<int16_t*>(s_hval);      // [4 * node]
+        int16_t* s_nin = reinterpret_cast<int16_t*>(s_h);         // (largest + 1) | count << 11
+        int16_t* s_in4 = reinterpret_cast<int16_t*>(s_ent);       // [4 * node], a tile has fewer than 512 nodes
         for (int n = threadIdx.x; n < nn; n += blockDim.x) {
             const int meta = n_meta[tb + n];
             const int start = meta & 2047, nin = meta >> 11;
@@ -786,97 +771,116 @@ __global__ void __launch_bounds__(256)
         if (count && (threadIdx.x & 31) == 0 && done && dem >= 0) atomicAdd(&dc.out[dem].fa_done, done);
         return;
     }
+    // The second wave: every cell of the tile by the reference formula, in level
+    // order, with the donors in other tiles (outlets of theirs) at their final
+    // values.  A cell below a donor that never completes stays as it is, and an
+    // outlet keeps the coarse wave's value.
     const int tx0 = (t % TW) * kTile, ty0 = (t / TW) * kTile;
-    tile_load(z, mask, fd, W, H, tx0, ty0, s_code, s_cls);
-    // donors in other tiles: outlets of their tiles, final after the coarse wave
-    for (int j = threadIdx.x; j < kTH * kTH; j += blockDim.x) {
-        const int hx = j % kTH, hy = j / kTH;
-        if (hx != 0 && hx != kTH - 1 && hy != 0 && hy != kTH - 1) continue;
-        const int gx = tx0 - 1 + hx, gy = ty0 - 1 + hy;
-        uint8_t ok = 0;
+    const int lx = threadIdx.x & 31, ly0 = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < kTile * kTile / 2; i += blockDim.x) {
+        s_bins[i] = 0;
+        reinterpret_cast<uint32_t*>(s_dm)[i] = 0;
+    }
+    if (threadIdx.x < kTile) s_wait[threadIdx.x] = s_bad[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_done = s_qn = 0, s_dem = -1, s_val[kNoCell] = make_float2(0.f, 0.f);
+    __syncthreads();
+    tile_stage(
+        fd, [&](size_t g, int, int) { return mask[g] ? kCellIn : (z[g] == kNoData ? kCellOff : kCellBlock); }, W, H, tx0,
+        ty0, s_code, s_cls, s_dm, s_bad);
+    if (threadIdx.x < kRing) {
+        const int h = ring_halo(threadIdx.x);
+        const int gx = tx0 - 1 + h % kTH, gy = ty0 - 1 + h / kTH;
+        bool ok = false;
         float2 v = make_float2(0.f, 0.f);
         if (gx >= 0 && gx < W && gy >= 0 && gy < H && mask[(size_t)gy * W + gx]) {
             const size_t g = (size_t)gy * W + gx;
             ok = t_pend[g] == 0;
             v = fa[g];
         }
-        s_hok[j] = ok;
-        s_hval[j] = v;
+        s_hok[threadIdx.x] = ok;
+        s_hval[threadIdx.x] = v;
     }
-    if (threadIdx.x == 0) s_done = 0, s_dem = -1;
     __syncthreads();
-    const int lx = threadIdx.x & 31, ly0 = threadIdx.x >> 5;
+    // the neighbour in direction scan_dir(k) of cell l when it lies in another tile
+    auto ring_of = [&](int l, int k) {
+        const int d = scan_dir(k);
+        return ring_index((l & (kTile - 1)) + 1 + dir_dx(d), l / kTile + 1 + dir_dy(d));
+    };
+    auto sum = [&](int l) {  // CalcMFD's donor sum in scan order
+        const uint32_t dm = s_dm[l];
+        float2 acc = make_float2(0.f, 0.f);
+        for (uint32_t m = (dm | (dm >> 8)) & 255u; m; m &= m - 1) {
+            const int k = __ffs(m) - 1;
+            acc = ff_add(acc, (dm >> k) & 1u ? s_val[l + scan_step(k)] : s_hval[ring_of(l, k)]);
+        }
+        return acc.x < 0.0f ? make_float2(0.f, 0.f) : acc;
+    };
     int done = 0, dem = -1;  // one DEM per tile
-    bool outlet[4], src[4];
+    bool outlet[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        int32_t pend = kBlocked;
+        const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
+        int32_t pd = l;
         float wl = 0.f;
         outlet[q] = false;
         if (s_cls[hc] == kCellIn) {
-            pend = 0;
-#pragma unroll
-            for (int d = 0; d < 8; ++d) {
-                const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-                if (!donates(s_code[nh], d)) continue;
-                const uint8_t cl = s_cls[nh];
-                if (cl == kCellBlock)
-                    pend |= kBlocked;
-                else if (cl == kCellIn) {
-                    if (in_tile(lx + dir_dx(d), ly + dir_dy(d)))
-                        ++pend;
-                    else if (!s_hok[nh])
-                        pend |= kBlocked;
-                }
-            }
             const int d = bit_dir(s_code[hc]);
-            if (d >= 0 && s_cls[hc + dir_dy(d) * kTH + dir_dx(d)] == kCellIn &&
-                !in_tile(lx + dir_dx(d), ly + dir_dy(d))) {
-                outlet[q] = true;
-                if (t_pend[(size_t)(ty0 + ly) * W + tx0 + lx] == 0) ++done;
+            const int rlx = lx + dir_dx(d < 0 ? 0 : d), rly = ly + dir_dy(d < 0 ? 0 : d);
+            if (d >= 0 && s_cls[(rly + 1) * kTH + rlx + 1] == kCellIn) {
+                outlet[q] = !in_tile(rlx, rly);
+                if (!outlet[q]) pd = (rly * kTile + rlx) | (1 << 10);
             }
-            wl = w ? w[(size_t)(ty0 + ly) * W + tx0 + lx] : 1.0f;
-            if (dem < 0) dem = dem_at(dc, (size_t)(ty0 + ly) * W + tx0 + lx);
+            if (outlet[q] && t_pend[g] == 0) ++done;
+            wl = w ? w[g] : 1.0f;
+            if (dem < 0) dem = dem_at(dc, g);
+            for (uint32_t m = s_dm[l] >> 8; m; m &= m - 1)
+                if (!s_hok[ring_of(l, __ffs(m) - 1)]) atomicOr(&s_bad[ly], 1u << lx);
         }
-        s_pend[l] = pend;
-        src[q] = pend == 0 && !outlet[q];
+        s_pd[l] = pd;
+        s_h[l] = 0;
         s_val[l] = make_float2(wl, 0.f);
     }
     dem = __reduce_max_sync(0xffffffffu, dem);
-    if ((threadIdx.x & 31) == 0 && dem >= 0) atomicMax(&s_dem, dem);
-    if (threadIdx.x == 0) s_qn = 0;
+    if (lx == 0 && dem >= 0) atomicMax(&s_dem, dem);
     __syncthreads();
-    tile_wave(
-        [&](int cur, int rnd) {
-            const int cx = cur & (kTile - 1), cy = cur / kTile, hc = (cy + 1) * kTH + cx + 1;
-            float2 acc = make_float2(0.f, 0.f);
+    tile_paths(s_pd, s_h, s_wait, s_bad, lx, ly0);
+    int level[4];
 #pragma unroll
-            for (int kk = 0; kk < 8; ++kk) {
-                const int d = scan_dir(kk);
-                const int nlx = cx + dir_dx(d), nly = cy + dir_dy(d);
-                const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-                if (!donates(s_code[nh], d) || s_cls[nh] != kCellIn) continue;
-                acc = ff_add(acc, in_tile(nlx, nly) ? s_val[nly * kTile + nlx] : s_hval[nh]);
-            }
-            if (acc.x < 0.0f) acc = make_float2(0.f, 0.f);
-            const float2 v = ff_add(s_val[cur], acc);
-            s_val[cur] = v;
-            fa[(size_t)(ty0 + cy) * W + tx0 + cx] = v;
-            ++done;
-            const int d = bit_dir(s_code[hc]);
-            if (d < 0) return -1;
-            const int rlx = cx + dir_dx(d), rly = cy + dir_dy(d);
-            const int rh = hc + dir_dy(d) * kTH + dir_dx(d);
-            if (!in_tile(rlx, rly) || s_cls[rh] != kCellIn) return -1;
-            // an outlet keeps the coarse wave's value
-            const int dr = bit_dir(s_code[rh]);
-            if (dr >= 0 && s_cls[rh + dir_dy(dr) * kTH + dir_dx(dr)] == kCellIn &&
-                !in_tile(rlx + dir_dx(dr), rly + dir_dy(dr)))
-                return -1;
-            return rly * kTile + rlx;
+    for (int q = 0; q < 4; ++q) {
+        const int ly = ly0 + 8 * q, l = ly * kTile + lx;
+        const bool on = s_cls[(ly + 1) * kTH + lx + 1] == kCellIn && !((s_bad[ly] >> lx) & 1u) && !outlet[q];
+        level[q] = on ? s_h[l] : -1;
+        if (level[q] == 0) s_val[l] = ff_add(s_val[l], sum(l));  // donors in other tiles only
+    }
+    tile_sort(
+        level,
+        [&](int q) {
+            const int l = (ly0 + 8 * q) * kTile + lx;
+            return entry_of(l, s_dm[l] & 255u) | (s_dm[l] >> 8 ? kMoreDonors : 0u);
         },
-        s_pend, s_q, &s_qn, &s_qend, src, lx, ly0);
+        s_bins, kTile * kTile / 2, s_ent, &s_qn, lx);
+    struct Cell {
+        float2 w;
+        uint32_t e;
+    };
+    tile_levels(
+        [&](uint32_t e) { return Cell{s_val[entry_cell(e)], e}; },
+        [&](const Cell& f) {
+            const int c = entry_cell(f.e);
+            float2 acc = ff_add(s_val[entry_d0(f.e)], s_val[entry_d1(f.e)]);
+            if (acc.x < 0.0f) acc = make_float2(0.f, 0.f);
+            if (f.e & kMoreDonors) acc = sum(c);
+            s_val[c] = ff_add(f.w, acc);
+        },
+        1, kTile * kTile, s_bins, s_ent);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (level[q] < 0) continue;
+        const int ly = ly0 + 8 * q;
+        fa[(size_t)(ty0 + ly) * W + tx0 + lx] = s_val[ly * kTile + lx];
+        ++done;
+    }
     done = wsum(done);
     if ((threadIdx.x & 31) == 0 && done) atomicAdd(&s_done, done);
     __syncthreads();

@@ -425,21 +425,6 @@ __device__ __forceinline__ float4 map_compose(const float4 outer, const float4 i
     return make_float4(__fmul_rn(a1, inner.x), __fadd_rn(__fmul_rn(a1, inner.y), b1), lo, hi);
 }
 
-__device__ __forceinline__ void sed_tile_load(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd, int W,
-                                              int H, int tx0, int ty0, uint8_t* s_code, uint8_t* s_cls) {
-    for (int j = threadIdx.x; j < kTH * kTH; j += blockDim.x) {
-        const int gx = tx0 - 1 + j % kTH, gy = ty0 - 1 + j / kTH;
-        uint8_t c = 0, cl = kCellOff;
-        if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
-            const size_t g = (size_t)gy * W + gx;
-            c = fd[g];
-            cl = (mask[g] && gx != 0 && gy != 0) ? kCellIn : kCellBlock;
-        }
-        s_code[j] = c;
-        s_cls[j] = cl;
-    }
-}
-
 // Static part of a cell: deposition from all donors (in scan order), the mix
 // coefficients and the new soil thickness; pend counts donors inside the tile,
 // ext those outside, kBlocked marks a blocked donor.
@@ -1194,8 +1179,6 @@ __global__ void __launch_bounds__(256, 4)
     }
 }
 
-constexpr uint8_t kStatNz = 4;  // k_sedt_final: flag in a waiting cell's status
-
 __global__ void __launch_bounds__(256, 6)
     k_sedt_final(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd, const float* __restrict__ ero,
                  const float* __restrict__ inci, const float* __restrict__ geli, float* depo, float* stone,
@@ -1249,123 +1232,150 @@ __global__ void __launch_bounds__(256, 6)
         }
         return;
     }
+    // The second wave: the waiting cells by the per-cell formula, in level order,
+    // with the donors in other tiles at their final values.  The levels count
+    // waiting cells only; a cell below an inflow that never completes stays as it is,
+    // and an outlet keeps the coarse wave's value.
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
-    __shared__ uint8_t s_hok[kTH * kTH];
-    __shared__ float s_hval[kTH * kTH];
-    __shared__ int32_t s_pend[kTile * kTile];
-    __shared__ float s_new[kTile * kTile];
-    __shared__ uint8_t s_stat[kTile * kTile];  // 1 settled, 2 waiting; kStatNz: the sediment column is not empty
-    __shared__ float s_A[kTile * kTile];       // a waiting cell's deposition and stone-mix coefficients,
-    __shared__ float s_B[kTile * kTile];       //   computed before the wave so that its rounds read no
-    __shared__ float s_dep[kTile * kTile];     //   global memory
-    __shared__ float s_stn[kTile * kTile];
-    __shared__ int16_t s_q[kTile * kTile];
-    __shared__ int s_done, s_dem, s_qn, s_qend;
+    __shared__ float s_hval[kRing];   // the ring's stone
+    __shared__ uint8_t s_hok[kRing];  //   and whether it is final
+    __shared__ int32_t s_pd[kTile * kTile];
+    __shared__ int32_t s_h[kTile * kTile];
+    __shared__ float s_new[kTile * kTile + 1];
+    __shared__ float2 s_ab[kTile * kTile];  // a waiting cell's stone-mix coefficients
+    __shared__ __align__(4) uint16_t s_dm[kTile * kTile];
+    __shared__ uint32_t s_ent[kTile * kTile];
+    __shared__ uint32_t s_bins[kTile * kTile / 2];
+    __shared__ uint32_t s_wait[kTile], s_bad[kTile], s_nz[kTile];  // rows of cells
+    __shared__ int s_done, s_dem, s_qn;
     const int W = k.W, H = k.H, TW = (W + kTile - 1) / kTile;
     const int tx0 = (t % TW) * kTile, ty0 = (t / TW) * kTile;
-    sed_tile_load(mask, fd, W, H, tx0, ty0, s_code, s_cls);
+    const int lx = threadIdx.x & 31, ly0 = threadIdx.x >> 5;
+    for (int i = threadIdx.x; i < kTile * kTile / 2; i += blockDim.x) {
+        s_bins[i] = 0;
+        reinterpret_cast<uint32_t*>(s_dm)[i] = 0;
+    }
+    if (threadIdx.x < kTile) s_wait[threadIdx.x] = s_bad[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_done = s_qn = 0, s_dem = -1, s_new[kNoCell] = 0.f;
+    __syncthreads();
+    tile_stage(
+        fd, [&](size_t g, int x, int y) { return mask[g] && x != 0 && y != 0 ? kCellIn : kCellBlock; }, W, H, tx0, ty0,
+        s_code, s_cls, s_dm, s_bad);
     if (threadIdx.x < kRing) {
         const int h = ring_halo(threadIdx.x);
         const int gx = tx0 - 1 + h % kTH, gy = ty0 - 1 + h / kTH;
-        uint8_t ok = 0;
+        bool ok = false;
         float v = 0.f;
         if (gx >= 0 && gx < W && gy >= 0 && gy < H) {
             const size_t g = (size_t)gy * W + gx;
             ok = t_pend[g] == 0;
             v = __ldcg(stone + g);
         }
-        s_hok[h] = ok;
-        s_hval[h] = v;
+        s_hok[threadIdx.x] = ok;
+        s_hval[threadIdx.x] = v;
     }
-    if (threadIdx.x == 0) s_done = 0, s_dem = -1;
     __syncthreads();
-    const int lx = threadIdx.x & 31, ly0 = threadIdx.x >> 5;
+    // the neighbour in direction scan_dir(k) of cell l when it lies in another tile
+    auto ring_of = [&](int l, int kk) {
+        const int d = scan_dir(kk);
+        return ring_index((l & (kTile - 1)) + 1 + dir_dx(d), l / kTile + 1 + dir_dy(d));
+    };
+    auto sum = [&](int l) {  // the donors' stone in scan order
+        const uint32_t dm = s_dm[l];
+        float from = 0.f;
+        for (uint32_t m = (dm | (dm >> 8)) & 255u; m; m &= m - 1) {
+            const int kk = __ffs(m) - 1;
+            from = __fadd_rn(from, __fmul_rn(1.0f, (dm >> kk) & 1u ? s_new[l + scan_step(kk)] : s_hval[ring_of(l, kk)]));
+        }
+        return from;
+    };
     int done = 0, dem = -1;  // one DEM per tile
-    bool src[4], outlet[4];
+    bool waits[4];
+    float dep[4], stn[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const int ly = ly0 + 8 * q, l = ly * kTile + lx, hc = (ly + 1) * kTH + lx + 1;
-        int32_t pend = kBlocked;
-        uint8_t st = 0;
+        int32_t pd = l;
         float v = 0.f;
-        outlet[q] = false;
+        bool nz = false;
+        waits[q] = false;
+        dep[q] = stn[q] = 0.f;
         if (s_cls[hc] == kCellIn) {
             const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
-            pend = 0;
-#pragma unroll
-            for (int d = 0; d < 8; ++d) {
-                const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
-                if (!donates(s_code[nh], d)) continue;
-                const uint8_t cl = s_cls[nh];
-                if (cl == kCellBlock)
-                    pend |= kBlocked;
-                else if (cl == kCellIn) {
-                    if (in_tile(lx + dir_dx(d), ly + dir_dy(d)))
-                        ++pend;
-                    else if (!s_hok[nh])
-                        pend |= kBlocked;
-                }
-            }
             const int d = bit_dir(s_code[hc]);
-            if (d >= 0 && s_cls[hc + dir_dy(d) * kTH + dir_dx(d)] == kCellIn &&
-                !in_tile(lx + dir_dx(d), ly + dir_dy(d))) {
-                outlet[q] = true;
-                if (t_stat[g] == 2 && t_pend[g] == 0) ++done;
-            }
-            st = t_stat[g];
+            const int rlx = lx + dir_dx(d < 0 ? 0 : d), rly = ly + dir_dy(d < 0 ? 0 : d);
+            const bool rin = d >= 0 && s_cls[(rly + 1) * kTH + rlx + 1] == kCellIn;
+            const bool outlet = rin && !in_tile(rlx, rly);
+            const bool st2 = t_stat[g] == 2;
+            if (outlet && st2 && t_pend[g] == 0) ++done;
             v = __ldcg(stone + g);
             if (dem < 0) dem = dem_at(dc, g);
-            if (st == 2 && !outlet[q]) {
+            if (st2 && !outlet) {
+                waits[q] = true;
+                if (rin) pd = (rly * kTile + rlx) | (1 << 10);
                 const SedInit in = sed_init(s_code, s_cls, lx, ly, tx0, ty0, W, ero, inci, geli, soilT, stone, k);
-                s_A[l] = in.L.A;
-                s_B[l] = in.L.B;
-                s_dep[l] = in.L.dep;
-                s_stn[l] = in.L.stn;
-                if (in.L.nz) st |= kStatNz;
+                s_ab[l] = make_float2(in.L.A, in.L.B);
+                dep[q] = in.L.dep;
+                stn[q] = in.L.stn;
+                nz = in.L.nz;
+                for (uint32_t m = s_dm[l] >> 8; m; m &= m - 1)
+                    if (!s_hok[ring_of(l, __ffs(m) - 1)]) atomicOr(&s_bad[ly], 1u << lx);
             }
         }
-        s_pend[l] = pend;
-        s_stat[l] = st;
+        const unsigned nb = __ballot_sync(0xffffffffu, nz);
+        if (lx == 0) s_nz[ly] = nb;
+        s_pd[l] = pd;
+        s_h[l] = 0;
         s_new[l] = v;
-        src[q] = pend == 0;
     }
     dem = __reduce_max_sync(0xffffffffu, dem);
-    if ((threadIdx.x & 31) == 0 && dem >= 0) atomicMax(&s_dem, dem);
-    if (threadIdx.x == 0) s_qn = 0;
+    if (lx == 0 && dem >= 0) atomicMax(&s_dem, dem);
     __syncthreads();
-    tile_wave(
-        [&](int cur, int rnd) {
-            const int cx = cur & (kTile - 1), cy = cur / kTile, hc = (cy + 1) * kTH + cx + 1;
-            const int d = bit_dir(s_code[hc]);
-            const int rlx = cx + (d >= 0 ? dir_dx(d) : 0), rly = cy + (d >= 0 ? dir_dy(d) : 0);
-            const bool rin = d >= 0 && s_cls[hc + dir_dy(d) * kTH + dir_dx(d)] == kCellIn;
-            if (rin && !in_tile(rlx, rly)) return -1;  // an outlet: the coarse wave stored it
-            const uint8_t stc = s_stat[cur];
-            if ((stc & 3) == 2) {
-                float from = 0.f;
+    tile_paths(s_pd, s_h, s_wait, s_bad, lx, ly0);
+    int level[4];
 #pragma unroll
-                for (int kk = 0; kk < 8; ++kk) {
-                    const int dd = scan_dir(kk);
-                    const int nlx = cx + dir_dx(dd), nly = cy + dir_dy(dd);
-                    const int nh = hc + dir_dy(dd) * kTH + dir_dx(dd);
-                    if (!donates(s_code[nh], dd) || s_cls[nh] != kCellIn) continue;
-                    from = __fadd_rn(from, __fmul_rn(1.0f, in_tile(nlx, nly) ? s_new[nly * kTile + nlx] : s_hval[nh]));
-                }
-                SedLocal L;
-                L.A = s_A[cur];
-                L.B = s_B[cur];
-                L.dep = s_dep[cur];
-                L.stn = s_stn[cur];
-                L.nz = (stc & kStatNz) != 0;
-                const float sn = L.nz ? sed_mix(L.A, L.B, from) : s_new[cur];
-                s_new[cur] = sn;
-                sed_store((size_t)(ty0 + cy) * W + tx0 + cx, L, sn, depo, stone, fines, soilT);
-                ++done;
-            }
-            return rin ? rly * kTile + rlx : -1;
+    for (int q = 0; q < 4; ++q) {
+        const int ly = ly0 + 8 * q, l = ly * kTile + lx;
+        level[q] = waits[q] && !((s_bad[ly] >> lx) & 1u) ? s_h[l] : -1;
+        // no waiting donor in the tile (the others' stone is not written here)
+        if (level[q] == 0 && ((s_nz[ly] >> lx) & 1u)) s_new[l] = sed_mix(s_ab[l].x, s_ab[l].y, sum(l));
+    }
+    tile_sort(
+        level,
+        [&](int q) {
+            const int l = (ly0 + 8 * q) * kTile + lx;
+            return entry_of(l, s_dm[l] & 255u) | (s_dm[l] >> 8 ? kMoreDonors : 0u);
         },
-        s_pend, s_q, &s_qn, &s_qend, src, lx, ly0);
+        s_bins, kTile * kTile / 2, s_ent, &s_qn, lx);
+    struct Cell {
+        float2 ab;
+        uint32_t e;
+        bool nz;
+    };
+    tile_levels(
+        [&](uint32_t e) {
+            const int c = entry_cell(e) & kPtr;
+            return Cell{s_ab[c], e, entry_cell(e) != kNoCell && ((s_nz[c / kTile] >> (c & (kTile - 1))) & 1u)};
+        },
+        [&](const Cell& f) {
+            float from = __fadd_rn(__fadd_rn(0.f, s_new[entry_d0(f.e)]), s_new[entry_d1(f.e)]);
+            if (f.e & kMoreDonors) from = sum(entry_cell(f.e));
+            const float sn = sed_mix(f.ab.x, f.ab.y, from);
+            if (f.nz) s_new[entry_cell(f.e)] = sn;
+        },
+        1, kTile * kTile, s_bins, s_ent);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (level[q] < 0) continue;
+        const int ly = ly0 + 8 * q, l = ly * kTile + lx;
+        SedLocal L;
+        L.dep = dep[q];
+        L.stn = stn[q];
+        L.nz = (s_nz[ly] >> lx) & 1u;
+        sed_store((size_t)(ty0 + ly) * W + tx0 + lx, L, s_new[l], depo, stone, fines, soilT);
+        ++done;
+    }
     done = wsum(done);
     if ((threadIdx.x & 31) == 0 && done) atomicAdd(&s_done, done);
     __syncthreads();
