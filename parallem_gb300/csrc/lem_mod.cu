@@ -493,16 +493,12 @@ __global__ void __launch_bounds__(256, 5)
     __shared__ uint8_t s_code[kTH * kTH];
     __shared__ uint8_t s_cls[kTH * kTH];
     __shared__ float s_new[C + 1];  // settled stone (the old stone until then)
-    // A, B, deposition and soil thickness per cell; before them, the halo's
-    // erosion terms (3 kTH x kTH floats) for the set-up
-    __shared__ float s_coef[4 * C];
-    float* const s_A = s_coef;
-    float* const s_B = s_coef + C;
-    float* const s_dep = s_coef + 2 * C;
-    float* const s_stn = s_coef + 3 * C;
-    float* const s_ero = s_coef;
-    float* const s_inc = s_coef + kTH * kTH;
-    float* const s_gel = s_coef + 2 * kTH * kTH;
+    // A, B, deposition and soil thickness per cell, then (between nodes) the cell's
+    // map; before them, the halo's erosion terms (3 kTH x kTH floats) for the set-up
+    __shared__ float4 s_cf[C];
+    float* const s_ero = reinterpret_cast<float*>(s_cf);
+    float* const s_inc = s_ero + kTH * kTH;
+    float* const s_gel = s_inc + kTH * kTH;
     // the in-tile paths (tile_paths), then where each ends, and the outlets' slots
     __shared__ int32_t s_pd[C];
     int16_t* const s_end = reinterpret_cast<int16_t*>(s_pd);
@@ -517,7 +513,8 @@ __global__ void __launch_bounds__(256, 5)
     // the settled cells by level, then the nodes by level and each node's slot
     __shared__ uint32_t s_ent[C];
     int16_t* const s_pos = reinterpret_cast<int16_t*>(s_ent + kMaxNodes);
-    // sorting bins, then the node at the top of a cell's run
+    // sorting bins, then the cell below in a run (-1: none), then the node at the top
+    // of a cell's run
     __shared__ uint32_t s_bins[C / 2];
     int16_t* const s_up = reinterpret_cast<int16_t*>(s_bins);
     __shared__ uint32_t s_wait[kTile], s_bad[kTile];
@@ -562,7 +559,7 @@ __global__ void __launch_bounds__(256, 5)
         s_gel[j] = g;
     }
     __syncthreads();
-    float cA[4], cB[4], cD[4], cS[4];  // the cells' coefficients until the staged terms are spent
+    float4 cf[4];                      // the cells' coefficients until the staged terms are spent
     int dem = -1;                      // one DEM per tile
     const float omd = 1.0f - k.ddk, omc = 1.0f - k.dck, omg = 1.0f - k.dgk;
 #pragma unroll
@@ -571,7 +568,7 @@ __global__ void __launch_bounds__(256, 5)
         uint32_t info = kKindEnd, dm = 0;
         int32_t pd = l;
         float snew = 0.f;
-        cA[q] = cB[q] = cD[q] = cS[q] = 0.f;
+        cf[q] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (s_cls[hc] == kCellIn) {
             const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
             snew = __ldcg(stone + g);
@@ -586,10 +583,7 @@ __global__ void __launch_bounds__(256, 5)
             }
             const SedLocal in =
                 sed_local(ad, ac, ag, s_ero[hc], s_inc[hc], s_gel[hc], st0, snew, k.ddk, k.dck, k.dgk);
-            cA[q] = in.A;
-            cB[q] = in.B;
-            cD[q] = in.dep;
-            cS[q] = in.stn;
+            cf[q] = make_float4(in.A, in.B, in.dep, in.stn);
             if (dem < 0) dem = dem_at(dc, g);
             const int d = bit_dir(s_code[hc]);
             const int rlx = lx + dir_dx(d < 0 ? 0 : d), rly = ly + dir_dy(d < 0 ? 0 : d);
@@ -610,13 +604,7 @@ __global__ void __launch_bounds__(256, 5)
     if (lx == 0 && dem >= 0) atomicMax(&s_dem, dem);
     __syncthreads();  // the staged erosion terms are spent
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const int l = (ly0 + 8 * q) * kTile + lx;
-        s_A[l] = cA[q];
-        s_B[l] = cB[q];
-        s_dep[l] = cD[q];
-        s_stn[l] = cS[q];
-    }
+    for (int q = 0; q < 4; ++q) s_cf[(ly0 + 8 * q) * kTile + lx] = cf[q];
     tile_paths(s_pd, s_h, s_wait, s_bad, lx, ly0);
     int key[4];
     int16_t end[4];
@@ -630,7 +618,7 @@ __global__ void __launch_bounds__(256, 5)
         end[q] = (int16_t)(s_pd[l] & kPtr);
         s_info[l] = (uint8_t)(info | (done ? kSedDone : 0) | (taint ? kSedTaint : 0));
         // a settled cell without donors mixes with nothing
-        if (key[q] == 0 && (info & kSedNz)) s_new[l] = sed_mix(s_A[l], s_B[l], 0.0f);
+        if (key[q] == 0 && (info & kSedNz)) s_new[l] = sed_mix(s_cf[l].x, s_cf[l].y, 0.0f);
     }
     constexpr uint8_t kWaits = kSedDone | kSedTaint;
     tile_sort(
@@ -652,7 +640,7 @@ __global__ void __launch_bounds__(256, 5)
     tile_levels(
         [&](uint32_t e) {
             const int c = entry_cell(e) & kPtr;  // (kNoCell's coefficients are not used)
-            return Cell{s_A[c], s_B[c], e, entry_cell(e) != kNoCell && (s_info[c] & kSedNz)};
+            return Cell{s_cf[c].x, s_cf[c].y, e, entry_cell(e) != kNoCell && (s_info[c] & kSedNz)};
         },
         [&](const Cell& f) {
             float from = __fadd_rn(__fadd_rn(0.f, s_new[entry_d0(f.e)]), s_new[entry_d1(f.e)]);
@@ -678,13 +666,13 @@ __global__ void __launch_bounds__(256, 5)
         const bool out = (s_info[e] & kSedKind) == kKindOutlet;
         if ((info & kWaits) == kSedDone) {
             ++done;
-            depo[g] = s_dep[l];
+            depo[g] = s_cf[l].z;
             if (info & kSedNz) {
                 const float sn = s_new[l];
                 __stcg(stone + g, sn);
                 fines[g] = __fsub_rn(100.0f, sn);
             }
-            soilT[g] = s_stn[l];
+            soilT[g] = s_cf[l].w;
         }
         if (info & kSedEntry) t_dst[g] = out ? (int32_t)((ty0 + e / kTile) * W + tx0 + (e & (kTile - 1))) : -1;
         stray |= (info & kWaits) == kWaits && !out;
@@ -748,17 +736,26 @@ __global__ void __launch_bounds__(256, 5)
         const bool waits = (s_info[l] & kWaits) == kWaits && (s_info[end[q]] & kSedKind) == kKindOutlet;
         fslot[q] = warp_slot(waits && !second_wave, &s_fn);
         if (!waits) continue;
-        if (fslot[q] >= 0) f_ds[fbase + fslot[q]] = make_float2(s_dep[l], s_stn[l]);
+        if (fslot[q] >= 0) f_ds[fbase + fslot[q]] = make_float2(s_cf[l].z, s_cf[l].w);
         if (s_node[l]) continue;
         float Cc = 0.f;
         const uint32_t dm = s_dm[l];
         for (uint32_t m = dm & ~(dm >> 8) & 255u; m; m &= m - 1)
             Cc = __fadd_rn(Cc, __fmul_rn(1.0f, s_new[l + scan_step(__ffs(m) - 1)]));
-        const float4 M = map_cell(s_A[l], s_B[l], Cc, (s_info[l] & kSedNz) != 0, s_new[l]);
-        s_A[l] = M.x;
-        s_B[l] = M.y;
-        s_dep[l] = M.z;
-        s_stn[l] = M.w;
+        s_cf[l] = map_cell(s_cf[l].x, s_cf[l].y, Cc, (s_info[l] & kSedNz) != 0, s_new[l]);
+    }
+    // the cell below in the same run: waiting and no node
+    int16_t* const s_down = s_up;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int ly = ly0 + 8 * q, l = ly * kTile + lx;
+        int c = -1;
+        if ((s_info[l] & (kWaits | kSedKind)) == (kWaits | kKindIn)) {
+            const int d = bit_dir(s_code[(ly + 1) * kTH + lx + 1]);
+            c = l + dir_dy(d) * kTile + dir_dx(d);
+            if ((s_info[c] & kWaits) != kWaits || s_node[c]) c = -1;
+        }
+        s_down[l] = (int16_t)c;
     }
     const int no = s_no, nt = s_nt;
     if (threadIdx.x < 32) outlet_starts(s_pcnt, s_pstart, no);
@@ -769,21 +766,13 @@ __global__ void __launch_bounds__(256, 5)
     // share a cell (a cell between nodes has one waiting donor).
     for (int i = threadIdx.x; i < nt; i += blockDim.x) {
         const int l = (int)s_ent[i];
-        if ((s_info[l] & kSedKind) != kKindIn) continue;
         float4 F = map_identity();
-        int c = l;
-        for (int guard = 0; guard < C; ++guard) {
-            const int d = bit_dir(s_code[(c / kTile + 1) * kTH + (c & (kTile - 1)) + 1]);
-            c += dir_dy(d) * kTile + dir_dx(d);  // in the tile: c is not an outlet
-            const uint32_t info = s_info[c];
-            if ((info & kWaits) != kWaits || s_node[c]) break;
-            F = map_compose(make_float4(s_A[c], s_B[c], s_dep[c], s_stn[c]), F);
-            s_A[c] = F.x;
-            s_B[c] = F.y;
-            s_dep[c] = F.z;
-            s_stn[c] = F.w;
+        for (int c = s_down[l], guard = 0; c >= 0 && guard < C; ++guard) {
+            const int below = s_down[c];
+            F = map_compose(s_cf[c], F);
+            s_cf[c] = F;
             s_up[c] = (int16_t)l;
-            if ((info & kSedKind) != kKindIn) break;
+            c = below;
         }
     }
     const int j = threadIdx.x;
@@ -845,7 +834,7 @@ __global__ void __launch_bounds__(256, 5)
             } else {
                 // the node that feeds this input, through the single-input cells in between
                 if (!s_node[cur]) {
-                    H = make_float4(s_A[cur], s_B[cur], s_dep[cur], s_stn[cur]);
+                    H = s_cf[cur];
                     cur = s_up[cur];
                 }
                 ref = -(s_pos[cur] - first + 1);
@@ -854,7 +843,7 @@ __global__ void __launch_bounds__(256, 5)
             p_map[pool + start + m] = H;
             ++m;
         }
-        p_abc[nbase + pos] = make_float4(s_A[l], s_B[l], Cc,
+        p_abc[nbase + pos] = make_float4(s_cf[l].x, s_cf[l].y, Cc,
                                          __int_as_float(start | (m << 11) | (s_info[l] & kSedNz ? 1 << 15 : 0)));
     }
     // the final pass's slots: a node reads its own value, a cell between nodes
@@ -871,7 +860,7 @@ __global__ void __launch_bounds__(256, 5)
                                             (ty0 + e / kTile) * W + tx0 + (e & (kTile - 1)),
                                             (info & kSedNz ? kFinNz : 0) |
                                                 ((info & kSedKind) == kKindOutlet ? kFinOutlet : 0));
-        f_map[fbase + fslot[q]] = node ? map_identity() : make_float4(s_A[l], s_B[l], s_dep[l], s_stn[l]);
+        f_map[fbase + fslot[q]] = node ? map_identity() : s_cf[l];
     }
     if (threadIdx.x == 0) t_fcnt[t] = second_wave ? -1 : s_fn;
     int32_t og = 0;
@@ -881,7 +870,7 @@ __global__ void __launch_bounds__(256, 5)
         og = (ty0 + o / kTile) * W + tx0 + (o & (kTile - 1));
         // (the coefficients of a waiting outlet, a node, are still in place)
         t_rec[og] = make_int4((pstart << 16) | (pcnt & 0xffff), (pstart & ~0xffff) | (pcnt >> 16),
-                              __float_as_int(s_dep[o]), __float_as_int(s_stn[o]));
+                              __float_as_int(s_cf[o].z), __float_as_int(s_cf[o].w));
         t_pend[og] = opend;
         if (opend == 0) og = ~og;  // settled here: a source of the coarse wave
     }
