@@ -49,6 +49,15 @@ __device__ __forceinline__ double dkey_inv(uint64_t k) {
     return __longlong_as_double((long long)b);
 }
 
+// A float as the double of the same value, without the FP64 pipe, which takes
+// two lanes a clock: a normal number's bits are rebiased, the others (zero, the
+// subnormal ones, infinities, NaN) take the conversion.
+__device__ __forceinline__ double dwiden(float f) {
+    const uint32_t b = __float_as_uint(f), m = b & 0x7FFFFFFFu;
+    if (m - 0x00800000u >= 0x7F000000u) return (double)f;
+    return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
 // Split of a double into an fp32 head (mantissa truncated to 24 bits) and an fp32
 // tail holding the next 24 bits, with integer operations only.  |z - hi - lo| <=
 // 2^-47 |z| for normal fp32-range magnitudes; tiny magnitudes collapse to zero.

@@ -478,8 +478,8 @@ constexpr int kMaxNodes = 512;  // nodes of a tile: entries (124 border cells), 
 // Bound by the chains of its one-warp phases (levels, runs) on few resident tiles
 // rather than by memory.  The cells settle in level order (see tile_levels) in the
 // place of a queue, donors and node inputs come from masks set while the codes are
-// staged, and shared arrays are reused so that five tiles share an SM: 1.55 -> 1.21
-// ms at 4096 x 4096 cells, 53 -> 45 us for a few tiles.
+// staged, runs follow stored links, and shared arrays are reused so that five tiles
+// share an SM: 1.55 -> 1.16 ms at 4096 x 4096 cells, 53 -> 43 us for a few tiles.
 __global__ void __launch_bounds__(256, 5)
     k_sedt_local(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd, const float* __restrict__ ero,
                  const float* __restrict__ inci, const float* __restrict__ geli, float* depo, float* stone,
@@ -1379,7 +1379,10 @@ __device__ __forceinline__ float dreybrodt(const float* tab, float T) {
     return tab[j] + f * (tab[j + 1] - tab[j]);
 }
 
-// six blocks per SM: a few spilled registers, measured faster than four
+// Bound by the instructions issued and by the FP64 pipe: three fp64 sums a cell,
+// which takes two lanes a clock (the conversions and the test against the base
+// level kept it busy as well: 441 -> 418 us at 4096 x 4096 cells without them).
+// Six blocks per SM: a few spilled registers, measured faster than four.
 __global__ void __launch_bounds__(256, 6)
     k_final(double* __restrict__ z, const double* __restrict__ z_init, const uint8_t* __restrict__ mask,
             const float2* __restrict__ fa, const float* __restrict__ ero, const float* __restrict__ inci,
@@ -1397,6 +1400,7 @@ __global__ void __launch_bounds__(256, 6)
     const int outlet_clim = o.outlet_clim;  // the cell whose climate elevation is outlet_z_clim
     const double outlet_z = o.outlet_z_clim;
     const double base = o.base_level;
+    const uint64_t base_key = dkey(base);
     const float rain0 = (float)c.rain, rinc = (float)c.rain_inc;
     const float dtemp_scalar = (float)(c.temp - c.temp0);
     BlockSums<4> sums(red);
@@ -1470,8 +1474,10 @@ __global__ void __launch_bounds__(256, 6)
         if ((int)i == outlet) {
             zn = base - 0.00012;
         } else {
-            zn = ((zn + (double)dz) - (double)wC) - (double)wP;
-            if (zn <= base) zn = base + 0.01;
+            // the sums are fp64, the conversions and the test take the integer pipe
+            zn = ((zn + dwiden(dz)) - dwiden(wC)) - dwiden(wP);
+            const uint64_t kn = dkey(zn);
+            if (kn != 0 && kn <= base_key) zn = base + 0.01;  // (NaN: no order)
         }
         z[i] = zn;
         // update_nutrient_content (updates.cu:48-76)
