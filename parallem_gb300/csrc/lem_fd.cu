@@ -849,6 +849,12 @@ __global__ void __launch_bounds__(256)
 
 // init_watershed_sinkMFD loop (newflow.cu:430-460): equal-height sink cells
 // adopt the largest neighbouring id until nothing changes.
+//
+// Bound by the trips to memory of a round.  A sink's neighbours are read in two
+// batches (elevations, then the ids of the equal ones), and ids also travel by way
+// of the cell they came from, so that the rounds grow with the logarithm of a
+// flat's width and not with the width: 133 -> 70 us for sixteen DEMs of 256 to 2048
+// cells a side, 76 -> 32 us for twelve of 128 to 1024.
 __global__ void k_flood_merge(const double* __restrict__ z, int32_t* ws, const int32_t* __restrict__ sinks,
                               int32_t* merging, ModelConsts k, DevScalars* sc) {
     if (sc->sinkcount_pass1 == 0) return;
@@ -863,28 +869,38 @@ __global__ void k_flood_merge(const double* __restrict__ z, int32_t* ws, const i
         *nmerge = 0;
     }
     grid.sync();
-    // one sink: adopt the largest id of its equal-height neighbours; false for
-    // a sink with none (a strict pit), which no later round needs to visit
+    // one sink: adopt the largest id of its equal-height neighbours, or the one
+    // that the cell its own id came from (in the same flat) has by now, and pass it
+    // on to that cell; false for a sink with no such neighbour (a strict pit), which
+    // no later round needs to visit
     auto relax = [&](int32_t c, int& changed) {
         const int x = c % W, y = c / W;
         const unsigned long long kc = dkey(z[c]);
         const int32_t mine = __ldcg(ws + c);
-        int32_t best = mine;
-        bool eq = false;
-        for (int d = 0; kc != 0 && d < 8; ++d) {
+        double zn[8];
+#pragma unroll
+        for (int d = 0; d < 8; ++d) {
             const int nx = x + dir_dx(d), ny = y + dir_dy(d);
-            if (nx < 0 || nx >= W || ny < 0 || ny >= H) continue;
-            const size_t nb = (size_t)ny * W + nx;
-            if (dkey(z[nb]) != kc) continue;
-            eq = true;
-            const int32_t o = __ldcg(ws + nb);
-            if (o > best) best = o;
+            const bool in = nx >= 0 && nx < W && ny >= 0 && ny < H;
+            zn[d] = in ? z[(size_t)ny * W + nx] : __longlong_as_double(-1);  // a NaN: equal to nothing
         }
+        uint32_t eq = 0;
+#pragma unroll
+        for (int d = 0; d < 8; ++d) eq |= kc != 0 && dkey(zn[d]) == kc ? 1u << d : 0u;
+        int32_t id[8];
+#pragma unroll
+        for (int d = 0; d < 8; ++d)
+            id[d] = (eq >> d) & 1u ? __ldcg(ws + ((ptrdiff_t)c + dir_dy(d) * (ptrdiff_t)W + dir_dx(d))) : mine;
+        // an id is the number, from one, of the sink cell it started at
+        int32_t best = max(mine, __ldcg(ws + max(mine, 1) - 1));
+#pragma unroll
+        for (int d = 0; d < 8; ++d) best = max(best, id[d]);
         if (best > mine) {
             atomicMax(ws + c, best);
+            if (mine > 0) atomicMax(ws + mine - 1, best);
             changed = 1;
         }
-        return eq;
+        return eq != 0;
     };
     int round = 0;
     for (;; ++round) {

@@ -105,3 +105,13 @@ def test_spill_heights_of_tied_boundaries(libs, n):
     # whole metres: many boundaries tie; above zero, since the reference takes a spill height of 0 for none
     z = np.where(z == NODATA, NODATA, np.floor(z) + 100.0)
     run_steps(libs, z, 1, np.full(1, 900.0), np.full(1, 9.0), False)
+
+
+@pytest.mark.parametrize("n", [12, 65, 200])
+def test_ids_of_winding_closed_flats(libs, n):
+    z = tilted(n, n, 0.8, 0.5)
+    # a winding pit floor as long as the grid has room for: every cell of it is a sink of one basin
+    for i, y in enumerate(range(4, n - 5, 3)):
+        z[y, 4:n - 4] = 50.0
+        z[y:min(y + 4, n - 5), 4 if i % 2 else n - 5] = 50.0
+    run_steps(libs, z, 1, np.full(1, 900.0), np.full(1, 9.0), False)
