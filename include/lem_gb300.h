@@ -102,7 +102,7 @@ typedef struct lem_totals {
     int32_t sed_uncomputed;  /* masked-in cells left out of sediment routing */
     int32_t merge_rounds;    /* sink flooding: rounds of the equal-height label merge   */
     int32_t label_rounds;    /*   rounds of the basin labelling (pointer jumping)       */
-    int32_t spill_rounds;    /*   rounds of the minimax spill relaxation                */
+    int32_t spill_rounds;    /*   rounds of the minimax spill (components merging)      */
     int32_t pad;
 } lem_totals;
 
