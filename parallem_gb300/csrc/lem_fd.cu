@@ -891,8 +891,9 @@ __global__ void k_flood_merge(const double* __restrict__ z, int32_t* ws, const i
 #pragma unroll
         for (int d = 0; d < 8; ++d)
             id[d] = (eq >> d) & 1u ? __ldcg(ws + ((ptrdiff_t)c + dir_dy(d) * (ptrdiff_t)W + dir_dx(d))) : mine;
-        // an id is the number, from one, of the sink cell it started at
-        int32_t best = max(mine, __ldcg(ws + max(mine, 1) - 1));
+        // an id is the number, from one, of the sink cell it started at; a sink on the
+        // grid's edge may have none (0) and has no such cell to follow
+        int32_t best = max(mine, __ldcg(ws + (mine > 0 ? mine - 1 : c)));
 #pragma unroll
         for (int d = 0; d < 8; ++d) best = max(best, id[d]);
         if (best > mine) {

@@ -8,6 +8,7 @@
 * The stateless accumulation, tiled and by the general wave, and the tiled
   contributing counts.
 * Spill heights: boundaries that tie, on few edges (one block) and on many.
+* Ids of flats that lie on the edge of a grid without a nodata ring.
 
 The tolerances are those of tests/test_gpu_parity.py.
 """
@@ -16,7 +17,7 @@ import pytest
 
 from parallem_gb300 import scenario as S
 from tests.helpers import NODATA, ringed
-from tests.test_gpu_parity import check_fa, libs, pair, run_steps  # noqa: F401
+from tests.test_gpu_parity import check_fa, check_fd, libs, pair, run_steps  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -115,3 +116,41 @@ def test_ids_of_winding_closed_flats(libs, n):
         z[y, 4:n - 4] = 50.0
         z[y:min(y + 4, n - 5), 4 if i % 2 else n - 5] = 50.0
     run_steps(libs, z, 1, np.full(1, 900.0), np.full(1, 9.0), False)
+
+
+def edge_lakes(h, w):
+    """A grid without a nodata ring: a closed flat over cell (0, 0), and flats and single pits on its other
+    edges, each at a height of its own, some of them reaching into the grid.  The ids of the corner's flat
+    are above those of the flat in row 0 and below those of the flats further down."""
+    y, x = np.mgrid[0:h, 0:w]
+    z = 500.0 + 0.8 * y + 0.5 * x + 3.0 * np.sin(x / 17.0) * np.cos(y / 23.0)
+    z[0:3, 0:3] = 50.0          # the corner
+    z[0, 10:13] = 300.0         # row 0 only: none of its cells has an id
+    z[0, 18] = 301.0
+    z[0:2, 22:25] = 302.0       # row 0, reaching in
+    z[h - 1, 5:8] = 303.0       # the last row
+    z[h - 1, 11] = 304.0
+    z[h - 2:h, 14:17] = 305.0   # reaching in
+    z[8:11, w - 1] = 306.0      # the last column
+    z[13, w - 1] = 307.0
+    z[16:19, w - 2:w] = 308.0   # reaching in
+    z[h - 2:h, w - 2:w] = 309.0  # the opposite corner
+    return z
+
+
+@pytest.mark.parametrize("shape", [(24, 30), (33, 64), (90, 131)])
+def test_ids_of_flats_on_the_edges_of_a_grid_without_a_ring(libs, shape):
+    z = edge_lakes(*shape)
+    o, g, mask = pair(libs, z, 900.0, 9.0, None, None)
+    o.flow_direction()
+    o.flow_accumulation()
+    soil = g.get("soilM")
+    for _ in range(10):  # the order in which the sinks are visited differs from call to call
+        g.set("soilM", soil)  # runoff changes soil moisture
+        g.flow_direction()
+        g.flow_accumulation()
+        g.synchronize()
+        check_fd(o, g, mask)
+        np.testing.assert_array_equal(g.get("watershed") == 0, o["watershed"] == 0)
+        np.testing.assert_array_equal(g.get("dem_routed"), o["dem_routed"])
+        check_fa(o, g, mask)
