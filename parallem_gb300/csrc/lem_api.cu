@@ -1,6 +1,9 @@
 // lem_api.cu -- the C ABI of include/lem_gb300.h: handle life cycle, field
 // transfers, climate state and stage orchestration.
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -379,6 +382,27 @@ void host_parallel(size_t n, const Fn& fn) {
     for (size_t i = 1; i < made; ++i) t[i].join();
 }
 
+// Whether a direct copy into these bytes of host memory is the faster one: true
+// when nearly all of their pages are mapped.  A copy that meets a page never
+// written waits about 43 us for it, and one through the staging takes 0.8 us a page
+// (64 KB) longer than a direct copy into mapped pages; so the direct copy is taken up
+// to one missing page in 32.  134 MB: direct 0.72 ms into mapped and 89 ms into fresh
+// pages, staged 2.4 and 3.0 ms; 9 MB: 0.07 and 6.5 ms, 0.44 and 0.50 ms; 0.07 MB: 0.02
+// and 0.40 ms, 0.03 and 0.06 ms.  The question takes 1 us, 10 us for 134 MB.  Memory that
+// is not the process's own is left to the copy, which says what is wrong with it.
+bool host_mapped(const void* host, size_t bytes) {
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), end = (uintptr_t)host + bytes;
+    const size_t pages = (end - (uintptr_t)host / page * page + page - 1) / page;
+    size_t missing = 0;
+    unsigned char in[1024];
+    for (uintptr_t at = (uintptr_t)host / page * page; at < end; at += sizeof in * page) {
+        const size_t n = std::min<size_t>(sizeof in, (end - at + page - 1) / page);
+        if (mincore(reinterpret_cast<void*>(at), n * page, in) != 0) return true;
+        for (size_t i = 0; i < n; ++i) missing += !(in[i] & 1);
+    }
+    return missing * 32 <= pages;
+}
+
 // Bytes per cell of a field's device representation, or 0 when it has none of its own.
 size_t raw_bytes(lem_field f) {
     switch (f) {
@@ -523,12 +547,9 @@ lem_status get_region_field(lem_handle* h, const HostDem& r, int id, lem_field f
     const void* src = f == LEM_F_DEM_ROUTED ? (o.sinkcount_pass1 ? s.zf : s.z) : raw_source(h, f);
     if (!src) return LEM_ERR_INVALID;
     const size_t elem = f == LEM_F_DEM_ROUTED ? 8 : raw_bytes(f);
-    // A field of the host's own type goes straight to the caller's memory where
-    // that is likely mapped (18 MB: 0.16 ms, 0.6 through the staging).  Arrays
-    // from 32 MB on usually stand on fresh pages, which a direct copy writes at
-    // 1.2 GB/s (a 4096 x 4096 DEM: 115 ms, 3.6 through the staging).
+    // a field of the host's own type goes straight to the caller's memory where that is mapped
     const bool same = f == LEM_F_DEM || f == LEM_F_DEM_ROUTED || f == LEM_F_CONTRIB || f == LEM_F_WATERSHED;
-    if (same && n * elem < (32u << 20)) {
+    if (same && host_mapped(host, n * elem)) {
         LEM_CUDA_TRY(cudaMemcpy2D(host, r.w * elem, static_cast<const char*>(src) + off * elem, W * elem, r.w * elem, r.h,
                                   cudaMemcpyDeviceToHost));
         return LEM_OK;
