@@ -361,16 +361,19 @@ bool any_flag(const lem_handle* h, uint32_t f) {
 // ---- field transfers of one DEM region (the whole grid for a single DEM)
 
 // fn(first, last) over [0, n) in equal parts, each on a thread of its own where a
-// part has at least kHostPart cells (at half of that, two threads take 0.22 ms
-// for a 512 x 512 grid and one 0.17).  A large grid handed to the host is first
-// touched here, so the threads share the page faults as well: 4096 x 4096 cells
-// take 3 ms, one thread 12.  The threads end before the call returns.
+// part has at least `part` cells (at half of kHostPart, two threads take 0.22 ms
+// for a 512 x 512 grid and one 0.17; loops that only widen or narrow integers are
+// done sooner and take twice as many: 800 x 800 codes 82 us on one thread, 92 on
+// two).  A large grid handed to the host is first touched here, so the threads
+// share the page faults as well: 4096 x 4096 cells take 3 ms, one thread 12.  The
+// threads end before the call returns.
 constexpr size_t kHostPart = 1 << 18;
 constexpr int kHostThreads = 8;
 template <class Fn>
-void host_parallel(size_t n, const Fn& fn) {
+void host_parallel(size_t n, size_t part, const Fn& fn) {
+    if (n < 2 * part) return fn(0, n);  // one part: asking for the number of processors takes 3 us
     const unsigned hw = std::thread::hardware_concurrency();
-    const size_t parts = std::min<size_t>(std::min<size_t>(kHostThreads, hw ? hw : 1), std::max<size_t>(1, n / kHostPart));
+    const size_t parts = std::min<size_t>(std::min<size_t>(kHostThreads, hw ? hw : 1), n / part);
     std::thread t[kHostThreads];
     size_t made = 1;  // part 0 is this thread's
     try {
@@ -438,7 +441,8 @@ bool is_code(lem_field f) { return f == LEM_F_FD || f == LEM_F_SFD || f == LEM_F
 // lem_get_field.  Codes: `mask` gives cells outside the catchment their -9999,
 // and in LEM_F_FD the outlet (a cell index of the region) flows west.
 void field_to_host(lem_field f, const void* raw, const uint8_t* mask, int64_t outlet, size_t n, void* host) {
-    host_parallel(n, [=](size_t lo, size_t hi) {
+    const size_t part = f == LEM_F_MASK || f == LEM_F_CONTRIB || f == LEM_F_WATERSHED ? 2 * kHostPart : kHostPart;
+    host_parallel(n, part, [=](size_t lo, size_t hi) {
         switch (f) {
             case LEM_F_DEM:
             case LEM_F_DEM_ROUTED:
@@ -496,7 +500,7 @@ lem_status set_region_field(lem_handle* h, const HostDem& r, lem_field f, const 
     if (f == LEM_F_DEM) {
         LEM_CUDA_TRY(cudaMemcpy2DAsync(s.z + off, W * 8, host, r.w * 8, r.w * 8, r.h, cudaMemcpyHostToDevice, h->st));
     } else if (f == LEM_F_FA) {
-        host_parallel(n, [&](size_t lo, size_t hi) {
+        host_parallel(n, kHostPart, [&](size_t lo, size_t hi) {
             const double* src = static_cast<const double*>(host);
             float2* t = static_cast<float2*>(stage);
             for (size_t i = lo; i < hi; ++i) {
@@ -507,7 +511,7 @@ lem_status set_region_field(lem_handle* h, const HostDem& r, lem_field f, const 
         LEM_CUDA_TRY(put(s.fa, 8));
     } else if (f == LEM_F_FD || f == LEM_F_SFD) {
         // int32 codes; -9999 (outside the catchment) keeps its low byte 0xF1
-        host_parallel(n, [&](size_t lo, size_t hi) {
+        host_parallel(n, 2 * kHostPart, [&](size_t lo, size_t hi) {
             const int32_t* src = static_cast<const int32_t*>(host);
             uint8_t* t = static_cast<uint8_t*>(stage);
             for (size_t i = lo; i < hi; ++i) t[i] = (uint8_t)(src[i] & 0xff);
@@ -518,7 +522,7 @@ lem_status set_region_field(lem_handle* h, const HostDem& r, lem_field f, const 
         const size_t per = f == LEM_F_SLOPES ? 8 : 1;
         float* dst = f == LEM_F_SLOPES ? s.slopes : float_field(h, f);
         if (!dst) return LEM_ERR_INVALID;
-        host_parallel(n, [&](size_t lo, size_t hi) {
+        host_parallel(n, kHostPart, [&](size_t lo, size_t hi) {
             const double* src = static_cast<const double*>(host);
             float* t = static_cast<float*>(stage);
             for (size_t i = per * lo; i < per * hi; ++i) t[i] = (float)src[i];
