@@ -93,7 +93,12 @@ constexpr int32_t kWordReady = kBlocked | 15;  // the bits that are 0 in a ready
 __device__ __forceinline__ int32_t wave_word(int count_and_block, uint32_t donors, uint32_t receivers) {
     return count_and_block | (int32_t)(donors << 8) | (int32_t)(receivers << 16);
 }
-constexpr int kWaveSpin = 1 << 26;  // polls of an idle warp before it gives up
+// Polls of an idle warp, with no progress seen, before it gives up.  Progress is a
+// change of the cells in flight, or of a count that a warp raises every kWaveBeat
+// cells of a path: a path of one warp may hold every cell of the grid and takes about
+// 1.7 us a cell (262144 cells: 0.46 s), so no fixed number of polls would do for it.
+constexpr uint32_t kWaveSpin = 1 << 23;
+constexpr int kWaveBeat = 256;
 
 // index step of direction d in a grid of width W
 __device__ __forceinline__ int32_t grid_step(int d, int W) { return dir_dy(d) * W + dir_dx(d); }
@@ -114,11 +119,12 @@ __device__ int wave_walk(const Op& op, int32_t* word, int32_t* list, int W, int 
     int32_t* const head = &sc->counters[1];
     int32_t* const inflight = &sc->counters[2];
     int32_t* const stop = &sc->counters[3];
+    int32_t* const beat = &sc->counters[4];
     const int nin = *tail;
     if (nin == 0) return 0;  // the same in every thread
     for (size_t i = nin + gtid; i < (size_t)N; i += gstride) list[i] = -1;
     if (gtid == 0) {
-        *head = *stop = 0;
+        *head = *stop = *beat = 0;
         *inflight = nin;
     }
     grid.sync();
@@ -130,14 +136,20 @@ __device__ int wave_walk(const Op& op, int32_t* word, int32_t* list, int W, int 
         if (lane == 0) ticket = atomicAdd(head, 1);
         ticket = __shfl_sync(0xffffffffu, ticket, 0);
         int32_t cur = -1;
-        for (int spin = 0;; ++spin) {
+        int32_t seen = -1, heard = -1;  // inflight and beat when they last changed
+        for (uint32_t spin = 0;; ++spin) {  // (lane 0's counts)
             if (lane == 0 && ticket < N) cur = *((volatile int32_t*)(list + ticket));
             cur = __shfl_sync(0xffffffffu, cur, 0);
             if (cur >= 0) break;
             int end = 0;
             if (lane == 0 && (spin & 15) == 15) {  // seldom: every waiting warp reads this one word
-                end = *((volatile int32_t*)inflight) == 0 || *((volatile int32_t*)stop);
-                if (!end && spin > kWaveSpin) {
+                const int32_t left = *((volatile int32_t*)inflight), at = *((volatile int32_t*)beat);
+                end = left == 0 || *((volatile int32_t*)stop);
+                if (left != seen || at != heard) {
+                    seen = left;
+                    heard = at;
+                    spin = 0;
+                } else if (!end && spin > kWaveSpin) {
                     raise_error(&sc->err, ErrFlags::kNoConverge);
                     atomicExch(stop, 1);
                     end = 1;
@@ -152,7 +164,7 @@ __device__ int wave_walk(const Op& op, int32_t* word, int32_t* list, int W, int 
         while (cur >= 0) {
             const uint32_t donors = (uint32_t)(info >> 8) & 255u;
             op.cell(cur, donors, op.donor(cur, b, lane < 8 && ((donors >> b) & 1u)));
-            ++done;
+            if ((++done & (kWaveBeat - 1)) == 0 && lane == 0) atomicAdd(beat, 1);
             __syncwarp();
             __threadfence();  // the finished cell, before its receivers' counts
             const bool on = lane < 8 && ((info >> (16 + b)) & 1);

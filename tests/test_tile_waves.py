@@ -51,6 +51,45 @@ def test_general_wave_with_several_receivers(libs, shape, slope, props):
               params=dict(flow_direction_type=1, mfd_proportions=props))
 
 
+@pytest.mark.parametrize("n", [5, 40, 333])
+def test_general_wave_along_one_path_of_all_cells(libs, n):
+    """Codes that run boustrophedon through every cell, with one negative weight: the general wave, whose other
+    warps wait for all of it."""
+    oracle, lem = libs
+    dem = ringed(np.full((n, n), 500.0), 2)
+    fd = np.full(dem.shape, -9999, np.int32)
+    for r in range(n):
+        row = fd[2 + r, 2:2 + n]
+        row[:] = 1 if r % 2 == 0 else 16
+        row[-1 if r % 2 == 0 else 0] = 4
+    st = S.initial_state(dem, 30.0, 800.0, 9.0)
+    g = lem.Model(dem, 30.0, 800.0, 9.0)
+    g.set_state(st)
+    g.flow_direction()
+    stone = st["stone"].copy()
+    stone[2, 2] = 300.0  # runs off less than nothing
+    g.set("stone", stone)
+    g.set("fd", fd)
+    g.set("sfd", fd)
+    g.flow_accumulation(lem.STEP_CONTRIB)
+    g.synchronize()
+    inside = dem[2:-2, 2:-2] != NODATA
+
+    def along(a):  # in path order
+        a = a[2:-2, 2:-2].copy()
+        a[1::2] = a[1::2, ::-1]
+        return a.reshape(-1)
+
+    assert inside.all() and g.totals()["fa_uncomputed"] == 0
+    w = along(g.get("runoff"))
+    assert w[0] < 0
+    want = np.concatenate([w[:1], np.cumsum(w[1:])])  # a negative sum of donors counts as none
+    # fp32 weights summed as float pairs: the accumulation tolerance of the parity tests
+    np.testing.assert_allclose(along(g.get("fa")), want, rtol=1e-5, atol=0)
+    np.testing.assert_array_equal(along(g.get("contrib")), np.arange(1, n * n + 1))
+    g.close()
+
+
 # a strip whose tiles the tables do not hold (the general wave), ragged grids, a code with two receivers
 @pytest.mark.parametrize("shape,double", [((1, 40), False), ((3, 40000), False), ((33, 31), False), ((257, 130), False),
                                           ((65, 97), True)])
