@@ -915,9 +915,10 @@ lem_status tune_record(lem_handle* h) {
     const int def = kTuneDefault;
     t.default_ms = t.tuned_ms = 0;
     for (int i = 0; i < kCoopKernels; ++i) {
+        auto launched = [&](int c) { return coop_for(h->s, h->k, i, coop_blocks_of(h, i, c)); };
         int best = def;
-        for (int c = 0; c < kTuneCands; ++c)
-            if (t.coop_ms[i][c] / t.coop_n[c] < t.coop_ms[i][best] / t.coop_n[best]) best = c;
+        for (int c = 0; c < kTuneCands; ++c)  // (on a small grid several launch the same blocks)
+            if (launched(c) != launched(def) && t.coop_ms[i][c] / t.coop_n[c] < t.coop_ms[i][best] / t.coop_n[best]) best = c;
         if (t.coop_ms[i][best] / t.coop_n[best] > kTuneMargin * t.coop_ms[i][def] / t.coop_n[def]) best = def;
         h->s.coop_blocks[i] = coop_blocks_of(h, i, best);
         t.default_ms += t.coop_ms[i][def] / t.coop_n[def];
@@ -1561,7 +1562,7 @@ lem_status lem_get_tuning(lem_handle* h, lem_tuning* out) {
     std::memset(out, 0, sizeof *out);
     out->state = h->tune.state;
     out->steps_left = h->tune.state == 1 ? h->tune.steps - h->tune.step : 0;
-    for (int i = 0; i < kCoopKernels; ++i) out->coop_blocks[i] = h->s.coop_blocks[i];
+    for (int i = 0; i < kCoopKernels; ++i) out->coop_blocks[i] = coop_for(h->s, h->k, i);
     out->default_ms = h->tune.default_ms;
     out->tuned_ms = h->tune.tuned_ms;
     out->flowdirs_tile_rows = h->s.fd_tma ? kFdRows[h->s.fd_rows] : 0;

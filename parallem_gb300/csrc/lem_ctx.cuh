@@ -135,7 +135,7 @@ struct DevState {
     int32_t n_live;             // tiles the canvas-wide kernels visit
     float* temp_tab;
     int32_t max_coop_blocks;    // co-resident blocks of the cooperative kernels
-    int32_t coop_blocks[kCoopKernels];  // blocks each cooperative kernel launches with (<= its coop_cap)
+    int32_t coop_blocks[kCoopKernels];  // blocks of each cooperative kernel's schedule (<= its coop_cap); coop_for: what it launches with
     int32_t coop_cap[kCoopKernels];     // co-resident blocks of each cooperative kernel
     const FdTmaMaps* fd_tma;    // host: the TMA flow-direction kernel's maps (null: rows TMA cannot address)
     int32_t fd_rows;            // its tile shape, an index into kFdRows
@@ -293,22 +293,27 @@ inline cudaError_t coop_launch(const void* fn, int blocks, void** args, cudaStre
     return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
-// Blocks of a cooperative kernel on a grid of that many 32x32 tiles: its schedule's
-// blocks, or `per_tile` for each tile where those are fewer.  A grid-wide barrier of
-// 608 blocks takes about 3 us and one of nine less than half of that, and the
-// blocks beyond the work do nothing else (a 96 x 96 grid: k_plateau_relax 34 us
-// with 608 blocks).
-inline int coop_for(const DevState& s, int kernel, int tiles, int per_tile) {
-    const int64_t b = (int64_t)tiles * per_tile;
-    return b < s.coop_blocks[kernel] ? (b > 0 ? (int)b : 1) : s.coop_blocks[kernel];
-}
-
 // Blocks of the general dependency wave on n cells: a warp for every 256 cells
 // covers the front of a slope (a row or two of the grid); more only watch the
 // list.
 inline int walk_blocks(int coop, size_t n) {
     const size_t b = (n + 2047) / 2048;
     return b < (size_t)coop ? (int)b : coop;
+}
+
+// Blocks a cooperative kernel launches with where its schedule gives it `blocks`:
+// at most kCoopPerTile for each of the 32x32 tiles it visits (0: a general wave).  A
+// grid-wide barrier of 608 blocks takes about 3 us and one of nine less than half of
+// that, and the blocks beyond the work do nothing else (a 96 x 96 grid:
+// k_plateau_relax 34 us with 608 blocks).
+constexpr int kCoopPerTile[kCoopKernels] = {1, 1, 1, 1, 2, 0, 2, 0};
+inline int coop_for(const DevState& s, const ModelConsts& k, int kernel, int blocks) {
+    if (kCoopPerTile[kernel] == 0) return walk_blocks(blocks, (size_t)k.W * k.H);
+    const int64_t b = (int64_t)tiles_of(s, k.W).n * kCoopPerTile[kernel];
+    return b < blocks ? (b > 0 ? (int)b : 1) : blocks;
+}
+inline int coop_for(const DevState& s, const ModelConsts& k, int kernel) {
+    return coop_for(s, k, kernel, s.coop_blocks[kernel]);
 }
 
 #define LEM_LAUNCH(L, kern, grid, block, ...)                  \

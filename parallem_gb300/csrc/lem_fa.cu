@@ -1046,7 +1046,7 @@ lem_status launch_flow_accumulation(const DevState& s, const ModelConsts& k, uin
         const TileSet ts = tiles_of(s, k.W);
         FatArgs a{s.z, s.mask, s.fd, s.w, s.fa, s.t_rec, s.t_dst, s.t_pend, s.t_ent, s.n_meta, s.p_ref,
                   reinterpret_cast<int2*>(s.f_idx), s.f_ds, s.t_fcnt, s.list_b, s.list_a, s.sc, s.dems,
-                  coop_for(s, kCkFatCoarse, ts.n, 2)};
+                  coop_for(s, k, kCkFatCoarse)};
         lem_status r = launch_fat(a, k, ts, 1, L);
         if (r != LEM_OK) return r;
         if (contrib) {
@@ -1068,7 +1068,7 @@ lem_status launch_flow_accumulation(const DevState& s, const ModelConsts& k, uin
         void* args[] = {(void*)&prop, (void*)&fa, (void*)&word, (void*)&contrib, (void*)&list,
                         (void*)&kk,   (void*)&sc, (void*)&dc,   (void*)&gate};
         L.pre("k_fa_walk");
-        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, walk_blocks(s.coop_blocks[kCkFaWalk], N), args, L.st));
+        LEM_CUDA_TRY(coop_launch((const void*)k_fa_walk, coop_for(s, k, kCkFaWalk), args, L.st));
         L.post();
     }
     if (flags & LEM_STEP_SET_OUTLET_FROM_FA) {  // some DEM moves its outlet this step

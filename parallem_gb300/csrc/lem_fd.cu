@@ -1616,7 +1616,7 @@ static lem_status direction_pass(const DevState& s, const ModelConsts& k, const 
         DevScalars* sc = s.sc;
         void* args[] = {(void*)&eqm,  (void*)&sp, (void*)&cand, (void*)&tq,  (void*)&tq_cap,
                         (void*)&mark, (void*)&kk, (void*)&sc,   (void*)&pass};
-        lem_status r = coop("k_plateau_relax", (const void*)k_plateau_relax, coop_for(s, kCkPlateau, ts.n, 1), args, L);
+        lem_status r = coop("k_plateau_relax", (const void*)k_plateau_relax, coop_for(s, k, kCkPlateau), args, L);
         if (r != LEM_OK) return r;
     }
     LEM_LAUNCH(L, k_plateau_final, flat_blocks(span, T, big), T, s.eqm, s.sp, s.list_a, s.sfd, s.mfd, slopes, k, s.sc,
@@ -1644,7 +1644,7 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
         ModelConsts kk = k;
         DevScalars* sc = s.sc;
         void* args[] = {(void*)&zz, (void*)&ws, (void*)&sinks, (void*)&merging, (void*)&kk, (void*)&sc};
-        if ((r = coop("k_flood_merge", (const void*)k_flood_merge, coop_for(s, kCkMerge, ts.n, 1), args, L)) != LEM_OK) return r;
+        if ((r = coop("k_flood_merge", (const void*)k_flood_merge, coop_for(s, k, kCkMerge), args, L)) != LEM_OK) return r;
     }
     {
         int32_t* ws = s.ws;
@@ -1657,7 +1657,7 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
         unsigned long long* ewt = s.ewt;
         void* args[] = {(void*)&ws,     (void*)&la, (void*)&lb, (void*)&ekey, (void*)&ewt,
                         (void*)&logmax, (void*)&kk, (void*)&sc, (void*)&tt};
-        if ((r = coop("k_flood_jump", (const void*)k_flood_jump, coop_for(s, kCkJump, ts.n, 1), args, L)) != LEM_OK) return r;
+        if ((r = coop("k_flood_jump", (const void*)k_flood_jump, coop_for(s, k, kCkJump), args, L)) != LEM_OK) return r;
     }
     {
         const dim3 eb(FE_BX, FE_BY), eg(ts.n, kTile / FE_BY);
@@ -1690,7 +1690,7 @@ lem_status launch_flow_direction(const DevState& s, const ModelConsts& k, const 
                         (void*)&cmaxw, (void*)&bidp, (void*)&blab, (void*)&up,    (void*)&wup,  (void*)&uv0,
                         (void*)&uv1,  (void*)&id0,  (void*)&id1,  (void*)&pick,  (void*)&reps, (void*)&list_cap,
                         (void*)&sc};
-        if ((r = coop("k_flood_spill", (const void*)k_flood_spill, coop_for(s, kCkSpill, ts.n, 1), args, L)) != LEM_OK) return r;
+        if ((r = coop("k_flood_spill", (const void*)k_flood_spill, coop_for(s, k, kCkSpill), args, L)) != LEM_OK) return r;
     }
     LEM_LAUNCH(L, k_flood_raise, flat_blocks(span, T, big), T, s.z, s.mask, s.ws, s.raise, s.zf, k, s.sc, s.dems,
                ts);

@@ -1602,7 +1602,7 @@ lem_status launch_erosion(const DevState& s, const ModelConsts& k, uint32_t flag
                         (void*)&pmap,  (void*)&pval, (void*)&depo, (void*)&stone, (void*)&fines, (void*)&soilT,
                         (void*)&tpend, (void*)&outs, (void*)&ready, (void*)&kk,   (void*)&sc};
         L.pre("k_sedt_coarse");
-        LEM_CUDA_TRY(coop_launch((const void*)k_sedt_coarse, coop_for(s, kCkSedCoarse, ts.n, 2), args, L.st));
+        LEM_CUDA_TRY(coop_launch((const void*)k_sedt_coarse, coop_for(s, k, kCkSedCoarse), args, L.st));
         L.post();
         LEM_LAUNCH(L, k_sedt_final, tiles, 256, s.mask, s.fd, s.ero, s.inci, s.geli, s.depo, s.stone, s.fines,
                    s.soilT, s.t_pend, s.t_stat, s.f_idx, s.f_map, s.f_ds, s.t_fcnt, s.p_val, k, s.sc, s.dems,
@@ -1624,8 +1624,7 @@ lem_status launch_erosion(const DevState& s, const ModelConsts& k, uint32_t flag
         void* args[] = {(void*)&prop, (void*)&coef, (void*)&nonzero, (void*)&depo, (void*)&stone, (void*)&fines, (void*)&soilT,
                         (void*)&word, (void*)&list, (void*)&kk,      (void*)&sc,   (void*)&dc,    (void*)&gate};
         L.pre("k_sed_walk");
-        LEM_CUDA_TRY(coop_launch((const void*)k_sed_walk, walk_blocks(s.coop_blocks[kCkSedWalk], (size_t)k.W * k.H), args,
-                                 L.st));
+        LEM_CUDA_TRY(coop_launch((const void*)k_sed_walk, coop_for(s, k, kCkSedWalk), args, L.st));
         L.post();
     }
     const bool diag = (flags & LEM_STEP_KEEP_DIAGNOSTICS) != 0;

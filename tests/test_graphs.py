@@ -155,3 +155,26 @@ def test_every_flow_direction_tile_shape_gives_the_same_steps(lem):
             np.testing.assert_array_equal(c.get(f), bt.get(i, f), err_msg=f)
     c.close()
     bt.close()
+
+
+def test_tuning_names_the_blocks_that_are_launched(lem):
+    """A small grid launches a block per 32x32 tile (two in the coarse waves) or per 2048 cells (the general
+    waves), whatever the schedule allows: lem_get_tuning says so, and the autotuner has nothing to choose between."""
+    dem = S.make_dem(92, 0.75, 600.0, 0.04, 10, 2, 91)
+    m = lem.Model(dem, 30.0, 900.0, 9.0)
+    m.set_state(S.initial_state(dem, 30.0, 900.0, 9.0))
+    want = {"k_plateau_relax": 9, "k_flood_merge": 9, "k_flood_jump": 9, "k_flood_spill": 9, "k_fat_coarse": 18,
+            "k_fa_walk": 5, "k_sedt_coarse": 18, "k_sed_walk": 5}
+    assert m.tuning()["coop_blocks"] == want
+    m.autotune(1)
+    for j in range(5):
+        m.step(900.0, 9.0, True)
+    m.synchronize()
+    t = m.tuning()
+    assert t["state"] == "tuned" and t["coop_blocks"] == want
+    m.close()
+    big = lem.Model(np.full((1024, 1024), 100.0), 30.0, 900.0, 9.0)
+    assert all(b <= 1024 for b in big.tuning()["coop_blocks"].values())
+    assert big.tuning()["coop_blocks"]["k_fa_walk"] == 512
+    assert big.tuning()["coop_blocks"]["k_plateau_relax"] > 9
+    big.close()
