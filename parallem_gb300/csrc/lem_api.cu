@@ -752,8 +752,6 @@ lem_status create_common(const lem_grid_desc* grid, const lem_params* params, in
     ALLOC(s.contrib, N);
     ALLOC(s.t_dst, N);
     ALLOC(s.t_pend, N);
-    ALLOC(s.t_rec, N);
-    ALLOC(s.t_nxt, N);
     {
         const size_t tiles = (size_t)((grid->width + kTile - 1) / kTile) * ((grid->height + kTile - 1) / kTile);
         ALLOC(s.t_ent, tiles * kTileEnt);
@@ -782,8 +780,15 @@ lem_status create_common(const lem_grid_desc* grid, const lem_params* params, in
     ALLOC(s.raise, N + 1);
     ALLOC(s.label_seen, N + 1);
     ALLOC(s.comp, N + 1);
-    ALLOC(s.cdist, N + 1);
-    ALLOC(s.cmaxw, N + 1);
+    // The coarse waves' records lie in the spill's two distance grids and their links in
+    // the general waves' words: neither is read by two stages, every stage writes what
+    // it reads, and a step's sediment takes either the tiles or the general wave.  A
+    // cell then needs no more memory than before it had records.
+    ALLOC(s.cdist, 2 * (N + 1));
+    s.cmaxw = s.cdist + (N + 1);
+    static_assert(sizeof(*s.t_rec) == 2 * sizeof(*s.cdist) && sizeof(*s.t_nxt) == sizeof(*s.pending), "shared grids");
+    s.t_rec = reinterpret_cast<int4*>(s.cdist);
+    s.t_nxt = s.pending;
     ALLOC(s.bid, N + 1);
     ALLOC(s.blab, N + 1);
     ALLOC(s.boff, N + 2);

@@ -86,12 +86,12 @@ struct DevState {
     // tiled accumulation (32x32 tiles): per cell, used at tile entries / outlets
     int32_t* t_dst;     // entry cell: the outlet of its tile its path reaches, or -1
     int32_t* t_pend;    // outlet: inflows still to arrive (kBlocked: never completes)
-    int4* t_rec;        // outlet: what the coarse waves read of it in one load.  Accumulation: the sum
+    int4* t_rec;        // (in cdist and cmaxw) outlet: what the coarse waves read of it in one load.  Accumulation: the sum
                         //   from inside its tile (float pair), (first << 16) | count of its inflows in
                         //   t_ent, the outlet it drains to (-1: none).  Sediment: (first << 16) | count
                         //   of its program's nodes, the same of their inputs, its deposition and new
                         //   soil thickness
-    int32_t* t_nxt;     // outlet: the outlet it drains to (sediment)
+    int32_t* t_nxt;     // (pending) outlet: the outlet it drains to (sediment)
     int32_t* t_ent;     // per tile, kTileEnt inflow cells (outlets of neighbours) grouped by outlet
     // tiled sediment routing: per tile, the cells that wait on other tiles as
     // programs (one per outlet, kTile*kTile slots per tile)

@@ -193,3 +193,12 @@ def test_ids_of_flats_on_the_edges_of_a_grid_without_a_ring(libs, shape):
         np.testing.assert_array_equal(g.get("watershed") == 0, o["watershed"] == 0)
         np.testing.assert_array_equal(g.get("dem_routed"), o["dem_routed"])
         check_fa(o, g, mask)
+
+
+@pytest.mark.parametrize("n,most", [(64, 1435508), (1024, 363404948)])
+def test_records_of_the_coarse_waves_take_no_memory_of_their_own(libs, n, most):
+    """`most`: the bytes of a grid whose coarse waves kept 12 bytes a cell (records and links take 20)."""
+    oracle, lem = libs
+    b = lem.Batch(n, n, 30.0, max_dems=1)
+    assert b.device_bytes() <= most
+    b.close()
