@@ -287,7 +287,8 @@ lem_status lem_set_limits(lem_handle* h, const lem_limits* limits);
 typedef struct lem_tuning {
     int32_t state;                          /* 0 default schedule, 1 tuning, 2 tuned            */
     int32_t steps_left;                     /* tuning steps still to run                        */
-    int32_t coop_blocks[LEM_TUNE_COOP];     /* blocks each cooperative kernel launches with    */
+    int32_t coop_blocks[LEM_TUNE_COOP];     /* blocks each cooperative kernel launches with: its
+                                               schedule's, fewer on a small grid               */
     double default_ms;                      /* ms per step of these kernels, default schedule  */
     double tuned_ms;                        /*   and with the schedule kept (as measured)       */
     int32_t flowdirs_tile_rows;             /* rows of the flow-direction kernel's 32-column TMA
