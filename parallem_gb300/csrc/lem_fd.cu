@@ -1283,7 +1283,7 @@ __global__ void __launch_bounds__(256)
     bool solo = false;
     int round = 1, live = n, nrep = nb;
     for (; live > 0; ++round) {
-        if (round >= round_cap_of(sc)) {
+        if (round > round_cap_of(sc)) {  // (as many rounds as the cap says have run)
             if (gtid == 0) raise_error(&sc->err, ErrFlags::kNoConverge);
             break;
         }

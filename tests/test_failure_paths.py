@@ -143,3 +143,23 @@ def test_cyclic_codes_complete_like_the_reference(libs):
         assert fa[r, 10] == pytest.approx(w[r, 10], rel=1e-6) and fa[r, 11] == pytest.approx(w[r, 11], rel=1e-6)
         if flags & lem.STEP_CONTRIB:
             np.testing.assert_array_equal(g.get("contrib"), o["contrib"])
+
+
+def test_spill_that_ends_in_the_last_round_allowed_is_no_error(libs):
+    """Pits of a strip that are all joined to basin 0 after two rounds of merging."""
+    oracle, lem = libs
+    x = NODATA
+    z = np.array([
+        [400, 400, 400, 439, 439, 452, 436, 436, x, x, 439, 436, 450, 454, 452, 451, x, x, 453, x, 453],
+        [400, 400, 400, 439, 439, 452, 451, 454, 451, 453, 451, 452, 451, 452, 453, 453, 451, 454, 451, 453, 453],
+        [400, 400, 400, 452, 450, 454, 451, 450, 453, 450, 454, x, 451, 451, 453, x, 454, 450, 454, 450, 452],
+        [x, 454, 451, 452, 453, 450, 453, 450, 453, 453, 450, 450, 451, x, 451, 453, 453, 452, 454, 453, 452]])
+    dem = ringed(z.astype(np.float64), 2)
+    o, g, _ = _pair(libs, dem)
+    g.limits(max_rounds=2)
+    g.flow_direction()
+    g.synchronize()
+    o.flow_direction()
+    np.testing.assert_array_equal(g.get("fd"), o["fd"])
+    np.testing.assert_array_equal(g.get("dem_routed"), o["dem_routed"])
+    assert g.totals()["spill_rounds"] == 3  # two, and the count the loop ends at
